@@ -21,6 +21,7 @@
 #include "../../include/contrafold_gb300.h"
 #include "cf_host.h"
 #include "cf_kernels.h"
+#include "cf_linear.h"
 #include "cf_queue.h"
 #include "cf_sample.h"
 #include "cf_warp.h"
@@ -253,12 +254,16 @@ struct cf_engine {
     DevBuf<int32_t> stream_idx;
     DevBuf<float> bonus;
     DevBuf<double> counts, unpaired;
+    DevBuf<int> fails;                            // sequences the sum-of-products kernels left (cf_linear.h)
+    DevBuf<cf::LinWeights<float>> lin32;          // their weights, made at the first call that needs them
+    DevBuf<cf::LinWeights<double>> lin64;
+    std::vector<double> host64;                   // the parameters, as set
     // stream-ordered allocation of every buffer above on the engine's stream
     void bind_buffers() {
         const cudaStream_t* s = &stream;
         blob32.sp = s; blob64.sp = s; arena.sp = s; seqs.sp = s; mask.sp = s; descs.sp = s; logz.sp = s;
         logz64.sp = s; structs.sp = s; post.sp = s; post_offs.sp = s; status.sp = s; samples.sp = s; seeds.sp = s;
-        stream_idx.sp = s; bonus.sp = s; counts.sp = s; unpaired.sp = s;
+        stream_idx.sp = s; bonus.sp = s; counts.sp = s; unpaired.sp = s; fails.sp = s; lin32.sp = s; lin64.sp = s;
     }
     size_t budget = 0;   // bytes; 0 = automatic (half of free memory at first use)
     int mode = 1;        // 0 plain, 1 batched
@@ -299,16 +304,103 @@ struct Plan {
     std::vector<int64_t> slice_words;
     int group = 1;
     int Lmax = 0;
+    int n_fold = 0;               // descs [0, n_fold) take the kernels above; the rest, sorted by falling length,
+    int lin_Lmax = 0;             // the sum-of-products kernels (longest length, arena slices)
+    std::vector<int> lin_begin;
+    int64_t arena_words() const {
+        int64_t w = 1;
+        for (int64_t x : slice_words) w = std::max(w, x);
+        return w;
+    }
 };
 
+// Longest sequence of a job that takes the sum-of-products kernels
+// (cf_linear.cu), in every mode and schedule; -1: none do.
+int lin_max_len(Job job) { return job == JOB_LOGZ ? cf::kLinMaxLen : job == JOB_LOGZ64 ? cf::kLinMaxLen64 : -1; }
+
+size_t budget_bytes(const cf_engine* eng) {
+    if (eng->budget != 0) return eng->budget;
+    size_t fr = 0, tot = 0;
+    cudaMemGetInfo(&fr, &tot);
+    return fr / 2;
+}
+
+// Weights of the sum-of-products kernels on the device.
+int ensure_weights(cf_engine* e, bool fp64) {
+    if (fp64) {
+        if (e->lin64.p) return CF_OK;
+        int rc = e->lin64.ensure(1);
+        if (rc) return rc;
+        cf::LinWeights<double> w;
+        cf::lin_weights(e->host64.data(), &w);
+        CF_CUDA(cudaMemcpyAsync(e->lin64.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
+    } else {
+        if (e->lin32.p) return CF_OK;
+        int rc = e->lin32.ensure(1);
+        if (rc) return rc;
+        cf::LinWeights<float> w;
+        cf::lin_weights(e->host64.data(), &w);
+        CF_CUDA(cudaMemcpyAsync(e->lin32.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
+    }
+    CF_CUDA(cudaStreamSynchronize(e->stream));   // once per parameter set: readable on every stream after it
+    return CF_OK;
+}
+
+int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<int> order, Plan& P);
+
 int make_plan(cf_engine* eng, Job job, const int64_t* offsets, int n, Plan& P) {
-    P.descs.resize(n);
-    std::vector<int> order(n);
+    auto len = [&](int b) { return (int)(offsets[b + 1] - offsets[b]); };
+    std::vector<int> order(n), lin;
     std::iota(order.begin(), order.end(), 0);
+    if (const int most_len = lin_max_len(job); most_len >= 0) {
+        const auto mid = std::stable_partition(order.begin(), order.end(), [&](int b) { return len(b) > most_len; });
+        lin.assign(mid, order.end());
+        order.erase(mid, order.end());
+        std::stable_sort(lin.begin(), lin.end(), [&](int x, int y) { return len(x) > len(y); });
+    }
+    P.n_fold = (int)order.size();
+    if (lin.empty() || P.n_fold > 0) {
+        const int rc = make_fold_plan(eng, job, offsets, std::move(order), P);
+        if (rc) return rc;
+    } else {
+        P.plain = eng->mode != 1;   // nothing left for the other kernels
+    }
+    P.lin_begin.clear();
+    if (lin.empty()) return CF_OK;
+    int rc = ensure_weights(eng, job == JOB_LOGZ64);
+    if (rc) return rc;
+    P.lin_Lmax = len(lin[0]);
+    const int64_t most = (int64_t)(budget_bytes(eng) / 4);
+    int64_t cur = 0, widest = 0;
+    P.lin_begin.push_back(P.n_fold);
+    for (int b : lin) {
+        const int64_t words = arena_words(job, len(b));
+        if (words > most) return fail(CF_ENOMEM, "sequence does not fit the arena budget");
+        if (cur + words > most) {
+            P.lin_begin.push_back((int)P.descs.size());
+            cur = 0;
+        }
+        SeqDesc D;
+        D.seq_off = offsets[b];
+        D.L = len(b);
+        D.idx = b;
+        D.ws_off = cur;
+        P.descs.push_back(D);
+        cur += words;
+        widest = std::max(widest, cur);
+    }
+    P.lin_begin.push_back((int)P.descs.size());
+    P.slice_words.push_back(widest);   // the slices share the arena with the others', one after another
+    return CF_OK;
+}
+
+int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<int> order, Plan& P) {
+    const int n = (int)order.size();
+    P.descs.resize(n);
     P.group = 1;
     P.Lmax = 0;
     int Lmin = n ? CF_MAX_LEN : 0;
-    for (int b = 0; b < n; ++b) {
+    for (int b : order) {
         P.Lmax = std::max<int>(P.Lmax, (int)(offsets[b + 1] - offsets[b]));
         Lmin = std::min<int>(Lmin, (int)(offsets[b + 1] - offsets[b]));
     }
@@ -351,13 +443,7 @@ int make_plan(cf_engine* eng, Job job, const int64_t* offsets, int n, Plan& P) {
         P.descs[k].ws_off = 0;
     }
     // arena slices within the budget
-    size_t budget = eng->budget;
-    if (budget == 0) {
-        size_t fr = 0, tot = 0;
-        cudaMemGetInfo(&fr, &tot);
-        budget = fr / 2;
-    }
-    const int64_t budget_words = (int64_t)(budget / 4);
+    const int64_t budget_words = (int64_t)(budget_bytes(eng) / 4);
     // batched schedule: the fused per-sequence CTA kernel keeps only a few
     // sequences per SM in flight (their tables stay in L2); the warp kernel
     // runs one sequence per warp (short sequences, sampling).
@@ -595,6 +681,7 @@ struct Exec {
     const SeqDesc* d_descs = nullptr;
     float* arena = nullptr;
     int* status = nullptr;
+    int* fails = nullptr;   // 1 + n words (jobs with sum-of-products kernels)
     PhaseTimer* timer = nullptr;
     int launches = 0;   // kernels launched by the last run
 };
@@ -609,15 +696,64 @@ struct Exec {
         if (X.timer && (rc = X.timer->end(stop_, st))) return rc;          \
     } while (0)
 
+// logZ of the descs [P.n_fold, end): one CTA each, then the log-domain kernel
+// for those whose values left the float's range (none, as a rule: it ends at
+// once; its grid covers all of them).
+int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d_seqs, const uint8_t* d_mask,
+               float* d_logz, double* d_logz64, cudaStream_t st) {
+    int rc;
+    const bool fp64 = job == JOB_LOGZ64;
+    const size_t smem = cf::lin_inside_smem_bytes(P.lin_Lmax, fp64), redo = cf::fold_smem_bytes(P.lin_Lmax, 1, fp64);
+    if ((rc = raise_smem_limit(fp64 ? (const void*)cf::k_lin_inside64 : (const void*)cf::k_lin_inside32, eng->device,
+                               std::max<size_t>(smem, 48 * 1024))))
+        return rc;
+    int sms = 0;
+    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
+    for (size_t s = 0; s + 1 < P.lin_begin.size(); ++s) {
+        cf::FoldArgs A{};
+        A.descs = X.d_descs + P.lin_begin[s];
+        A.n = P.lin_begin[s + 1] - P.lin_begin[s];
+        A.group = 1;
+        A.seqs = d_seqs;
+        A.mask = d_mask;
+        A.blob32 = eng->blob32.p;
+        A.blob64 = eng->blob64.p;
+        A.ws = X.arena;
+        A.logz = d_logz;
+        A.logz64 = d_logz64;
+        A.status = X.status;
+        cf::LinArgs La;
+        La.descs = A.descs;
+        La.n = A.n;
+        La.seqs = d_seqs;
+        La.mask = d_mask;
+        La.weights = fp64 ? (const void*)eng->lin64.p : (const void*)eng->lin32.p;
+        La.ws = X.arena;
+        La.logz = fp64 ? (void*)d_logz64 : (void*)d_logz;
+        La.fails = X.fails;
+        const int rgrid = std::min(A.n, cf::kFoldMinBlocks * sms);
+        CF_CUDA(cudaMemsetAsync(X.fails, 0, sizeof(int), st));
+        if (fp64) {
+            CF_PHASE(0, (cf::k_lin_inside64<<<A.n, cf::kLinThreads, smem, st>>>(La)));
+            CF_PHASE(0, (cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails)));
+        } else {
+            CF_PHASE(0, (cf::k_lin_inside32<<<A.n, cf::kLinThreads, smem, st>>>(La)));
+            CF_PHASE(0, (cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails)));
+        }
+    }
+    return CF_OK;
+}
+
 // Launches `job` over a planned batch whose inputs are already on the device.
 int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d_seqs, const uint8_t* d_mask,
                float gamma, float* d_logz, double* d_logz64, char* d_structs, float* d_post,
                const int64_t* d_post_offs, cudaStream_t st, const SampleJob* sj = nullptr) {
-    const int n = (int)P.descs.size();
+    const int n = P.n_fold;
     X.launches = 0;
     if (X.timer) X.timer->reset();
-    if (n == 0) return CF_OK;
     int rc;
+    if (!P.lin_begin.empty() && (rc = run_linear(eng, job, P, X, d_seqs, d_mask, d_logz, d_logz64, st))) return rc;
+    if (n == 0) return CF_OK;
     if (P.cta) {
         cf::FoldArgs A;
         A.descs = X.d_descs;
@@ -911,15 +1047,15 @@ int run_host(cf_engine* eng, Job job, const uint8_t* seqs, const int64_t* offset
     }
     if ((rc = eng->descs.ensure(n))) return rc;
     CF_CUDA(cudaMemcpyAsync(eng->descs.p, P.descs.data(), sizeof(SeqDesc) * n, cudaMemcpyHostToDevice, st));
-    int64_t maxw = 1;
-    for (int64_t w : P.slice_words) maxw = std::max(maxw, w);
-    if ((rc = eng->arena.ensure((size_t)maxw))) return rc;
+    if ((rc = eng->arena.ensure((size_t)P.arena_words()))) return rc;
     if ((rc = eng->status.ensure(2))) return rc;
+    if (!P.lin_begin.empty() && (rc = eng->fails.ensure((size_t)n + 1))) return rc;
     CF_CUDA(cudaMemsetAsync(eng->status.p, 0, sizeof(int), st));
     Exec X;
     X.d_descs = eng->descs.p;
     X.arena = eng->arena.p;
     X.status = eng->status.p;
+    X.fails = eng->fails.p;
     if ((rc = run_device(eng, job, P, X, eng->seqs.p, d_mask, gamma, d_logz, d_logz64, d_structs, d_post, d_post_offs,
                          st, &sj)))
         return rc;
@@ -994,6 +1130,7 @@ int cf_engine_destroy(cf_engine* e) {
     e->descs.release(); e->logz.release(); e->logz64.release(); e->structs.release(); e->post.release();
     e->post_offs.release(); e->status.release(); e->samples.release(); e->seeds.release(); e->stream_idx.release();
     e->bonus.release(); e->counts.release(); e->unpaired.release();
+    e->fails.release(); e->lin32.release(); e->lin64.release();
     if (e->stream) cudaStreamSynchronize(e->stream);   // the stream-ordered frees
 
     if (e->stream_lo) cudaStreamDestroy(e->stream_lo);
@@ -1033,6 +1170,18 @@ int cf_engine_set_params(cf_engine* e, const float* params32, const double* para
     if ((rc = e->blob64.ensure(CF_BLOB_LEN))) return rc;
     CF_CUDA(cudaMemcpyAsync(e->blob32.p, params32, sizeof(float) * CF_BLOB_LEN, cudaMemcpyHostToDevice, e->stream));
     CF_CUDA(cudaMemcpyAsync(e->blob64.p, params64, sizeof(double) * CF_BLOB_LEN, cudaMemcpyHostToDevice, e->stream));
+    e->host64.assign(params64, params64 + CF_BLOB_LEN);
+    // weights made of the parameters before these: again, in place (plans and their graphs read them there)
+    if (e->lin32.p) {
+        cf::LinWeights<float> w;
+        cf::lin_weights(params64, &w);
+        CF_CUDA(cudaMemcpyAsync(e->lin32.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
+    }
+    if (e->lin64.p) {
+        cf::LinWeights<double> w;
+        cf::lin_weights(params64, &w);
+        CF_CUDA(cudaMemcpyAsync(e->lin64.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
+    }
     CF_CUDA(cudaStreamSynchronize(e->stream));
     return CF_OK;
 }
@@ -1202,9 +1351,7 @@ extern "C" int cf_grad(cf_engine* e, const uint8_t* seqs, const int64_t* offsets
         return rc;
     CF_CUDA(cudaMemcpyAsync(e->descs.p, P.descs.data(), sizeof(SeqDesc) * n, cudaMemcpyHostToDevice, st));
     CF_CUDA(cudaMemsetAsync(e->status.p, 0, sizeof(int), st));
-    int64_t maxw = 1;
-    for (int64_t w : P.slice_words) maxw = std::max(maxw, w);
-    if ((rc = e->arena.ensure((size_t)maxw))) return rc;
+    if ((rc = e->arena.ensure((size_t)P.arena_words()))) return rc;
     const size_t smem = cf::adj_smem_bytes(P.Lmax);
     {
         int dev_max = 0;
@@ -1251,7 +1398,7 @@ struct cf_plan {
     int n = 0;
     DevBuf<SeqDesc> descs;
     DevBuf<float> arena;
-    DevBuf<int> status;
+    DevBuf<int> status, fails;
     DevBuf<int64_t> post_offs;   // CF_JOB_BPP: sequence b's matrix at sum_{c<b} L_c^2 floats
     PhaseTimer timer;
     int launches = 0;
@@ -1272,6 +1419,13 @@ namespace {
 // then records kernel launches only.
 int plan_prepare_smem(cf_engine* e, Job job, const Plan& P) {
     size_t bytes;
+    if (!P.lin_begin.empty()) {
+        const bool fp64 = job == JOB_LOGZ64;
+        const int rc = raise_smem_limit(fp64 ? (const void*)cf::k_lin_inside64 : (const void*)cf::k_lin_inside32,
+                                        e->device, std::max<size_t>(cf::lin_inside_smem_bytes(P.lin_Lmax, fp64), 48 * 1024));
+        if (rc) return rc;
+        if (P.n_fold == 0) return CF_OK;
+    }
     if (P.cta) {
         bytes = cf::fold_smem_bytes(P.Lmax, 1, false);
     } else if (P.warp) {
@@ -1304,15 +1458,25 @@ int cf_plan_create(cf_engine* e, int32_t job, const int64_t* offsets, int32_t n,
     p->job = job == CF_JOB_LOGZ ? JOB_LOGZ : job == CF_JOB_LOGZ64 ? JOB_LOGZ64 : job == CF_JOB_BPP ? JOB_BPP
            : job == CF_JOB_MEA ? JOB_MEA : JOB_MFE;
     p->n = n;
-    if ((rc = make_plan(e, p->job, offsets, n, p->P)) || (rc = p->descs.ensure(std::max(n, 1))) ||
+    rc = make_plan(e, p->job, offsets, n, p->P);
+    if (!rc && n > 0 && p->P.n_fold == 0) {
+        // every sequence takes the sum-of-products kernels: the schedule the batch is tuned to is still what
+        // cf_plan_schedule and cf_plan_group report
+        Plan S;
+        std::vector<int> all(n);
+        std::iota(all.begin(), all.end(), 0);
+        if (!(rc = make_fold_plan(e, p->job, offsets, std::move(all), S))) {
+            p->P.plain = S.plain; p->P.cta = S.cta; p->P.warp = S.warp; p->P.cluster = S.cluster; p->P.group = S.group;
+        }
+    }
+    if (rc || (rc = p->descs.ensure(std::max(n, 1))) ||
         (rc = p->status.ensure(2))) {
         delete p;
         return rc;
     }
-    int64_t maxw = 1;
-    for (int64_t w : p->P.slice_words) maxw = std::max(maxw, w);
-    if ((rc = p->arena.ensure((size_t)maxw))) {
-        p->descs.release(); p->status.release();
+    if ((rc = p->arena.ensure((size_t)p->P.arena_words())) ||
+        (!p->P.lin_begin.empty() && (rc = p->fails.ensure((size_t)n + 1)))) {
+        p->descs.release(); p->status.release(); p->arena.release();
         delete p;
         return rc;
     }
@@ -1341,6 +1505,7 @@ int cf_plan_destroy(cf_plan* p) {
     cudaDeviceSynchronize();
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     p->descs.release(); p->arena.release(); p->status.release(); p->post_offs.release();
+    p->fails.release();
     delete p;
     return CF_OK;
 }
@@ -1356,6 +1521,7 @@ int cf_plan_run(cf_plan* p, const uint8_t* d_seqs, const uint8_t* d_mask, float 
     X.d_descs = p->descs.p;
     X.arena = p->arena.p;
     X.status = p->status.p;
+    X.fails = p->fails.p;
     X.timer = p->timer.on ? &p->timer : nullptr;
     float* lz = p->job == JOB_LOGZ ? static_cast<float*>(d_out) : nullptr;
     double* lz64 = p->job == JOB_LOGZ64 ? static_cast<double*>(d_out) : nullptr;

@@ -355,6 +355,42 @@ __global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside64(FoldA
         A.logz64[sm->idx[g]] = in_view<double>(A, sm->ws[g], sm->L[g]).T.F5[sm->L[g]];
 }
 
+// Sequences that the sum-of-products kernels left (fails[0] of them, descs
+// indices fails[1 ..]; usually none), one CTA each, in the log domain.
+template <class S>
+__device__ __forceinline__ void inside_redo(const FoldArgs& A, const int* fails, const typename S::Real* blob,
+                                            typename S::Real* out) {
+    using R = typename S::Real;
+    const int n = fails[0];
+    if ((int)blockIdx.x >= n) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto* sm = reinterpret_cast<SmemFold<R>*>(smem_raw);
+    load_tabs(&sm->tabs, blob);
+    load_poly_tables(&sm->poly);
+    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const SeqDesc D = A.descs[fails[1 + k]];
+            sm->L[0] = D.L;
+            sm->ws[0] = D.ws_off;
+            sm->soff[0] = D.seq_off;
+            sm->idx[0] = D.idx;
+            sm->n = sm->gcap = 1;
+            sm->Lmax = D.L;
+        }
+        __syncthreads();
+        build_group_seqs(sm, A);
+        inside_group<S>(sm, A);
+        if (threadIdx.x == 0) out[sm->idx[0]] = in_view<R>(A, sm->ws[0], sm->L[0]).T.F5[sm->L[0]];
+    }
+}
+__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo32(FoldArgs A, const int* fails) {
+    inside_redo<LseAcc32>(A, fails, A.blob32, A.logz);
+}
+__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo64(FoldArgs A, const int* fails) {
+    inside_redo<Lse64>(A, fails, A.blob64, A.logz64);
+}
+
 // ---------------------------------------------------------------------------
 // Outside + posterior + MEA (FP32)
 // ---------------------------------------------------------------------------

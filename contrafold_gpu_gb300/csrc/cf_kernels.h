@@ -68,6 +68,9 @@ struct ClusterKernels {
 ClusterKernels cluster_kernels();
 __global__ void k_inside64(FoldArgs A);
 __global__ void k_viterbi64(FoldArgs A);
+// log-domain logZ of the sequences listed in fails (cf_linear.cu)
+__global__ void k_inside_redo32(FoldArgs A, const int* fails);
+__global__ void k_inside_redo64(FoldArgs A, const int* fails);
 
 size_t fold_smem_bytes(int Lmax, int group, bool fp64);
 
