@@ -143,8 +143,14 @@ __device__ __forceinline__ AdjView adj_view(const FoldArgs& A, const SeqDesc& D,
 __device__ __forceinline__ float bon(const double* U, int lo, int hi) { return (float)(U[hi] - U[lo]); }
 __device__ __forceinline__ float ubon(const double* U, int k) { return (float)(U[k] - U[k - 1]); }
 
-__device__ __forceinline__ SeqView adj_setup(AdjSmem* sm, const FoldArgs& A, SeqDesc& D) {
-    D = A.descs[blockIdx.x];
+// list (nullable): [0] its length, [1 ..] the descs indices to take
+__device__ __forceinline__ bool adj_mine(const FoldArgs& A, const int* list, SeqDesc& D) {
+    if (list != nullptr && (int)blockIdx.x >= list[0]) return false;
+    D = A.descs[list != nullptr ? list[1 + blockIdx.x] : (int)blockIdx.x];
+    return true;
+}
+
+__device__ __forceinline__ SeqView adj_setup(AdjSmem* sm, const FoldArgs& A, const SeqDesc& D) {
     load_tabs(&sm->tabs, A.blob32);
     load_window(sm);
     int8_t* s = reinterpret_cast<int8_t*>(sm + 1);
@@ -207,10 +213,12 @@ __device__ __forceinline__ float fm2_warp(const InTabs<float>& T, int i, int j, 
 // Inside with bonus (accurate float32 log-sum-exp); FM2 kept on every ckpt-th
 // diagonal.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kFoldThreads) k_adj_inside(FoldArgs A, const float* bonus, int ckpt) {
+__global__ void __launch_bounds__(kFoldThreads) k_adj_inside(FoldArgs A, const float* bonus, int ckpt,
+                                                              const int* list) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* sm = reinterpret_cast<AdjSmem*>(smem_raw);
     SeqDesc D;
+    if (!adj_mine(A, list, D)) return;
     const SeqView Q = adj_setup(sm, A, D);
     const ParamView<float> P{sm->tabs.blob};
     const AdjView V = adj_view(A, D, ckpt);
@@ -545,10 +553,11 @@ __device__ __forceinline__ double fixp_value(double hi, unsigned long long lo) {
 }  // namespace
 
 __global__ void __launch_bounds__(kFoldThreads) k_adj_outside(FoldArgs A, const float* bonus, int ckpt,
-                                                               double* counts_out, double* unpaired_out) {
+                                                               double* counts_out, double* unpaired_out, const int* list) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* sm = reinterpret_cast<AdjSmem*>(smem_raw);
     SeqDesc D;
+    if (!adj_mine(A, list, D)) return;
     const SeqView Q = adj_setup(sm, A, D);
     const ParamView<float> P{sm->tabs.blob};
     const AdjView V = adj_view(A, D, ckpt);

@@ -233,6 +233,39 @@ const TuneRow* match_tuning(const std::vector<TuneRow>& rows, Job job, int n, in
 
 }  // namespace
 
+namespace {
+// Side streams of the sum-of-products inside: its length classes run at the
+// same time, each with its own shared memory.  Made at the first batch of
+// several classes; every owner (an engine's calls, a plan) has its own, so
+// runs of different plans never share an event.
+struct LinStreams {
+    static constexpr int kSide = 4;
+    cudaStream_t side[kSide] = {};
+    cudaEvent_t fork = nullptr, join[kSide] = {};
+    int ensure() {
+        if (fork) return CF_OK;
+        cudaEvent_t f = nullptr;
+        CF_CUDA(cudaEventCreateWithFlags(&f, cudaEventDisableTiming));
+        for (int k = 0; k < kSide; ++k) {
+            if (!side[k]) CF_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+            if (!join[k]) CF_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
+        }
+        fork = f;
+        return CF_OK;
+    }
+    void release() {
+        for (int k = 0; k < kSide; ++k) {
+            if (side[k]) cudaStreamDestroy(side[k]);
+            if (join[k]) cudaEventDestroy(join[k]);
+            side[k] = nullptr;
+            join[k] = nullptr;
+        }
+        if (fork) cudaEventDestroy(fork);
+        fork = nullptr;
+    }
+};
+}  // namespace
+
 struct cf_engine {
     int device = 0;
     cudaStream_t stream = nullptr;       // the stream of the engine's calls: one of the two below
@@ -258,6 +291,7 @@ struct cf_engine {
     DevBuf<cf::LinWeights<float>> lin32;          // their weights, made at the first call that needs them
     DevBuf<cf::LinWeights<double>> lin64;
     std::vector<double> host64;                   // the parameters, as set
+    LinStreams lin_streams;
     // stream-ordered allocation of every buffer above on the engine's stream
     void bind_buffers() {
         const cudaStream_t* s = &stream;
@@ -316,7 +350,10 @@ struct Plan {
 
 // Longest sequence of a job that takes the sum-of-products kernels
 // (cf_linear.cu), in every mode and schedule; -1: none do.
-int lin_max_len(Job job) { return job == JOB_LOGZ ? cf::kLinMaxLen : job == JOB_LOGZ64 ? cf::kLinMaxLen64 : -1; }
+int lin_max_len(Job job) {
+    return job == JOB_LOGZ ? cf::kLinMaxLen : job == JOB_LOGZ64 ? cf::kLinMaxLen64
+         : job == JOB_GRAD ? cf::kLinMaxLenGrad : -1;
+}
 
 size_t budget_bytes(const cf_engine* eng) {
     if (eng->budget != 0) return eng->budget;
@@ -359,6 +396,9 @@ int make_plan(cf_engine* eng, Job job, const int64_t* offsets, int n, Plan& P) {
         std::stable_sort(lin.begin(), lin.end(), [&](int x, int y) { return len(x) > len(y); });
     }
     P.n_fold = (int)order.size();
+    int Lmax = 0;
+    for (int b = 0; b < n; ++b) Lmax = std::max(Lmax, len(b));
+    P.grad_ckpt = eng->grad_ckpt > 0 ? eng->grad_ckpt : cf::adj_auto_checkpoint(Lmax);
     if (lin.empty() || P.n_fold > 0) {
         const int rc = make_fold_plan(eng, job, offsets, std::move(order), P);
         if (rc) return rc;
@@ -374,7 +414,7 @@ int make_plan(cf_engine* eng, Job job, const int64_t* offsets, int n, Plan& P) {
     int64_t cur = 0, widest = 0;
     P.lin_begin.push_back(P.n_fold);
     for (int b : lin) {
-        const int64_t words = arena_words(job, len(b));
+        const int64_t words = arena_words(job, len(b), P.grad_ckpt);
         if (words > most) return fail(CF_ENOMEM, "sequence does not fit the arena budget");
         if (cur + words > most) {
             P.lin_begin.push_back((int)P.descs.size());
@@ -552,7 +592,6 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         }
         P.warp = false;   // not even one CTA of warp slots fits: per-sequence kernels, sliced
     }
-    P.grad_ckpt = eng->grad_ckpt > 0 ? eng->grad_ckpt : cf::adj_auto_checkpoint(P.Lmax);
     P.slice_begin.clear();
     P.slice_words.clear();
     int64_t cur = 0;
@@ -682,6 +721,7 @@ struct Exec {
     float* arena = nullptr;
     int* status = nullptr;
     int* fails = nullptr;   // 1 + n words (jobs with sum-of-products kernels)
+    LinStreams* lin_streams = nullptr;
     PhaseTimer* timer = nullptr;
     int launches = 0;   // kernels launched by the last run
 };
@@ -696,6 +736,51 @@ struct Exec {
         if (X.timer && (rc = X.timer->end(stop_, st))) return rc;          \
     } while (0)
 
+// Before the launches of a plan (and outside a stream capture): shared-memory
+// limits and side streams of its sum-of-products inside.
+int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S) {
+    const bool fp64 = job == JOB_LOGZ64, train = job == JOB_GRAD;
+    int classes = 0;
+    for (size_t k = P.n_fold; k < P.descs.size(); ++classes) {
+        const int L = P.descs[k].L, rc = raise_smem_limit((const void*)cf::lin_inside_kernel(L, fp64, train).fn, eng->device,
+                                                          std::max<size_t>(cf::lin_inside_smem_bytes(L, fp64), 48 * 1024));
+        if (rc) return rc;
+        while (k < P.descs.size() && cf::lin_class_end(P.descs[k].L, fp64) == cf::lin_class_end(L, fp64)) ++k;
+    }
+    return classes > 1 ? S->ensure() : CF_OK;
+}
+
+// The inside of descs [k0, k1), sorted by falling length: a launch for each
+// length class, on side streams beside st but for the first.  A launch of all
+// of them would give every CTA the longest one's shared memory (1,024 x 50-500
+// nt on GB300: one CTA an SM, 15.0 ms).
+int launch_lin_inside(const Plan& P, const cf::LinArgs& A, int k0, int k1, bool fp64, bool train, LinStreams* S,
+                      cudaStream_t st, int& launches) {
+    int used = 0;
+    for (int k = k0; k < k1;) {
+        const int L = P.descs[k].L, end = cf::lin_class_end(L, fp64);
+        int q = k;
+        while (q < k1 && cf::lin_class_end(P.descs[q].L, fp64) == end) ++q;
+        const cf::LinKernel K = cf::lin_inside_kernel(L, fp64, train);
+        cudaStream_t on = st;
+        if (k > k0) {
+            on = S->side[used];
+            CF_CUDA(cudaStreamWaitEvent(on, S->fork, 0));
+        } else if (q < k1) {
+            CF_CUDA(cudaEventRecord(S->fork, st));
+        }
+        cf::LinArgs B = A;
+        B.first = k - k0;
+        K.fn<<<q - k, K.threads, cf::lin_inside_smem_bytes(L, fp64), on>>>(B);
+        ++launches;
+        CF_CUDA(cudaGetLastError());
+        if (k > k0) CF_CUDA(cudaEventRecord(S->join[used++], on));
+        k = q;
+    }
+    for (int u = 0; u < used; ++u) CF_CUDA(cudaStreamWaitEvent(st, S->join[u], 0));
+    return CF_OK;
+}
+
 // logZ of the descs [P.n_fold, end): one CTA each, then the log-domain kernel
 // for those whose values left the float's range (none, as a rule: it ends at
 // once; its grid covers all of them).
@@ -703,16 +788,15 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
                float* d_logz, double* d_logz64, cudaStream_t st) {
     int rc;
     const bool fp64 = job == JOB_LOGZ64;
-    const size_t smem = cf::lin_inside_smem_bytes(P.lin_Lmax, fp64), redo = cf::fold_smem_bytes(P.lin_Lmax, 1, fp64);
-    if ((rc = raise_smem_limit(fp64 ? (const void*)cf::k_lin_inside64 : (const void*)cf::k_lin_inside32, eng->device,
-                               std::max<size_t>(smem, 48 * 1024))))
-        return rc;
+    if ((rc = prepare_linear(eng, job, P, X.lin_streams))) return rc;
+    const size_t redo = cf::fold_smem_bytes(P.lin_Lmax, 1, fp64);
     int sms = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
     for (size_t s = 0; s + 1 < P.lin_begin.size(); ++s) {
+        const int k0 = P.lin_begin[s], k1 = P.lin_begin[s + 1];
         cf::FoldArgs A{};
-        A.descs = X.d_descs + P.lin_begin[s];
-        A.n = P.lin_begin[s + 1] - P.lin_begin[s];
+        A.descs = X.d_descs + k0;
+        A.n = k1 - k0;
         A.group = 1;
         A.seqs = d_seqs;
         A.mask = d_mask;
@@ -722,9 +806,8 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         A.logz = d_logz;
         A.logz64 = d_logz64;
         A.status = X.status;
-        cf::LinArgs La;
+        cf::LinArgs La{};
         La.descs = A.descs;
-        La.n = A.n;
         La.seqs = d_seqs;
         La.mask = d_mask;
         La.weights = fp64 ? (const void*)eng->lin64.p : (const void*)eng->lin32.p;
@@ -733,13 +816,14 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         La.fails = X.fails;
         const int rgrid = std::min(A.n, cf::kFoldMinBlocks * sms);
         CF_CUDA(cudaMemsetAsync(X.fails, 0, sizeof(int), st));
-        if (fp64) {
-            CF_PHASE(0, (cf::k_lin_inside64<<<A.n, cf::kLinThreads, smem, st>>>(La)));
-            CF_PHASE(0, (cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails)));
-        } else {
-            CF_PHASE(0, (cf::k_lin_inside32<<<A.n, cf::kLinThreads, smem, st>>>(La)));
-            CF_PHASE(0, (cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails)));
-        }
+        cudaEvent_t stop = nullptr;
+        if (X.timer && (rc = X.timer->begin(0, st, &stop))) return rc;
+        if ((rc = launch_lin_inside(P, La, k0, k1, fp64, false, X.lin_streams, st, X.launches))) return rc;
+        if (fp64) cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
+        else cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
+        ++X.launches;
+        CF_CUDA(cudaGetLastError());
+        if (X.timer && (rc = X.timer->end(stop, st))) return rc;
     }
     return CF_OK;
 }
@@ -1056,6 +1140,7 @@ int run_host(cf_engine* eng, Job job, const uint8_t* seqs, const int64_t* offset
     X.arena = eng->arena.p;
     X.status = eng->status.p;
     X.fails = eng->fails.p;
+    X.lin_streams = &eng->lin_streams;
     if ((rc = run_device(eng, job, P, X, eng->seqs.p, d_mask, gamma, d_logz, d_logz64, d_structs, d_post, d_post_offs,
                          st, &sj)))
         return rc;
@@ -1131,6 +1216,7 @@ int cf_engine_destroy(cf_engine* e) {
     e->post_offs.release(); e->status.release(); e->samples.release(); e->seeds.release(); e->stream_idx.release();
     e->bonus.release(); e->counts.release(); e->unpaired.release();
     e->fails.release(); e->lin32.release(); e->lin64.release();
+    e->lin_streams.release();
     if (e->stream) cudaStreamSynchronize(e->stream);   // the stream-ordered frees
 
     if (e->stream_lo) cudaStreamDestroy(e->stream_lo);
@@ -1347,24 +1433,26 @@ extern "C" int cf_grad(cf_engine* e, const uint8_t* seqs, const int64_t* offsets
         d_bonus = e->bonus.p;
     }
     if ((rc = e->counts.ensure((size_t)n * CF_BLOB_LEN)) || (rc = e->unpaired.ensure(std::max<size_t>(nbytes, 1))) ||
-        (rc = e->logz.ensure(n)) || (rc = e->descs.ensure(n)) || (rc = e->status.ensure(2)))
+        (rc = e->logz.ensure(n)) || (rc = e->descs.ensure(n)) || (rc = e->status.ensure(2)) ||
+        (rc = e->fails.ensure((size_t)n + 1)))
         return rc;
     CF_CUDA(cudaMemcpyAsync(e->descs.p, P.descs.data(), sizeof(SeqDesc) * n, cudaMemcpyHostToDevice, st));
     CF_CUDA(cudaMemsetAsync(e->status.p, 0, sizeof(int), st));
     if ((rc = e->arena.ensure((size_t)P.arena_words()))) return rc;
-    const size_t smem = cf::adj_smem_bytes(P.Lmax);
+    const size_t smem = cf::adj_smem_bytes(std::max(P.Lmax, P.lin_Lmax));
+    const size_t out_smem = cf::lin_outside_smem_bytes(P.lin_Lmax);
+    if ((rc = prepare_linear(e, JOB_GRAD, P, &e->lin_streams))) return rc;
     {
         int dev_max = 0;
         CF_CUDA(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
         if (smem > (size_t)dev_max) return fail(CF_EINVAL, "sequence too long for the adjoint kernels");
-        for (const void* k : {(const void*)cf::k_adj_inside, (const void*)cf::k_adj_outside}) {
-            const int rs = raise_smem_limit(k, e->device, std::max<size_t>(smem, 48 * 1024));
-            if (rs) return rs;
-        }
+        const std::pair<const void*, size_t> ks[] = {{(const void*)cf::k_adj_inside, smem}, {(const void*)cf::k_adj_outside, smem},
+                                                     {(const void*)cf::k_lin_outside32, out_smem}};
+        for (const auto& k : ks)
+            if ((rc = raise_smem_limit(k.first, e->device, std::max<size_t>(k.second, 48 * 1024)))) return rc;
     }
-    for (size_t sl = 0; sl + 1 < P.slice_begin.size(); ++sl) {
-        const int k0 = P.slice_begin[sl], k1 = P.slice_begin[sl + 1];
-        cf::FoldArgs A;
+    auto args = [&](int k0, int k1) {
+        cf::FoldArgs A{};
         A.descs = e->descs.p + k0;
         A.n = k1 - k0;
         A.group = 1;
@@ -1374,14 +1462,36 @@ extern "C" int cf_grad(cf_engine* e, const uint8_t* seqs, const int64_t* offsets
         A.blob64 = e->blob64.p;
         A.ws = e->arena.p;
         A.logz = e->logz.p;
-        A.logz64 = nullptr;
-        A.structs = nullptr;
-        A.post_out = nullptr;
-        A.post_offs = nullptr;
-        A.gamma = 0.f;
         A.status = e->status.p;
-        cf::k_adj_inside<<<A.n, cf::kFoldThreads, smem, st>>>(A, d_bonus, P.grad_ckpt);
-        cf::k_adj_outside<<<A.n, cf::kFoldThreads, smem, st>>>(A, d_bonus, P.grad_ckpt, e->counts.p, e->unpaired.p);
+        return A;
+    };
+    auto adjoint = [&](const cf::FoldArgs& A, const int* list) {
+        cf::k_adj_inside<<<A.n, cf::kFoldThreads, smem, st>>>(A, d_bonus, P.grad_ckpt, list);
+        cf::k_adj_outside<<<A.n, cf::kFoldThreads, smem, st>>>(A, d_bonus, P.grad_ckpt, e->counts.p, e->unpaired.p, list);
+    };
+    for (size_t sl = 0; sl + 1 < P.lin_begin.size(); ++sl) {   // sums of products; what leaves their range, in the log domain
+        const cf::FoldArgs A = args(P.lin_begin[sl], P.lin_begin[sl + 1]);
+        cf::LinArgs La{};
+        La.descs = A.descs;
+        La.seqs = A.seqs;
+        La.mask = A.mask;
+        La.weights = e->lin32.p;
+        La.ws = A.ws;
+        La.logz = A.logz;
+        La.bonus = d_bonus;
+        La.counts = e->counts.p;
+        La.unpaired = e->unpaired.p;
+        La.fails = e->fails.p;
+        CF_CUDA(cudaMemsetAsync(e->fails.p, 0, sizeof(int), st));
+        int launches = 0;
+        if ((rc = launch_lin_inside(P, La, P.lin_begin[sl], P.lin_begin[sl + 1], false, true, &e->lin_streams, st, launches)))
+            return rc;
+        cf::k_lin_outside32<<<A.n, cf::kLinOutThreads, out_smem, st>>>(La);
+        adjoint(A, e->fails.p);
+        CF_CUDA(cudaGetLastError());
+    }
+    for (size_t sl = 0; P.n_fold > 0 && sl + 1 < P.slice_begin.size(); ++sl) {
+        adjoint(args(P.slice_begin[sl], P.slice_begin[sl + 1]), nullptr);
         CF_CUDA(cudaGetLastError());
     }
     CF_CUDA(cudaMemcpyAsync(counts_out, e->counts.p, sizeof(double) * n * CF_BLOB_LEN, cudaMemcpyDeviceToHost, st));
@@ -1399,6 +1509,7 @@ struct cf_plan {
     DevBuf<SeqDesc> descs;
     DevBuf<float> arena;
     DevBuf<int> status, fails;
+    LinStreams lin_streams;
     DevBuf<int64_t> post_offs;   // CF_JOB_BPP: sequence b's matrix at sum_{c<b} L_c^2 floats
     PhaseTimer timer;
     int launches = 0;
@@ -1417,12 +1528,10 @@ namespace {
 
 // Shared memory run_device will ask for: set before a stream capture, which
 // then records kernel launches only.
-int plan_prepare_smem(cf_engine* e, Job job, const Plan& P) {
+int plan_prepare_smem(cf_engine* e, Job job, const Plan& P, LinStreams* S) {
     size_t bytes;
     if (!P.lin_begin.empty()) {
-        const bool fp64 = job == JOB_LOGZ64;
-        const int rc = raise_smem_limit(fp64 ? (const void*)cf::k_lin_inside64 : (const void*)cf::k_lin_inside32,
-                                        e->device, std::max<size_t>(cf::lin_inside_smem_bytes(P.lin_Lmax, fp64), 48 * 1024));
+        const int rc = prepare_linear(e, job, P, S);
         if (rc) return rc;
         if (P.n_fold == 0) return CF_OK;
     }
@@ -1506,6 +1615,7 @@ int cf_plan_destroy(cf_plan* p) {
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     p->descs.release(); p->arena.release(); p->status.release(); p->post_offs.release();
     p->fails.release();
+    p->lin_streams.release();
     delete p;
     return CF_OK;
 }
@@ -1522,6 +1632,7 @@ int cf_plan_run(cf_plan* p, const uint8_t* d_seqs, const uint8_t* d_mask, float 
     X.arena = p->arena.p;
     X.status = p->status.p;
     X.fails = p->fails.p;
+    X.lin_streams = &p->lin_streams;
     X.timer = p->timer.on ? &p->timer : nullptr;
     float* lz = p->job == JOB_LOGZ ? static_cast<float*>(d_out) : nullptr;
     double* lz64 = p->job == JOB_LOGZ64 ? static_cast<double*>(d_out) : nullptr;
@@ -1532,7 +1643,7 @@ int cf_plan_run(cf_plan* p, const uint8_t* d_seqs, const uint8_t* d_mask, float 
         const bool hit = p->gexec != nullptr && p->g_seqs == d_seqs && p->g_mask == d_mask && p->g_out == d_out &&
                          p->g_gamma == gamma;
         if (!hit) {   // (re)capture the launches of one run
-            int rc = plan_prepare_smem(p->eng, p->job, p->P);
+            int rc = plan_prepare_smem(p->eng, p->job, p->P, &p->lin_streams);
             if (rc) return rc;
             if (p->gexec) {
                 CF_CUDA(cudaGraphExecDestroy(p->gexec));

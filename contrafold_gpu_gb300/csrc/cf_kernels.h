@@ -83,8 +83,10 @@ size_t plain_smem_bytes(int Lmax);
 
 // Adjoint (cf_adjoint.cu): inside with a soft unpaired bonus (FM2 kept on
 // every ckpt-th diagonal), then the outside with the expected counts folded in.
-__global__ void k_adj_inside(FoldArgs A, const float* bonus, int ckpt);
-__global__ void k_adj_outside(FoldArgs A, const float* bonus, int ckpt, double* counts_out, double* unpaired_out);
+// list (nullable): only the descs it names (cf_linear.h).
+__global__ void k_adj_inside(FoldArgs A, const float* bonus, int ckpt, const int* list);
+__global__ void k_adj_outside(FoldArgs A, const float* bonus, int ckpt, double* counts_out, double* unpaired_out,
+                              const int* list);
 size_t adj_smem_bytes(int Lmax);
 int64_t adj_arena_words(int L, int ckpt);
 int adj_auto_checkpoint(int L);

@@ -17,7 +17,9 @@ namespace cf {
 // 2e-5 there.
 constexpr int kLinMaxLen = 512;
 constexpr int kLinMaxLen64 = 416;   // double: what one CTA's shared memory holds (225 KB)
-constexpr int kLinThreads = 256;
+constexpr int kLinMaxLenGrad = 400;  // the gradient kernel's rings and sums (226 KB)
+constexpr int kLinOutThreads = 512;
+constexpr int kLinSmemMax = 232448;  // shared memory one CTA can have on sm_103a
 
 // Every position costs a factor kLinScale, taken out of log Z again at the
 // end: random sequences gain 0.02 to 0.13 nats a position, so scaled values
@@ -43,17 +45,28 @@ void lin_weights(const double* blob, LinWeights<float>* w);
 void lin_weights(const double* blob, LinWeights<double>* w);
 
 struct LinArgs {
-    const SeqDesc* descs;      // [n], one CTA each
-    int n;
+    const SeqDesc* descs;      // CTA b takes descs[first + b]
+    int first;
     const uint8_t* seqs;
     const uint8_t* mask;       // nullable
     const void* weights;       // LinWeights<R>
     float* ws;                 // arena base
     void* logz;                // R[batch], written at SeqDesc::idx
-    int* fails;                // [0] count, [1 ..] descs indices whose values left the range
+    const float* bonus;        // gradients: unpaired bonus of each position, nullable
+    double* counts;            // [batch][CF_BLOB_LEN]
+    double* unpaired;          // at SeqDesc::seq_off
+    int* fails;                // [0] count, [1 ..] indices into descs whose values left the range
 };
-__global__ void k_lin_inside32(LinArgs A);
-__global__ void k_lin_inside64(LinArgs A);
+struct LinKernel {
+    void (*fn)(LinArgs);
+    int threads;
+};
+// the inside of sequences of up to L nt; train: with bonuses, and the tables the derivatives need
+LinKernel lin_inside_kernel(int L, bool fp64, bool train);
+int lin_class_end(int L, bool fp64);   // sequences up to this length share the launch of an L-nt one
 size_t lin_inside_smem_bytes(int Lmax, bool fp64);
+// gradients: the derivatives, after lin_inside_kernel(train)
+__global__ void k_lin_outside32(LinArgs A);
+size_t lin_outside_smem_bytes(int Lmax);
 
 }  // namespace cf
