@@ -327,7 +327,9 @@ struct Plan {
     bool plain = false;           // reference launch shape (mode 0): cf_plain.cu kernels for BPP/MEA
     bool cta = false;             // persistent CTA-per-sequence fused kernel (batched path)
     bool warp = false;            // persistent warp-per-sequence kernel (batched path)
-    bool cluster = false;         // a thread-block cluster per group (latency of long sequences)
+    bool cluster = false;         // a thread-block cluster per sequence (latency of long sequences)
+    bool lat = false;             // the latency kernels, one sequence on ctas CTAs
+    int ctas = 1;
     bool queue = false;           // dataflow schedule (disabled: never set, see cf_queue.cu)
     int seats = 0;                // its sequences in progress per CTA
     int wgrid = 0;                // its grid
@@ -510,7 +512,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
     // once; between other engines' steady launches that took seconds
     if (eng->shared && sched == 4) sched = 3;
     P.cluster = batched && sched == 4 && (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE);
-    if (P.cluster) P.group = eng->group > 0 ? std::min(cf::kMaxGroup, eng->group) : 1;
+    if (P.cluster) P.group = 1;
     P.queue = batched && sched == 5 && (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE);
     if (P.queue) {
         // sequences in progress per CTA: enough open chunks for the 8 warps on
@@ -592,14 +594,39 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         }
         P.warp = false;   // not even one CTA of warp slots fits: per-sequence kernels, sliced
     }
+    // the latency kernels: one sequence per cluster, or (at most one CTA per SM) per CTA.  Not on a shared device: a
+    // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first
+    int sms = 0;
+    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
+    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= sms &&
+                          (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE));
     P.slice_begin.clear();
     P.slice_words.clear();
     int64_t cur = 0;
     int start = 0;
+    auto words = [&](int k) {
+        const int64_t w = arena_words(job, P.descs[k].L, P.grad_ckpt);
+        return P.lat ? cf::pad32(w) + cf::lat_term_words(P.descs[k].L) : w;
+    };
+    // CTAs a sequence.  Two of a cluster's fit an SM; a cluster of two is only worth its barriers where it spreads over
+    // two SMs.  (GB300, MEA, ms with 1 / 2 / 4 / 8: 1 x 60 nt 1.4 / 1.6 / 1.5 / 1.5, 1 x 400 nt 35 / 28 / 22 / 20, 48 x
+    // 40-400 nt 33 / 27 / 22 / 20, 70 x 200 nt 9.3 / 9.3 / 8.8 / 15, 140 x 200 nt 9.8 / 11 / 17 / 31.)
+    if (P.lat) {
+        P.ctas = P.cluster ? cf::kClusterCtas : 1;
+        if (!P.cluster && P.Lmax > 128)
+            P.ctas = n * 8 <= 2 * sms ? 8 : n * 4 <= 2 * sms ? 4 : n * 2 <= sms ? 2 : 1;
+    }
+    if (P.lat) {   // no room for the longest sequence's terms or codes: the grouped kernels need less
+        int dev_max = 0;
+        CF_CUDA(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, eng->device));
+        bool fits = cf::fold_smem_bytes(P.Lmax, 1, false) + cf::kLatStaticSmem <= (size_t)dev_max;
+        for (int k = 0; k < n && fits; ++k) fits = words(k) <= budget_words;
+        if (!fits) P.lat = P.cluster = false;
+    }
     for (int k = 0; k < n; k += P.group) {
         int64_t gw = 0;
         const int kend = std::min(n, k + P.group);
-        for (int t = k; t < kend; ++t) gw += arena_words(job, P.descs[t].L, P.grad_ckpt);
+        for (int t = k; t < kend; ++t) gw += words(t);
         if (gw > budget_words) return fail(CF_ENOMEM, "sequence group does not fit the arena budget");
         if (cur + gw > budget_words && k > start) {
             P.slice_begin.push_back(start);
@@ -609,7 +636,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         }
         for (int t = k; t < kend; ++t) {
             P.descs[t].ws_off = cur;
-            cur += arena_words(job, P.descs[t].L, P.grad_ckpt);
+            cur += words(t);
         }
     }
     P.slice_begin.push_back(start);
@@ -643,21 +670,26 @@ int ensure_smem(cf_engine* eng, size_t bytes) {
     std::vector<const void*> ks = {(const void*)cf::k_plain_inside32, (const void*)cf::k_plain_outside32,
                                    (const void*)cf::k_plain_posterior32, (const void*)cf::k_plain_mea32,
                                    (const void*)cf::k_inside64, (const void*)cf::k_viterbi64};
-    for (bool wide : {false, true}) {
-        const cf::FoldKernels fk = cf::fold_kernels(wide);
-        for (cf::FoldKernel k : {fk.inside, fk.inside_acc, fk.outside, fk.posterior, fk.mea, fk.fused_mea, fk.fused_bpp,
-                                 fk.fused_mea_shared})
-            ks.push_back((const void*)k);
-    }
+    const cf::FoldKernels fk = cf::fold_kernels();
+    for (cf::FoldKernel k : {fk.inside, fk.inside_acc, fk.outside, fk.posterior, fk.mea, fk.fused_mea, fk.fused_bpp,
+                             fk.fused_mea_shared})
+        ks.push_back((const void*)k);
     for (int mode = 0; mode < 4; ++mode) ks.push_back(cf::warp_kernel(mode));
     for (int mode = 0; mode < 3; ++mode) ks.push_back(cf::cta_kernel(mode));
-    const cf::ClusterKernels ck = cf::cluster_kernels();
-    for (cf::FoldKernel k : {ck.mea, ck.bpp, ck.inside_acc}) ks.push_back((const void*)k);
     for (const void* k : ks) {
         const int rc = raise_smem_limit(k, eng->device, bytes);
         if (rc) return rc;
     }
     eng->smem_optin = bytes;
+    return CF_OK;
+}
+
+int ensure_lat_smem(cf_engine* eng, const Plan& P) {
+    const cf::LatKernels lk = cf::lat_kernels(P.ctas > 1);
+    for (cf::FoldKernel k : {lk.mea, lk.bpp, lk.inside_acc}) {
+        const int rc = raise_smem_limit((const void*)k, eng->device, cf::fold_smem_bytes(P.Lmax, 1, false));
+        if (rc) return rc;
+    }
     return CF_OK;
 }
 
@@ -931,6 +963,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
     const bool fp64 = job == JOB_LOGZ64 || job == JOB_MFE;
     const size_t smem = cf::fold_smem_bytes(P.Lmax, P.group, fp64);
     if ((rc = ensure_smem(eng, std::max(smem, cf::plain_smem_bytes(P.Lmax))))) return rc;
+    if (P.lat && (rc = ensure_lat_smem(eng, P))) return rc;
 
     for (size_t s = 0; s + 1 < P.slice_begin.size(); ++s) {
         const int k0 = P.slice_begin[s], k1 = P.slice_begin[s + 1];
@@ -952,24 +985,26 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         A.status = X.status;
         const int grid = (A.n + P.group - 1) / P.group;
         const dim3 blk(cf::kFoldThreads);
-        // at most one CTA per SM: the wide per-phase kernels (twice the threads on
-        // each diagonal, the latency of small batches of long sequences)
-        int sms = 0;
-        CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
-        // (not on a shared device: a 512-thread CTA waits for an SM with room
-        // for all of it, which other engines' smaller CTAs kept taking first)
-        const bool wide = grid <= sms && !eng->shared;
-        const dim3 blkw(wide ? cf::kFoldThreadsWide : cf::kFoldThreads);
-        const cf::FoldKernels fk = cf::fold_kernels(wide);
-        const cf::FoldKernel k_in = fk.inside, k_inacc = fk.inside_acc, k_out = fk.outside, k_post = fk.posterior,
-                             k_dec = fk.mea;
-        // cluster schedule: every group on kClusterCtas CTAs of one cluster
-        const cf::ClusterKernels ck = cf::cluster_kernels();
-        const dim3 cgrid(grid * cf::kClusterCtas);
+        const cf::FoldKernels fk = cf::fold_kernels();
+        const cf::LatKernels lk = cf::lat_kernels(P.ctas > 1);
+        auto launch_lat = [&](cf::FoldKernel k) {   // a CTA or a cluster per sequence
+            cudaLaunchConfig_t C = {};
+            C.gridDim = dim3(A.n * P.ctas);
+            C.blockDim = dim3(P.ctas > 1 ? cf::kFoldThreads : cf::kLatThreads);
+            C.dynamicSmemBytes = smem;
+            C.stream = st;
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = P.ctas;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            C.attrs = &at;
+            C.numAttrs = P.ctas > 1 ? 1 : 0;
+            return cudaLaunchKernelEx(&C, k, A);
+        };
         switch (job) {
             case JOB_LOGZ:
-                if (P.cluster) CF_PHASE(0, (ck.inside_acc<<<cgrid, blk, smem, st>>>(A)));
-                else CF_PHASE(0, (k_inacc<<<grid, blkw, smem, st>>>(A)));
+                if (P.lat) CF_PHASE(0, CF_CUDA(launch_lat(lk.inside_acc)));
+                else CF_PHASE(0, (fk.inside_acc<<<grid, blk, smem, st>>>(A)));
                 break;
             case JOB_LOGZ64:
                 CF_PHASE(0, (cf::k_inside64<<<grid, blk, smem, st>>>(A)));
@@ -993,26 +1028,27 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
                     }
                     break;
                 }
-                if (P.cluster) {   // fused only: the phases are timed as one
-                    CF_PHASE(0, ((job == JOB_BPP ? ck.bpp : ck.mea)<<<cgrid, blk, smem, st>>>(A)));
+                // fused only: on a cluster the phases are timed as one, one CTA's as the grouped kernels'
+                if (P.cluster || (P.lat && X.timer == nullptr)) {
+                    CF_PHASE(0, CF_CUDA(launch_lat(job == JOB_BPP ? lk.bpp : lk.mea)));
                     break;
                 }
                 if (X.timer == nullptr) {   // one launch for all phases; per-phase kernels when timing
                     const cf::FoldKernel fused = job == JOB_BPP ? fk.fused_bpp
                                                : eng->shared ? fk.fused_mea_shared : fk.fused_mea;
-                    CF_PHASE(0, (fused<<<grid, blkw, smem, st>>>(A)));
+                    CF_PHASE(0, (fused<<<grid, blk, smem, st>>>(A)));
                     break;
                 }
-                CF_PHASE(0, (k_in<<<grid, blkw, smem, st>>>(Ai)));
-                CF_PHASE(1, (k_out<<<grid, blkw, smem, st>>>(A)));
+                CF_PHASE(0, (fk.inside<<<grid, blk, smem, st>>>(Ai)));
+                CF_PHASE(1, (fk.outside<<<grid, blk, smem, st>>>(A)));
                 if (job == JOB_BPP) {
-                    CF_PHASE(2, (k_post<<<grid, blkw, smem, st>>>(A)));
+                    CF_PHASE(2, (fk.posterior<<<grid, blk, smem, st>>>(A)));
                 } else {
                     cf::FoldArgs Ap = A;
                     Ap.post_out = nullptr;
                     Ap.logz = nullptr;
-                    CF_PHASE(2, (k_post<<<grid, blkw, smem, st>>>(Ap)));
-                    CF_PHASE(3, (k_dec<<<grid, blkw, smem, st>>>(A)));
+                    CF_PHASE(2, (fk.posterior<<<grid, blk, smem, st>>>(Ap)));
+                    CF_PHASE(3, (fk.mea<<<grid, blk, smem, st>>>(A)));
                 }
                 break;
             }
@@ -1020,8 +1056,8 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
                 CF_PHASE(0, (cf::k_viterbi64<<<grid, blk, smem, st>>>(A)));
                 break;
             case JOB_SAMPLE: {
-                if (P.cluster) CF_PHASE(0, (ck.inside_acc<<<cgrid, blk, smem, st>>>(A)));
-                else CF_PHASE(0, (k_inacc<<<grid, blkw, smem, st>>>(A)));
+                if (P.lat) CF_PHASE(0, CF_CUDA(launch_lat(lk.inside_acc)));
+                else CF_PHASE(0, (fk.inside_acc<<<grid, blk, smem, st>>>(A)));
                 if (!sj || sj->n_samples <= 0) break;
                 cf::SampleArgs S;
                 S.descs = A.descs;
@@ -1546,6 +1582,10 @@ int plan_prepare_smem(cf_engine* e, Job job, const Plan& P, LinStreams* S) {
     } else {
         const bool fp64 = job == JOB_LOGZ64 || job == JOB_MFE;
         bytes = std::max(cf::fold_smem_bytes(P.Lmax, P.group, fp64), cf::plain_smem_bytes(P.Lmax));
+        if (P.lat) {
+            const int rc = ensure_lat_smem(e, P);
+            if (rc) return rc;
+        }
     }
     return ensure_smem(e, bytes);
 }

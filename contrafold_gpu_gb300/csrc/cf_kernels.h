@@ -20,8 +20,7 @@ constexpr int kFoldMinBlocks = CF_FOLD_MIN_BLOCKS;   // resident CTAs per SM the
 #define CF_FOLD_MIN_BLOCKS_MEA 4
 #endif
 constexpr int kFoldMinBlocksMea = CF_FOLD_MIN_BLOCKS_MEA;
-constexpr int kFoldThreadsWide = 512;   // per-phase fold CTA when the grid has at most one CTA per SM:
-                                        // a long sequence's diagonal spreads over twice the threads
+constexpr int kLatThreads = 512;    // threads of the one-CTA latency kernels (cf_latency.cu)
 constexpr int kMaxGroup = 32;       // sequences per CTA on the batched path
 
 struct FoldArgs {
@@ -42,30 +41,27 @@ struct FoldArgs {
     int* status;               // device status word (CF_OK or an error code)
 };
 
-// FP32 per-phase kernels (k_inside32, k_inside32acc, k_outside32,
-// k_posterior32, k_mea32), instantiated for kFoldThreads and kFoldThreadsWide
-// threads per CTA in cf_fold.cu and reached through fold_kernels().
+// FP32 grouped kernels, kFoldThreads threads per CTA (cf_fold.cu)
 using FoldKernel = void (*)(FoldArgs);
 struct FoldKernels {
     FoldKernel inside, inside_acc, outside, posterior, mea;
     FoldKernel fused_mea, fused_bpp;   // k_fold_group32: all phases of MEA / BPP in one launch
     FoldKernel fused_mea_shared;       // fused MEA at the other kernels' register budget (shared device)
 };
-FoldKernels fold_kernels(bool wide);
-// k_fold_cluster32: one group folded by the kClusterCtas CTAs of a cluster
-// (grid = groups x kClusterCtas, kFoldThreads per CTA)
-constexpr int kClusterCtas = 8;
+FoldKernels fold_kernels();
+// Latency kernels (cf_latency.cu): one sequence on one CTA of kLatThreads, or
+// on the 2 to kClusterCtas CTAs of a cluster.  They need
+// lat_term_words(L) words behind the sequence's arena.
+constexpr int kClusterCtas = 8;   // the largest portable cluster
 #ifndef CF_CLUSTER_CHAIN_PF
-#define CF_CLUSTER_CHAIN_PF 8   // bifurcation-chain pipeline depth in the cluster kernels
+#define CF_CLUSTER_CHAIN_PF 8   // MEA decode's chain pipeline depth in the latency kernels
 #endif
-#ifndef CF_CLUSTER_MIN_BLOCKS
-#define CF_CLUSTER_MIN_BLOCKS 2   // resident CTAs per SM the cluster kernels' registers target
-#endif
-constexpr int kClusterMinBlocks = CF_CLUSTER_MIN_BLOCKS;
-struct ClusterKernels {
+struct LatKernels {
     FoldKernel mea, bpp, inside_acc;
 };
-ClusterKernels cluster_kernels();
+LatKernels lat_kernels(bool cluster);   // kLatThreads threads; kFoldThreads in a cluster's CTAs
+int64_t lat_term_words(int L);
+constexpr int kLatStaticSmem = 18 * 1024;   // at most, beside the grouped kernels' dynamic shared memory
 __global__ void k_inside64(FoldArgs A);
 __global__ void k_viterbi64(FoldArgs A);
 // log-domain logZ of the sequences listed in fails (cf_linear.cu)
