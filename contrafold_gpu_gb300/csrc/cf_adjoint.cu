@@ -168,8 +168,8 @@ __device__ __forceinline__ float single_e(const ParamView<float>& P, const SmemT
     const int l1 = p - i, l2 = j - q;
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
     if (l1 == 0 && l2 == 0) return __fadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
-    const float jB1 = tb->jB[idx4(si, sj1, si1, sj)];
-    const float jB2 = tb->jB[idx4(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p])];
+    const float jB1 = tb->jB(si, sj1, si1, sj);
+    const float jB2 = tb->jB(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p]);
     float snuc = 0.0f;
     if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
     else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_adj_inside(FoldArgs A, const f
                     const float b = __fadd_rn(bon(V.U, i, p), bon(V.U, q, j));
                     part = sr.plus(part, __fadd_rn(__fadd_rn(e, inner), b));
                 }
-                const float jB = sm->tabs.jB[idx4(si, sj1, si1, sj)];
+                const float jB = sm->tabs.jB(si, sj1, si1, sj);
                 float acc = __fadd_rn(__fadd_rn(jB, P.hp(d <= DHP ? d : DHP)), bon(V.U, i, j));
                 acc = sr.plus(acc, warp_lse(part));
                 if (fm2 > CF_HALF32) {
@@ -464,7 +464,7 @@ __device__ __forceinline__ void count_cell(const AdjSmem* sm, const ParamView<fl
         const float fco = V.fco(i, d);
         if (fco > CF_HALF32) {
             const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-            const float jB = sm->tabs.jB[idx4(si, sj1, si1, sj)];
+            const float jB = sm->tabs.jB(si, sj1, si1, sj);
             // single-branch loops: window slot c = (l1, l2), inner pair (p+1, q)
             unsigned long long outer_jB = 0;
             for (int c = lane; c < kWin; c += 32) {

@@ -175,7 +175,7 @@ constexpr int kFexpBins = 10;   // unit bins of -x over [0, 10)
 struct PolyTables {
     float4 lse[8];
     float4 fexp[6];
-    float2 lse_bin[kLseBins];     // {boundary inside the bin or +FLT_MAX, int bits: boundaries below}
+    float2 lse_bin[kLseBins];     // {boundary inside the bin or +FLT_MAX, int bits: boundaries below, in bytes of lse}
     float2 fexp_bin[kFexpBins];   // {-boundary inside the bin or -FLT_MAX, int bits: boundaries above}
 };
 
@@ -213,7 +213,7 @@ __device__ __forceinline__ void load_poly_tables(PolyTables* t) {
                     if (T[i] <= lo) ++base;
                     else if (T[i] < hi) inner = T[i];
                 }
-                t->lse_bin[b] = make_float2(inner, __int_as_float(base));
+                t->lse_bin[b] = make_float2(inner, __int_as_float(base * (int)sizeof(float4)));
             }
         } else if (k < 16 + kLseBins + kFexpBins) {
             const int b = k - 16 - kLseBins;
@@ -283,13 +283,18 @@ __device__ __forceinline__ float lse32(const PolyTables* __restrict__ pt, float 
     return lse32_select(a, b);
 #else
     // the larger and the smaller argument (the reference swaps on a < b; for
-    // the finite inputs here fmaxf / fminf give the same pair)
+    // the finite inputs here fmaxf / fminf give the same pair, and |a - b| the
+    // same rounding as their difference)
     const float hi = fmaxf(a, b);
     const float lo = fminf(a, b);
-    const float d = __fsub_rn(hi, lo);
-    const float2 e = pt->lse_bin[min(__float2int_rz(d), kLseBins - 1)];
-    const int seg = __float_as_int(e.y) + (d >= e.x);
-    const float r = cubic(pt->lse[seg], d);
+    const float d = fabsf(__fsub_rn(a, b));
+    // 8 floor(d) for d < 12, the bin's byte offset: 2^20 + d rounded towards
+    // zero holds floor(8 d) in its low bits.  (A float-to-integer conversion
+    // runs at an eighth of the rate and waits some 20 cycles more.)
+    const int at = __float_as_int(__fadd_rz(fminf(d, 11.5f), 1048576.0f)) & 0x78;
+    const float2 e = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(pt->lse_bin) + at);
+    const int seg = __float_as_int(e.y) + (d >= e.x ? (int)sizeof(float4) : 0);
+    const float r = cubic(*reinterpret_cast<const float4*>(reinterpret_cast<const char*>(pt->lse) + seg), d);
     const float res = __fadd_rn(lo, r);
     // The reference also returns hi when lo is below the zero threshold; for
     // finite inputs that case is covered: lo < -5e29 < hi makes d at least

@@ -384,7 +384,7 @@ __device__ void viterbi_traceback(const SmemTabs<double>* tb, const SeqV& Q, con
         } else if (typ == 1) {
             const double val = T.FC[T.at(i, j)];
             const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-            const double jB = tb->jB[idx4(si, sj1, si1, sj)];
+            const double jB = tb->jB(si, sj1, si1, sj);
             const int d = j - i;
             bool done = fabs(__dadd_rn(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP)), -val)) <= EPS;
             if (!done) {
@@ -403,7 +403,7 @@ __device__ void viterbi_traceback(const SmemTabs<double>* tb, const SeqV& Q, con
                         if (p == i && q == j) {
                             e = __dadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
                         } else {
-                            const double jB2 = tb->jB[idx4(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p])];
+                            const double jB2 = tb->jB(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p]);
                             double snuc = 0.0;
                             if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
                             else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);

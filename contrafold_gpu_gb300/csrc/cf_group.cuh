@@ -45,10 +45,10 @@ template <typename R>
 __device__ __forceinline__ SeqV seq_v(SmemFold<R>* sm, int g) {
     const int cs = code_stride(sm->Lmax), W = pb_words(sm->Lmax);
     unsigned char* base = dyn_smem(sm);
-    const int8_t* s = reinterpret_cast<const int8_t*>(base + (2 * g) * cs);
+    const uint8_t* s = base + (2 * g) * cs;
     const int8_t* pc = reinterpret_cast<const int8_t*>(base + (2 * g + 1) * cs);
     const uint32_t* PB = reinterpret_cast<const uint32_t*>(base + 2 * sm->gcap * cs) + (size_t)g * 4 * W;
-    return SeqV{s, pc, PB, W, sm->L[g]};
+    return SeqV{Codes{s}, pc, PB, W, sm->L[g]};
 }
 
 // Build codes and partner bit sets of the group's sequences (descriptors
@@ -58,7 +58,7 @@ __device__ __forceinline__ void build_group_seqs(SmemFold<R>* sm, const FoldArgs
     const int cs = code_stride(sm->Lmax), W = pb_words(sm->Lmax);
     unsigned char* base = dyn_smem(sm);
     for (int g = 0; g < sm->n; ++g) {
-        int8_t* s = reinterpret_cast<int8_t*>(base + (2 * g) * cs);
+        uint8_t* s = base + (2 * g) * cs;
         int8_t* pc = reinterpret_cast<int8_t*>(base + (2 * g + 1) * cs);
         uint32_t* PB = reinterpret_cast<uint32_t*>(base + 2 * sm->gcap * cs) + (size_t)g * 4 * W;
         build_seq(A.seqs, A.mask, sm->soff[g], sm->L[g], W, s, pc, PB);

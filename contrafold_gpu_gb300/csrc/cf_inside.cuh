@@ -61,20 +61,35 @@ struct Max64 {
 };
 
 // Shared-memory scoring tables for semiring real type R.
+//
+// A window's candidate needs bp of its pair and ScoreJunctionB's sum hc + tm,
+// which depends on the two bases of the pair and one beside each.  Both are
+// stored together by two pair codes (Codes::pair): entry X * 25 + Y with
+// X = (a, c), Y = (d, b) for the pair (a, b), c beside a and d beside b.  In a
+// row of a window one of X and Y is the row's, the other one byte of the
+// sequence, so a candidate reads its scores with one multiply-add and one
+// shared-memory access.
+template <typename R>
+struct alignas(2 * sizeof(R)) JunctionEntry {
+    R bp;   // bp[b][a]
+    R jB;   // hc[a][b] + tm[a][b][c][d]: the reference's ScoreJunctionB sum
+};
 template <typename R>
 struct SmemTabs {
+    JunctionEntry<R> jb[625];
     R blob[CF_BLOB_LEN + 3];
-    R jB[625];   // hc[a][b] + tm[a][b][c][d]: the reference's ScoreJunctionB sum
+    __device__ __forceinline__ R jB(int a, int b, int c, int d) const { return jb[(a * 5 + c) * 25 + d * 5 + b].jB; }
 };
 
 template <typename R>
 __device__ __forceinline__ void load_tabs(SmemTabs<R>* t, const R* __restrict__ g) {
     for (int k = threadIdx.x; k < CF_BLOB_LEN; k += blockDim.x) t->blob[k] = g[k];
     for (int k = threadIdx.x; k < 625; k += blockDim.x) {
-        const int a = k / 125, c = (k / 25) % 5;
-        const R hc = g[CF_OFF_HC + a * 5 + c];
-        const R tm = g[CF_OFF_TM + k];
-        t->jB[k] = hc + tm;   // single rounded add (fp contraction cannot apply)
+        const int a = k / 125, c = (k / 25) % 5, d = (k / 5) % 5, b = k % 5;
+        const R hc = g[CF_OFF_HC + a * 5 + b];
+        const R tm = g[CF_OFF_TM + idx4(a, b, c, d)];
+        t->jb[k].bp = g[CF_OFF_BP + b * 5 + a];
+        t->jb[k].jB = hc + tm;   // single rounded add (fp contraction cannot apply)
     }
 }
 
@@ -147,12 +162,6 @@ __device__ __forceinline__ typename S::Real junctionA_rev(const ParamView<typena
 #endif
 constexpr int kChainPF = CF_CHAIN_PF;
 constexpr int kChainAsync = CF_CHAIN_ASYNC;
-// CF_FLAT_WALK = 1 walks the single-branch windows (inside_B, outside_B,
-// posterior_pair) in flattened lockstep (each lane on its own row sequence),
-// 0 in row lockstep.  Results are identical.
-#ifndef CF_FLAT_WALK
-#define CF_FLAT_WALK 0
-#endif
 // CF_CHAIN_UNROLL = 1 unrolls the asynchronous pipeline over its ring slots
 // (constant slot addresses, more code)
 #ifndef CF_CHAIN_UNROLL
@@ -271,13 +280,21 @@ __device__ __forceinline__ void prefetched_chain(int n, Ld ld, Step step) {
     }
 }
 
+// What a window's candidate loads ahead of its use: its table value and the
+// pair code of its position.
+template <typename R>
+struct Candidate {
+    R v;
+    int code;
+};
+
 // One row of a lockstep window walk (see inside_B): every lane of the group
 // runs `slots` iterations (the largest candidate count among them) and takes
 // the set bits of its own mask, highest first (HI) or lowest first; the
 // table value of the next candidate, `ld(bit)`, is loaded before the current
 // one is used, `use(bit, v)`.  (Two to eight loads ahead measured slower, in
 // the batched and in the cluster kernels alike.)
-template <bool HI, typename R, class Ld, class Use>
+template <bool HI, typename V, class Ld, class Use>
 __device__ __forceinline__ void lockstep_row(uint32_t msk, int slots, Ld ld, Use use) {
     auto take = [&](int& bit) -> bool {
         if (msk == 0u) return false;
@@ -291,12 +308,12 @@ __device__ __forceinline__ void lockstep_row(uint32_t msk, int slots, Ld ld, Use
         return true;
     };
     int bit = 0;
-    R v = R(0);
+    V v{};
     bool h = take(bit);
     if (h) v = ld(bit);
     for (int k = 0; k < slots; ++k) {
         int bn = 0;
-        R vn = R(0);
+        V vn{};
         const bool hn = take(bn);
         if (hn) vn = ld(bn);
         if (h) use(bit, v);
@@ -411,90 +428,52 @@ __device__ __forceinline__ void inside_B(const S& sr, const SmemTabs<typename S:
     const int L = Q.L, m = T.m, d = j - i;
     const R NEG = S::neg(), HALF = S::half();
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-    const R jB = tb->jB[idx4(si, sj1, si1, sj)];
+    const R jB = tb->jB(si, sj1, si1, sj);
     R acc = sr.plus(NEG, S::add(jB, P.hp(d <= DHP ? d : DHP)));
     const int nrows = (d < CMAX ? d : CMAX) + 1;
-    // one single-branch candidate: inner pair (p+1, q) of row l1, table value v
-    auto fold = [&](int l1, int q, R sn0, R sn1, R v) {
-        // no zero-threshold test on v: a visited candidate is a pairable
-        // cell, whose FC always holds its hairpin term, and acc (likewise) is
-        // finite, so a sub-threshold v would leave acc unchanged in any case
-        const int p = i + l1;
-        const int l2 = j - q, a = p + 1;
-        R e;
-        if (l1 == 0 && l2 == 0) {
-            e = S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
-        } else {
-            const int sq = Q.s[q], sa = Q.s[a];
-            const R jB2 = tb->jB[idx4(sq, sa, Q.s[q + 1], Q.s[p])];
-            const R snuc = l2 == 0 ? sn0 : (l2 == 1 ? sn1 : R(0));
-            e = S::add(S::add(S::add(P.cs(l1, l2), P.bp(sa, sq)), jB), jB2);
-            // the reference adds snuc = 0 too; that add is skipped where snuc is 0
-            // for the whole row (l1 >= 2): x + 0 is x except that -0 becomes +0,
-            // which no comparison, log-sum-exp or max can see and later sums keep
-            // only in the sign of a zero (the Viterbi is bound by the FP64 pipe:
-            // one add of six per candidate)
-            if (l1 < 2) e = S::add(e, snuc);
-        }
-        acc = sr.plus(acc, S::add(e, v));
-    };
-#if CF_FLAT_WALK
-    // Flattened lockstep: each lane walks its own candidate sequence (rows
-    // l1 ascending, q descending within a row) and moves to its next row as
-    // soon as its row is exhausted, so a lane idles only once it has no
-    // candidates left -- not at the end of every row, as the row-lockstep
-    // walk does.  The next candidate's table value is loaded before the
-    // current one is folded.
-    int l1 = -1, qlo = 0;
-    uint32_t msk = 0u;
-    R sn0 = R(0), sn1 = R(0);
-    auto next = [&](int& ql1, int& qq, R& q0, R& q1) -> bool {
-        while (msk == 0u) {
-            if (++l1 >= nrows) return false;
-            const int p = i + l1;
-            qlo = (p + 2 > l1 + j - CMAX) ? p + 2 : l1 + j - CMAX;
-            msk = Q.window(p + 1, qlo, j - qlo + 1);
-            sn0 = l1 == 1 ? P.b01(si1) : R(0);
-            sn1 = l1 == 0 ? P.b01(sj) : (l1 == 1 ? P.i11(si1, sj) : R(0));
-        }
-        const int bit = 31 - __clz(msk);
-        msk ^= 1u << bit;
-        ql1 = l1;
-        qq = qlo + bit;
-        q0 = sn0;
-        q1 = sn1;
-        return true;
-    };
-    int cl1 = 0, cq = 0;
-    R c0 = R(0), c1 = R(0), cv = R(0);
-    bool have = next(cl1, cq, c0, c1);
-    if (have) cv = T.FC[tri_off(cq - 2 - (i + cl1), m) + i + cl1 + 1];
-    while (__any_sync(lanes, have)) {
-        int nl1 = 0, nq = 0;
-        R n0 = R(0), n1 = R(0), nv = R(0);
-        const bool hn = have && next(nl1, nq, n0, n1);
-        if (hn) nv = T.FC[tri_off(nq - 2 - (i + nl1), m) + i + nl1 + 1];
-        if (have) fold(cl1, cq, c0, c1, cv);
-        have = hn;
-        cl1 = nl1; cq = nq; c0 = n0; c1 = n1; cv = nv;
-    }
-#else
-    // rows p = i + l1, l1 = 0 .. min(30, d); row q range [qlo, j],
-    // qlo = max(p + 2, l1 + j - 30)
-    const int nr = __reduce_max_sync(lanes, nrows);
-    for (int l1 = 0; l1 < nr; ++l1) {
-        const int p = i + l1;
-        const int qlo = (p + 2 > l1 + j - CMAX) ? p + 2 : l1 + j - CMAX;
-        // the 1-nt bulge and 1x1 terms of this row by l2 = 0, 1 (zero beyond)
-        const R sn0 = l1 == 1 ? P.b01(si1) : R(0);
-        const R sn1 = l1 == 0 ? P.b01(sj) : (l1 == 1 ? P.i11(si1, sj) : R(0));
-        uint32_t msk = l1 < nrows ? Q.window(p + 1, qlo, j - qlo + 1) : 0u;
+    // row p = i + l1; q range [j - C, j] with C = min(d - 2, 30) - l1, so that
+    // candidate `bit` has l2 = C - bit.  FC[p + 1][q - 1] has span x - l2, x =
+    // d - 2 - l1: tri_off(x - l2) = tri_off(x) - l2 (2 (m - x) + 1 + l2) / 2.
+    // `near` rows (l1 < 2) hold the stacking pair and the 1-nt bulge and 1x1
+    // terms; the reference adds a zero for those in the other rows too, which
+    // is skipped: x + 0 is x except that -0 becomes +0, which no comparison,
+    // log-sum-exp or max can see and later sums keep only in the sign of a zero
+    // (the Viterbi is bound by the FP64 pipe: one add of six per candidate).
+    auto row = [&](int l1, auto near) {
+        const int p = i + l1, C = (d - 2 < CMAX ? d - 2 : CMAX) - l1, x = d - 2 - l1;
+        uint32_t msk = l1 < nrows ? Q.window(p + 1, j - C, C + 1) : 0u;
         const int slots = __reduce_max_sync(lanes, __popc(msk));
-        lockstep_row<true, R>(
-            msk, slots, [&](int bit) -> R { return T.FC[tri_off(qlo + bit - 2 - p, m) + p + 1]; },
-            [&](int bit, R v) { fold(l1, qlo + bit, sn0, sn1, v); });
-    }
-#endif
+        if (slots == 0) return;
+        const int at2 = 2 * (tri_off(x, m) + p + 1), step = 2 * (m - x) + 1;
+        const JunctionEntry<R>* jb = tb->jb + (l1 < nrows ? Q.s.pair(p) : 0);
+        const uint8_t* code = Q.s.p + j - C;
+        const R* cs = tb->blob + CF_OFF_CS + l1 * 31;
+        lockstep_row<true, Candidate<R>>(
+            msk, slots,
+            [&](int bit) -> Candidate<R> {
+                const int l2 = C - bit;
+                return {T.FC[(at2 - l2 * (step + l2)) >> 1], code[bit]};
+            },
+            [&](int bit, const Candidate<R>& c) {
+                // no zero-threshold test on the value: a visited candidate is
+                // a pairable cell, whose FC always holds its hairpin term, and
+                // acc (likewise) is finite, so a sub-threshold value would
+                // leave acc unchanged in any case
+                const int l2 = C - bit;
+                const JunctionEntry<R> b = jb[c.code * 25];
+                R e = S::add(S::add(S::add(cs[l2], b.bp), jB), b.jB);
+                if constexpr (near) {
+                    if (l1 == 0)
+                        e = l2 == 0 ? S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj)) : S::add(e, l2 == 1 ? P.b01(sj) : R(0));
+                    else
+                        e = S::add(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sj) : R(0)));
+                }
+                acc = sr.plus(acc, S::add(e, c.v));
+            });
+    };
+    const int nr = __reduce_max_sync(lanes, nrows);
+    for (int l1 = 0; l1 < 2 && l1 < nr; ++l1) row(l1, std::true_type{});
+    for (int l1 = 2; l1 < nr; ++l1) row(l1, std::false_type{});
     if (fm2 > HALF) {
         const R jA = junctionA<S>(P, L, Q, i, j);
         acc = sr.plus(acc, S::add(S::add(S::add(fm2, jA), P.mp()), P.mb()));

@@ -53,7 +53,7 @@ struct ChainTables {
 __device__ __forceinline__ void load_chain_tables(ChainTables* C, const PolyTables* pt) {
     for (int k = threadIdx.x; k < kLseBins; k += blockDim.x) {
         const float2 bin = pt->lse_bin[k];
-        const int seg = __float_as_int(bin.y);
+        const int seg = __float_as_int(bin.y) / (int)sizeof(float4);
         C->below[k] = pt->lse[seg];
         C->above[k] = pt->lse[min(seg + 1, 7)];
         C->edge[k] = bin.x;
@@ -202,7 +202,7 @@ __device__ __forceinline__ void inside_E(const SmemTabs<float>* __restrict__ tb,
     const ParamView<float> P{tb->blob};
     const int m = T.m, d = j - i;
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-    const float jB = tb->jB[idx4(si, sj1, si1, sj)];
+    const float jB = tb->jB(si, sj1, si1, sj);
     // row l1: q from lo(l1) to j
     auto lo = [&](int l1) { return i + 2 + l1 > l1 + j - CMAX ? i + 2 + l1 : l1 + j - CMAX; };
     const uint32_t msk = lane <= (d < CMAX ? d : CMAX) ? Q.window(i + lane + 1, lo(lane), j - lo(lane) + 1) : 0u;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void inside_E(const SmemTabs<float>* __restrict__ tb,
                 e = S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
             } else {
                 const int sq = Q.s[q], sa = Q.s[p + 1];
-                const float jB2 = tb->jB[idx4(sq, sa, Q.s[q + 1], Q.s[p])];
+                const float jB2 = tb->jB(sq, sa, Q.s[q + 1], Q.s[p]);
                 e = S::add(S::add(S::add(P.cs(l1, l2), P.bp(sa, sq)), jB), jB2);
                 if (l1 < 2) {
                     const float sn = l1 == 0 ? (l2 == 1 ? P.b01(sj) : 0.0f)
@@ -235,7 +235,7 @@ __device__ __forceinline__ void inside_F(const S& sr, const SmemTabs<float>* __r
                                          const InTabs<float>& T, int i, int j, float fm2, const TermBuf& B, int cell) {
     const ParamView<float> P{tb->blob};
     const int d = j - i;
-    const float jB = tb->jB[idx4(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j])];
+    const float jB = tb->jB(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j]);
     float acc = sr.plus(CF_NEG32, S::add(jB, P.hp(d <= DHP ? d : DHP)));
     const float* t = B.at(d, cell);
     acc = fold_chain(sr, acc, B.count(d, cell), Stored{t, B.stride});
@@ -378,7 +378,7 @@ __device__ __forceinline__ void outside_E(const SmemTabs<float>* __restrict__ tb
     const int L = Q.L, m = T.m, t = b - a;
     const int sa = Q.s[a], sb1 = Q.s[b + 1], sb2 = Q.s[b + 2];
     const float bp_ab = P.bp(sa, sb1);
-    const float jB2 = tb->jB[idx4(sb1, sa, sb2, Q.s[a - 1])];
+    const float jB2 = tb->jB(sb1, sa, sb2, Q.s[a - 1]);
     const int l1max = (a - 2 < CMAX) ? a - 2 : CMAX;
     const int r1 = CMAX - lane;   // this lane's row: l1 descending
     const int jmax = (b + 1 + CMAX - r1 < L - 1) ? b + 1 + CMAX - r1 : L - 1;
@@ -394,7 +394,7 @@ __device__ __forceinline__ void outside_E(const SmemTabs<float>* __restrict__ tb
         if (l1 == 0 && l2 == 0) {
             e = __fadd_rn(P.bp(si1, sj), P.stack(si, Q.s[j + 1], si1, sj));
         } else {
-            const float jBij = tb->jB[idx4(si, Q.s[j + 1], si1, sj)];
+            const float jBij = tb->jB(si, Q.s[j + 1], si1, sj);
             e = __fadd_rn(__fadd_rn(__fadd_rn(P.cs(l1, l2), bp_ab), jBij), jB2);
             if (l1 < 2) {
                 const float sn = l1 == 0 ? (l2 == 1 ? P.b01(sb2) : 0.0f)

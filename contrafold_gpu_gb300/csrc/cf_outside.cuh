@@ -235,102 +235,56 @@ __device__ __forceinline__ void outside_B(const Lse32& sr, const SmemTabs<float>
         }
     }
     // jB of the inner pair (p+1, q) = (a, b+1): hc[s[q]][s[p+1]] + tm[s[q]][s[p+1]][s[q+1]][s[p]]
-    const float jB2 = tb->jB[idx4(sb1, sa, Q.s[b + 2], Q.s[a - 1])];
+    const float jB2 = tb->jB(sb1, sa, Q.s[b + 2], Q.s[a - 1]);
     const int l1max = (a - 2 < CMAX) ? a - 2 : CMAX;   // i = a-1-l1 >= 1
-    auto rowmask = [&](int l1) -> uint32_t {
-        const int jmax = (b + 1 + CMAX - l1 < L - 1) ? b + 1 + CMAX - l1 : L - 1;
-        return Q.window(a - 1 - l1, b + 2, jmax - b);
-    };
-    // single-branch source (i, j) = (a-1-l1, j) with l2 = j - (b+1)
-    auto src_val = [&](int l1, int j) -> float {
-        const int i = a - 1 - l1;
-        return T.FCo[tri_off(j - i, m) + i];
-    };
-    // the 1-nt bulge and 1x1 terms of row l1 by l2 = 0, 1 (l2 = 1 is j = b+2)
+    // row l1: sources (i, j) = (a - 1 - l1, b + 1 + l2), l2 the mask's bit;
+    // FCo[i][j] has span x + l2, x = t + 2 + l1: tri_off(x + l2) = tri_off(x) +
+    // l2 (2 (m - x) + 1 - l2) / 2.  `near` rows as in inside_B.
     const int sb2 = Q.s[b + 2];
-    auto snuc_row = [&](int l1, float& sn0, float& sn1) {
-        const int si1 = l1 <= l1max ? Q.s[a - l1] : 4;   // rows past this lane's last are empty
-        sn0 = l1 == 1 ? P.b01(si1) : 0.0f;
-        sn1 = l1 == 0 ? P.b01(sb2) : (l1 == 1 ? P.i11(si1, sb2) : 0.0f);
-    };
-    auto source = [&](int l1, int j, float v, float sn0, float sn1) {
-        const int i = a - 1 - l1;
-        if (!(v > CF_HALF32)) return;
-        const int l2 = j - (b + 1);
-        const int si = Q.s[i], si1 = Q.s[i + 1], sj = Q.s[j];
-        float e;
-        if (l1 == 0 && l2 == 0) {
-            e = __fadd_rn(P.bp(si1, sj), P.stack(si, Q.s[j + 1], si1, sj));
-        } else {
-            const float jBij = tb->jB[idx4(si, Q.s[j + 1], si1, sj)];
-            e = __fadd_rn(__fadd_rn(__fadd_rn(P.cs(l1, l2), bp_ab), jBij), jB2);
-            if (l1 < 2) e = __fadd_rn(e, l2 == 0 ? sn0 : (l2 == 1 ? sn1 : 0.0f));   // + 0 skipped (see inside_B)
-        }
-        acc = sr.plus(acc, __fadd_rn(v, e));
-    };
     uint32_t m0 = 0u;
-#if CF_FLAT_WALK
-    // flattened lockstep (see inside_B): rows l1max .. 0 of this lane, within a
-    // row highest j first; row 0 without its stacking source
-    {
-        int l1 = l1max + 1;
-        uint32_t msk = 0u;
-        float sn0 = 0.0f, sn1 = 0.0f;
-        auto next = [&](int& ql1, int& qj, float& q0, float& q1) -> bool {
-            while (msk == 0u) {
-                if (--l1 < 0) return false;
-                msk = rowmask(l1);
-                if (l1 == 0) {
-                    m0 = msk;
-                    msk &= ~1u;   // the stacking source comes after the FM1o term
-                }
-                snuc_row(l1, sn0, sn1);
-            }
-            const int bit = 31 - __clz(msk);
-            msk ^= 1u << bit;
-            ql1 = l1;
-            qj = b + 1 + bit;
-            q0 = sn0;
-            q1 = sn1;
-            return true;
-        };
-        int cl1 = 0, cj = 0;
-        float c0 = 0.0f, c1 = 0.0f, cv = 0.0f;
-        bool have = next(cl1, cj, c0, c1);
-        if (have) cv = src_val(cl1, cj);
-        while (__any_sync(lanes, have)) {
-            int nl1 = 0, nj = 0;
-            float n0 = 0.0f, n1 = 0.0f, nv = 0.0f;
-            const bool hn = have && next(nl1, nj, n0, n1);
-            if (hn) nv = src_val(nl1, nj);
-            if (have) source(cl1, cj, cv, c0, c1);
-            have = hn;
-            cl1 = nl1; cj = nj; c0 = n0; c1 = n1; cv = nv;
-        }
-    }
-#else
-    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
-    for (int l1 = lm; l1 >= 0; --l1) {
-        uint32_t msk = l1 <= l1max ? rowmask(l1) : 0u;
-        if (l1 == 0) {
+    auto row = [&](int l1, auto near) {
+        const int i = a - 1 - l1, x = t + 2 + l1;
+        const int jmax = (b + 1 + CMAX - l1 < L - 1) ? b + 1 + CMAX - l1 : L - 1;
+        const bool mine = l1 <= l1max;
+        uint32_t msk = mine ? Q.window(i, b + 2, jmax - b) : 0u;
+        if (near && l1 == 0) {
             m0 = msk;
             msk &= ~1u;   // the stacking source comes after the FM1o term
         }
         const int slots = __reduce_max_sync(lanes, __popc(msk));
-        float sn0, sn1;
-        snuc_row(l1, sn0, sn1);
-        lockstep_row<true, float>(
-            msk, slots, [&](int bit) { return src_val(l1, b + 1 + bit); },
-            [&](int bit, float v) { source(l1, b + 1 + bit, v, sn0, sn1); });
-    }
-#endif
+        if (slots == 0) return;
+        const int at2 = 2 * (tri_off(x, m) + i), step = 2 * (m - x) + 1;
+        const JunctionEntry<float>* jb = tb->jb + (mine ? Q.s.pair(i) * 25 : 0);
+        const uint8_t* code = Q.s.p + b + 1;
+        const float* cs = tb->blob + CF_OFF_CS + l1 * 31;
+        const int si1 = near && mine ? Q.s[a - l1] : 4;
+        lockstep_row<true, Candidate<float>>(
+            msk, slots,
+            [&](int l2) -> Candidate<float> { return {T.FCo[(at2 + l2 * (step - l2)) >> 1], code[l2]}; },
+            [&](int l2, const Candidate<float>& c) {
+                if (!(c.v > CF_HALF32)) return;
+                float e = __fadd_rn(__fadd_rn(__fadd_rn(cs[l2], bp_ab), jb[c.code].jB), jB2);
+                if constexpr (near) {
+                    if (l1 == 0) e = __fadd_rn(e, l2 == 1 ? P.b01(sb2) : 0.0f);
+                    else e = __fadd_rn(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sb2) : 0.0f));
+                }
+                acc = sr.plus(acc, __fadd_rn(c.v, e));
+            });
+    };
+    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
+    for (int l1 = lm; l1 >= 2; --l1) row(l1, std::false_type{});
+    for (int l1 = lm < 1 ? lm : 1; l1 >= 0; --l1) row(l1, std::true_type{});
     if (l1max >= 0) {
         if (b + 1 < L) {
             const float v = T.FM1o[tri_off(t + 2, m) + a - 1];
             const float jAji = junctionA_rev<Lse32>(P, L, Q, a - 1, b + 1);
             acc = sr.plus(acc, __fadd_rn(__fadd_rn(__fadd_rn(v, jAji), P.mp()), bp_ab));
         }
-        if (m0 & 1u) source(0, b + 1, src_val(0, b + 1), 0.0f, 0.0f);   // stacking: no snuc
+        if (m0 & 1u) {   // the stacking source (a - 1, b + 1)
+            const float v = T.FCo[tri_off(t + 2, m) + a - 1];
+            if (v > CF_HALF32)
+                acc = sr.plus(acc, __fadd_rn(v, __fadd_rn(bp_ab, P.stack(Q.s[a - 1], sb2, sa, sb1))));
+        }
     }
     T.FCo[tri_off(t, m) + a] = acc;
 }
@@ -353,46 +307,25 @@ __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restric
     const int sa = Q.s[a], sb = Q.s[b];
     const float bp_ab = P.bp(sa, sb);
     // jB of the inner pair (p+1, q) = (a, b)
-    const float jB2 = tb->jB[idx4(sb, sa, Q.s[b + 1], Q.s[a - 1])];
+    const float jB2 = tb->jB(sb, sa, Q.s[b + 1], Q.s[a - 1]);
     float post = 0.0f;
     const int l1max = live ? ((a - 2 < CMAX) ? a - 2 : CMAX) : -1;   // i = a-1-l1 >= 1
+    // row l1: sources (i, j) = (a - 1 - l1, b + l2), l2 the mask's bit; FCo[i][j]
+    // has span x + l2, x = b - a + 1 + l1 (addresses as in outside_B)
+    const int sb1 = Q.s[b + 1];
     auto rowmask = [&](int l1) -> uint32_t {
         const int jmax = (b + CMAX - l1 < L - 1) ? b + CMAX - l1 : L - 1;
         return Q.window(a - 1 - l1, b + 1, jmax - b + 1);
-    };
-    // single-branch source (i, j) = (a-1-l1, j), l2 = j - b
-    auto src_val = [&](int l1, int j) -> float {
-        const int i = a - 1 - l1;
-        return T.FCo[tri_off(j - i, m) + i];
-    };
-    // the 1-nt bulge and 1x1 terms of row l1 by l2 = 0, 1 (l2 = 1 is j = b+1)
-    const int sb1 = Q.s[b + 1];
-    auto snuc_row = [&](int l1, float& sn0, float& sn1) {
-        const int si1 = l1 <= l1max ? Q.s[a - l1] : 4;   // rows past this lane's last are empty
-        sn0 = l1 == 1 ? P.b01(si1) : 0.0f;
-        sn1 = l1 == 0 ? P.b01(sb1) : (l1 == 1 ? P.i11(si1, sb1) : 0.0f);
-    };
-    auto source = [&](int l1, int j, float fco, float sn0, float sn1) {
-        const int i = a - 1 - l1;
-        const float outside = __fsub_rn(fco, Z);
-        if (!(outside > CF_HALF32)) return;
-        const int l2 = j - b;
-        const int si = Q.s[i], si1 = Q.s[i + 1], sj = Q.s[j];
-        float e;
-        if (l1 == 0 && l2 == 0) {
-            e = __fadd_rn(__fadd_rn(__fadd_rn(outside, P.bp(si1, sj)), P.stack(si, Q.s[j + 1], si1, sj)), fcin);
-        } else {
-            const float jBij = tb->jB[idx4(si, Q.s[j + 1], si1, sj)];
-            e = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(outside, jBij), P.cs(l1, l2)), fcin), bp_ab), jB2);
-            if (l1 < 2) e = __fadd_rn(e, l2 == 0 ? sn0 : (l2 == 1 ? sn1 : 0.0f));   // + 0 skipped (see inside_B)
-        }
-        post = __fadd_rn(post, fexp32(pt, e));
     };
     // row 0: the stacking source (a-1, b), its multiloop term, then j ascending
     uint32_t m0 = 0u;
     if (l1max >= 0) {
         m0 = rowmask(0);
-        if (m0 & 1u) source(0, b, src_val(0, b), 0.0f, 0.0f);   // stacking: no snuc
+        if (m0 & 1u) {
+            const float out = __fsub_rn(T.FCo[tri_off(b - a + 1, m) + a - 1], Z);
+            if (out > CF_HALF32)
+                post = __fadd_rn(post, fexp32(pt, __fadd_rn(__fadd_rn(__fadd_rn(out, bp_ab), P.stack(Q.s[a - 1], sb1, sa, sb)), fcin)));
+        }
         if (b < L) {
             const float v = T.FM1o[tri_off(b - a + 1, m) + a - 1];
             if (v > CF_HALF32) {
@@ -403,54 +336,34 @@ __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restric
         }
         m0 &= ~1u;
     }
-#if CF_FLAT_WALK
-    // flattened lockstep (see inside_B): rows 0 .. l1max of this lane, within
-    // a row lowest j first
-    {
-        int l1 = 0;
-        uint32_t msk = m0;
-        float sn0 = 0.0f, sn1 = 0.0f;
-        snuc_row(0, sn0, sn1);
-        auto next = [&](int& ql1, int& qj, float& q0, float& q1) -> bool {
-            while (msk == 0u) {
-                if (++l1 > l1max) return false;
-                msk = rowmask(l1);
-                snuc_row(l1, sn0, sn1);
-            }
-            const int bit = __ffs(msk) - 1;
-            msk &= msk - 1u;
-            ql1 = l1;
-            qj = b + bit;
-            q0 = sn0;
-            q1 = sn1;
-            return true;
-        };
-        int cl1 = 0, cj = 0;
-        float c0 = 0.0f, c1 = 0.0f, cv = 0.0f;
-        bool have = next(cl1, cj, c0, c1);
-        if (have) cv = src_val(cl1, cj);
-        while (__any_sync(lanes, have)) {
-            int nl1 = 0, nj = 0;
-            float n0 = 0.0f, n1 = 0.0f, nv = 0.0f;
-            const bool hn = have && next(nl1, nj, n0, n1);
-            if (hn) nv = src_val(nl1, nj);
-            if (have) source(cl1, cj, cv, c0, c1);
-            have = hn;
-            cl1 = nl1; cj = nj; c0 = n0; c1 = n1; cv = nv;
-        }
-    }
-#else
-    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
-    for (int l1 = 0; l1 <= lm; ++l1) {
-        uint32_t msk = l1 == 0 ? m0 : (l1 <= l1max ? rowmask(l1) : 0u);
+    auto row = [&](int l1, auto near) {
+        const int i = a - 1 - l1, x = b - a + 1 + l1;
+        const bool mine = l1 <= l1max;
+        const uint32_t msk = l1 == 0 ? m0 : mine ? rowmask(l1) : 0u;
         const int slots = __reduce_max_sync(lanes, __popc(msk));
-        float sn0, sn1;
-        snuc_row(l1, sn0, sn1);
-        lockstep_row<false, float>(
-            msk, slots, [&](int bit) { return src_val(l1, b + bit); },
-            [&](int bit, float v) { source(l1, b + bit, v, sn0, sn1); });
-    }
-#endif
+        if (slots == 0) return;
+        const int at2 = 2 * (tri_off(x, m) + i), step = 2 * (m - x) + 1;
+        const JunctionEntry<float>* jb = tb->jb + (mine ? Q.s.pair(i) * 25 : 0);
+        const uint8_t* code = Q.s.p + b;
+        const float* cs = tb->blob + CF_OFF_CS + l1 * 31;
+        const int si1 = near && mine ? Q.s[a - l1] : 4;
+        lockstep_row<false, Candidate<float>>(
+            msk, slots,
+            [&](int l2) -> Candidate<float> { return {T.FCo[(at2 + l2 * (step - l2)) >> 1], code[l2]}; },
+            [&](int l2, const Candidate<float>& c) {
+                const float outside = __fsub_rn(c.v, Z);
+                if (!(outside > CF_HALF32)) return;
+                float e = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(outside, jb[c.code].jB), cs[l2]), fcin), bp_ab), jB2);
+                if constexpr (near) {
+                    if (l1 == 0) e = __fadd_rn(e, l2 == 1 ? P.b01(sb1) : 0.0f);
+                    else e = __fadd_rn(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sb1) : 0.0f));
+                }
+                post = __fadd_rn(post, fexp32(pt, e));
+            });
+    };
+    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
+    for (int l1 = 0; l1 <= lm && l1 < 2; ++l1) row(l1, std::true_type{});
+    for (int l1 = 2; l1 <= lm; ++l1) row(l1, std::false_type{});
     if (!live) return 0.0f;
     const float outside = __fsub_rn(T.F5o[b], Z);
     const float f5k = T.F5[a - 1];

@@ -47,7 +47,7 @@ __device__ __forceinline__ void plain_inside_cell(const S& sr, const SmemTabs<ty
     R fc = NEG;
     if (fc_cell) {
         const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-        const R jB = tb->jB[idx4(si, sj1, si1, sj)];
+        const R jB = tb->jB(si, sj1, si1, sj);
         R acc = sr.plus(NEG, S::add(jB, P.hp(d <= DHP ? d : DHP)));
         const int pmax = (i + CMAX < j) ? i + CMAX : j;
         for (int p = i; p <= pmax; ++p) {
@@ -67,7 +67,7 @@ __device__ __forceinline__ void plain_inside_cell(const S& sr, const SmemTabs<ty
                     e = S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
                 } else {
                     const int sq = Q.s[q];
-                    const R jB2 = tb->jB[idx4(sq, sa, Q.s[q + 1], sp)];
+                    const R jB2 = tb->jB(sq, sa, Q.s[q + 1], sp);
                     R snuc = R(0);
                     if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
                     else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);
@@ -175,7 +175,7 @@ __device__ __forceinline__ void plain_outside_cell(const Lse32& sr, const SmemTa
         }
         const float bp_ab = P.bp(sa, sb1);
         // jB of the inner pair (p+1, q) = (a, b+1): hc[s[q]][s[p+1]] + tm[s[q]][s[p+1]][s[q+1]][s[p]]
-        const float jB2 = tb->jB[idx4(sb1, sa, Q.s[b + 2 <= L + 1 ? b + 2 : L + 1], Q.s[a - 1])];
+        const float jB2 = tb->jB(sb1, sa, Q.s[b + 2 <= L + 1 ? b + 2 : L + 1], Q.s[a - 1]);
         for (int l1 = CMAX; l1 >= 0; --l1) {
             const int i = a - 1 - l1;
             if (i < 1) continue;
@@ -195,7 +195,7 @@ __device__ __forceinline__ void plain_outside_cell(const Lse32& sr, const SmemTa
                 if (l1 == 0 && l2 == 0) {
                     e = __fadd_rn(P.bp(si1, sj), P.stack(si, Q.s[j + 1], si1, sj));
                 } else {
-                    const float jBij = tb->jB[idx4(si, Q.s[j + 1], si1, sj)];
+                    const float jBij = tb->jB(si, Q.s[j + 1], si1, sj);
                     float snuc = 0.0f;
                     if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
                     else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);
@@ -235,7 +235,7 @@ __device__ __forceinline__ float plain_posterior_cell(const SmemTabs<float>* __r
     const int sa = Q.s[a], sb = Q.s[b];
     const float bp_ab = P.bp(sa, sb);
     // jB of the inner pair (p+1, q) = (a, b)
-    const float jB2 = tb->jB[idx4(sb, sa, Q.s[b + 1], Q.s[a - 1])];
+    const float jB2 = tb->jB(sb, sa, Q.s[b + 1], Q.s[a - 1]);
     float post = 0.0f;
     for (int l1 = 0; l1 <= CMAX; ++l1) {
         const int i = a - 1 - l1;
@@ -252,7 +252,7 @@ __device__ __forceinline__ float plain_posterior_cell(const SmemTabs<float>* __r
                     if (l1 == 0 && l2 == 0) {
                         e = __fadd_rn(__fadd_rn(__fadd_rn(outside, P.bp(si1, sj)), P.stack(si, Q.s[j + 1], si1, sj)), fcin);
                     } else {
-                        const float jBij = tb->jB[idx4(si, Q.s[j + 1], si1, sj)];
+                        const float jBij = tb->jB(si, Q.s[j + 1], si1, sj);
                         float snuc = 0.0f;
                         if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
                         else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);

@@ -120,7 +120,7 @@ struct QueueCtx {
 
     __device__ __forceinline__ SeqV seq(int s) const {
         unsigned char* b = codes + (size_t)s * Y.seat_bytes;
-        return SeqV{reinterpret_cast<const int8_t*>(b), reinterpret_cast<const int8_t*>(b + Y.cs),
+        return SeqV{Codes{b}, reinterpret_cast<const int8_t*>(b + Y.cs),
                     reinterpret_cast<const uint32_t*>(b + 2 * Y.cs), Y.W, seats[s].D.L};
     }
     __device__ __forceinline__ float* base(int s) const {
@@ -176,7 +176,7 @@ struct QueueCtx {
         if (item >= A.n) return false;
         const SeqDesc D = A.descs[item];
         unsigned char* b = codes + (size_t)s * Y.seat_bytes;
-        build_seq_warp_q(D, reinterpret_cast<int8_t*>(b), reinterpret_cast<int8_t*>(b + Y.cs),
+        build_seq_warp_q(D, b, reinterpret_cast<int8_t*>(b + Y.cs),
                          reinterpret_cast<uint32_t*>(b + 2 * Y.cs));
         if (lane == 0) {
             seats[s].D = D;
@@ -186,16 +186,11 @@ struct QueueCtx {
         return true;
     }
 
-    __device__ __forceinline__ void build_seq_warp_q(const SeqDesc& D, int8_t* s, int8_t* pc, uint32_t* PB) {
+    __device__ __forceinline__ void build_seq_warp_q(const SeqDesc& D, uint8_t* s, int8_t* pc, uint32_t* PB) {
         const int L = D.L;
         for (int t = lane; t < L + 2; t += 32) {
-            int8_t code = 4, p = 4;
-            if (t >= 1 && t <= L) {
-                code = base_code(A.seqs[D.seq_off + t - 1]);
-                p = (A.mask != nullptr && A.mask[D.seq_off + t - 1] != 0) ? (int8_t)5 : code;
-            }
-            s[t] = code;
-            pc[t] = p;
+            s[t] = pair_code(A.seqs, D.seq_off, L, t);
+            pc[t] = t >= 1 && t <= L && A.mask != nullptr && A.mask[D.seq_off + t - 1] != 0 ? (int8_t)5 : (int8_t)(s[t] / 5);
         }
         __syncwarp();
         for (int w = 0; w < Y.W; ++w) {

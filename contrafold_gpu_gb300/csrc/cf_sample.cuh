@@ -116,7 +116,7 @@ __device__ __forceinline__ void enum_fc(const SampleCtx<QV>& X, int i, int j, in
     const QV& Q = X.Q;
     const int L = Q.L, d = j - i;
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-    const float jB = X.tb->jB[idx4(si, sj1, si1, sj)];
+    const float jB = X.tb->jB(si, sj1, si1, sj);
     if (!ch.chunk(lane == 0, __fadd_rn(jB, P.hp(d <= DHP ? d : DHP)), 0)) return;
     const int pmax = (i + CMAX < j) ? i + CMAX : j;
     for (int p = i; p <= pmax; ++p) {
@@ -136,7 +136,7 @@ __device__ __forceinline__ void enum_fc(const SampleCtx<QV>& X, int i, int j, in
                 if (l1 == 0 && l2 == 0) {
                     e = __fadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
                 } else {
-                    const float jB2 = X.tb->jB[idx4(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p])];
+                    const float jB2 = X.tb->jB(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p]);
                     float sn = 0.0f;
                     if (l1 == 0 && l2 == 1) sn = P.b01(sj);
                     else if (l1 == 1 && l2 == 0) sn = P.b01(si1);

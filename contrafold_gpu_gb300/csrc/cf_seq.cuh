@@ -10,12 +10,25 @@ namespace cf {
 // plus one spare word so a funnel shift may read word w+1).
 __host__ __device__ __forceinline__ int pb_words(int Lmax) { return ((Lmax + 2) >> 5) + 2; }
 
+// Base codes of a sequence, one byte a position: the code of the position and
+// of the next one together, s[k] * 5 + s[k + 1] (see SmemTabs).
+struct Codes {
+    const uint8_t* p;
+    __device__ __forceinline__ int pair(int k) const { return p[k]; }
+    __device__ __forceinline__ int operator[](int k) const { return (p[k] * 205) >> 10; }   // / 5, exact below 64
+};
+__device__ __forceinline__ uint8_t pair_code(const uint8_t* __restrict__ seqs, int64_t off, int L, int t) {
+    const int x = t >= 1 && t <= L ? base_code(seqs[off + t - 1]) : 4;
+    const int y = t + 1 >= 1 && t + 1 <= L ? base_code(seqs[off + t]) : 4;
+    return (uint8_t)(x * 5 + y);
+}
+
 // Sequence view: base codes s[0..L+1] (N sentinels), pairing codes pc[0..L+1]
 // (5 = forced unpaired), and for each base c in A C G U the bit set PB[c] of
 // positions b whose pairing code is a canonical partner of c.  pairable(a, b)
 // (canonical and neither forced, cpu.py:186,206) is bit b of PB[pc[a]].
 struct SeqV {
-    const int8_t* s;
+    Codes s;
     const int8_t* pc;
     const uint32_t* PB;   // [4][W]
     int W;
@@ -39,15 +52,10 @@ __device__ __forceinline__ bool partner_code(int c, int x) { return (CANON6 >> (
 // Build s, pc, PB for one sequence (whole CTA).  Position b of PB covers
 // 0 .. L+1; higher bits are zero.
 __device__ __forceinline__ void build_seq(const uint8_t* __restrict__ seqs, const uint8_t* __restrict__ mask,
-                                          int64_t off, int L, int W, int8_t* s, int8_t* pc, uint32_t* PB) {
+                                          int64_t off, int L, int W, uint8_t* s, int8_t* pc, uint32_t* PB) {
     for (int t = threadIdx.x; t < L + 2; t += blockDim.x) {
-        int8_t code = 4, p = 4;
-        if (t >= 1 && t <= L) {
-            code = base_code(seqs[off + t - 1]);
-            p = (mask != nullptr && mask[off + t - 1] != 0) ? (int8_t)5 : code;
-        }
-        s[t] = code;
-        pc[t] = p;
+        s[t] = pair_code(seqs, off, L, t);
+        pc[t] = t >= 1 && t <= L && mask != nullptr && mask[off + t - 1] != 0 ? (int8_t)5 : (int8_t)(s[t] / 5);
     }
     __syncthreads();
     // one warp per 32-position word, four ballots (one per base)

@@ -49,16 +49,11 @@ __host__ __device__ __forceinline__ int warp_region_bytes(int Lmax) {
 }
 
 __device__ __forceinline__ void build_seq_warp(const uint8_t* __restrict__ seqs, const uint8_t* __restrict__ mask,
-                                               int64_t off, int L, int W, int8_t* s, int8_t* pc, uint32_t* PB,
+                                               int64_t off, int L, int W, uint8_t* s, int8_t* pc, uint32_t* PB,
                                                int lane) {
     for (int t = lane; t < L + 2; t += 32) {
-        int8_t code = 4, p = 4;
-        if (t >= 1 && t <= L) {
-            code = base_code(seqs[off + t - 1]);
-            p = (mask != nullptr && mask[off + t - 1] != 0) ? (int8_t)5 : code;
-        }
-        s[t] = code;
-        pc[t] = p;
+        s[t] = pair_code(seqs, off, L, t);
+        pc[t] = t >= 1 && t <= L && mask != nullptr && mask[off + t - 1] != 0 ? (int8_t)5 : (int8_t)(s[t] / 5);
     }
     __syncwarp();
     for (int w = 0; w < W; ++w) {
@@ -234,8 +229,8 @@ __global__ void __launch_bounds__(kWarpThreads, CF_WARP_MIN_BLOCKS) k_fold_warp(
     const int W = pb_words(A.Lmax);
     const int cs = (A.Lmax + 2 + 15) & ~15;
     unsigned char* mine = smem_raw + sizeof(WarpSmemHead) + (size_t)wib * warp_region_bytes(A.Lmax);
-    int8_t* s = reinterpret_cast<int8_t*>(mine);
-    int8_t* pc = s + cs;
+    uint8_t* s = mine;
+    int8_t* pc = reinterpret_cast<int8_t*>(mine + cs);
     uint32_t* PB = reinterpret_cast<uint32_t*>(mine + 2 * cs);
     uint32_t* stack = PB + 4 * W;
     const int64_t slot = (int64_t)blockIdx.x * (kWarpThreads / 32) + wib;
@@ -247,7 +242,7 @@ __global__ void __launch_bounds__(kWarpThreads, CF_WARP_MIN_BLOCKS) k_fold_warp(
         if (item >= A.n) break;
         const SeqDesc D = A.descs[item];
         build_seq_warp(A.seqs, A.mask, D.seq_off, D.L, W, s, pc, PB, lane);
-        const SeqV Q{s, pc, PB, W, D.L};
+        const SeqV Q{Codes{s}, pc, PB, W, D.L};
         fold_one<MODE>(A, sm, D, Q, base, stack, lane);
         __syncwarp();
     }
