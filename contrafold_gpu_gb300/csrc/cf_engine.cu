@@ -142,7 +142,8 @@ struct TuneRow {
 //    13.3k; 60 nt: n=2048 172k vs 186k, n=4096 238k vs 191k);
 //  * sampling of large mixed batches up to 400 nt folds 4 sequences per CTA
 //    (4,096 x U{40..400} x 100 samples: 1.30M samples/s against 1.20M with
-//    the MEA-tuned length table's 2);
+//    the MEA-tuned length table's 2), where that leaves two waves of CTAs
+//    (3,648 sequences on 152 SMs);
 //  * everything else folds grouped (lengths within 25 %: one wave of full
 //    CTAs; mixed: several waves).
 std::vector<TuneRow> default_tuning() {
@@ -153,7 +154,7 @@ std::vector<TuneRow> default_tuning() {
     t[1].max_len = 80; t[1].min_batch = 4096; t[1].uniform = 0; t[1].jobs = lbm; t[1].sched = 1;
     t[2].max_len = 80; t[2].uniform = 0; t[2].jobs = lbm; t[2].sched = 3;
     t[3].max_len = 256; t[3].min_batch = 2048; t[3].uniform = 0; t[3].jobs = lbm; t[3].sched = 1;
-    t[4].max_len = 400; t[4].min_batch = 1024; t[4].uniform = 0; t[4].jobs = 1u << JOB_SAMPLE; t[4].sched = 3;
+    t[4].max_len = 400; t[4].min_batch = 3648; t[4].uniform = 0; t[4].jobs = 1u << JOB_SAMPLE; t[4].sched = 3;
     t[4].group = 4;
     return t;
 }
@@ -462,7 +463,9 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         // CTAs (kFoldMinBlocks per SM) each holding n / slots sequences (200 nt:
         // n=1000 9.9k -> 14.4k, n=3125 15.0k -> 23.9k MEA folds/s against two
         // per CTA); mixed lengths keep several waves so the long sequences' CTAs
-        // do not set the end alone (40-400 nt: 11.8k with 2 per CTA, 6.5k with 9)
+        // do not set the end alone (40-400 nt: 11.8k with 2 per CTA, 6.5k with 9;
+        // 25 samples of 1,024 / 2,048 x 40-400 nt with 1, 2, 4 per CTA: 60 / 117,
+        // 68 / 88, 92 / 118 ms; Viterbi 1,024 x 100-500 nt with 1, 2: 108, 139 ms)
         const int Lmed = n ? (int)(offsets[order[n / 2] + 1] - offsets[order[n / 2]]) : 0;
         int sms = 0;
         CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
@@ -473,7 +476,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         // whole waves: the fewest waves whose groups fit kMaxGroup sequences
         const int waves = std::max(1, (n + cf::kMaxGroup * slots - 1) / (cf::kMaxGroup * slots));
         const int wave_group = std::min(cf::kMaxGroup, std::max(1, (n + waves * slots - 1) / (waves * slots)));
-        const int wave2 = std::min(cf::kMaxGroup, std::max(1, (n + 2 * slots - 1) / (2 * slots)));
+        const int wave2 = std::min(cf::kMaxGroup, std::max(1, n / (2 * slots)));   // two whole waves at least
         P.group = eng->group > 0 ? std::min(cf::kMaxGroup, eng->group)
                                  : uniform ? wave_group : std::min(group_for_length(Lmed), wave2);
     }
@@ -594,11 +597,13 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         }
         P.warp = false;   // not even one CTA of warp slots fits: per-sequence kernels, sliced
     }
-    // the latency kernels: one sequence per cluster, or (at most one CTA per SM) per CTA.  Not on a shared device: a
-    // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first
+    // The latency kernels: a sequence on a cluster or, one after another on an SM, on CTAs of their own.  They win until
+    // the grouped kernels' CTAs fill the device (GB300, MEA, ms, latency / grouped: 200 nt n = 300 20 / 32, 450 29 / 34,
+    // 600 39 / 38; 40-400 nt n = 300 37 / 83, 800 71 / 90, 1,024 89 / 97).  Not on a shared device: a 512-thread CTA
+    // waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
     int sms = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
-    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= sms &&
+    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= (uniform ? 7 * sms / 2 : 6 * sms) &&
                           (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE));
     P.slice_begin.clear();
     P.slice_words.clear();
