@@ -613,10 +613,11 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         const int64_t w = arena_words(job, P.descs[k].L, P.grad_ckpt);
         return P.lat ? cf::pad32(w) + cf::lat_term_words(P.descs[k].L) : w;
     };
+    if (job == JOB_MFE) P.group = 1;   // cf_viterbi.cu: a sequence a CTA, or a cluster
     // CTAs a sequence.  Two of a cluster's fit an SM; a cluster of two is only worth its barriers where it spreads over
     // two SMs.  (GB300, MEA, ms with 1 / 2 / 4 / 8: 1 x 60 nt 1.4 / 1.6 / 1.5 / 1.5, 1 x 400 nt 35 / 28 / 22 / 20, 48 x
     // 40-400 nt 33 / 27 / 22 / 20, 70 x 200 nt 9.3 / 9.3 / 8.8 / 15, 140 x 200 nt 9.8 / 11 / 17 / 31.)
-    if (P.lat) {
+    if (P.lat || (job == JOB_MFE && batched && !eng->shared)) {
         P.ctas = P.cluster ? cf::kClusterCtas : 1;
         if (!P.cluster && P.Lmax > 128)
             P.ctas = n * 8 <= 2 * sms ? 8 : n * 4 <= 2 * sms ? 4 : n * 2 <= sms ? 2 : 1;
@@ -674,7 +675,8 @@ int ensure_smem(cf_engine* eng, size_t bytes) {
     if ((size_t)dev_max < bytes) return fail(CF_EINVAL, "sequence too long for shared-memory staging");
     std::vector<const void*> ks = {(const void*)cf::k_plain_inside32, (const void*)cf::k_plain_outside32,
                                    (const void*)cf::k_plain_posterior32, (const void*)cf::k_plain_mea32,
-                                   (const void*)cf::k_inside64, (const void*)cf::k_viterbi64};
+                                   (const void*)cf::k_inside64, (const void*)cf::k_viterbi64,
+                                   (const void*)cf::k_viterbi_cluster64};
     const cf::FoldKernels fk = cf::fold_kernels();
     for (cf::FoldKernel k : {fk.inside, fk.inside_acc, fk.outside, fk.posterior, fk.mea, fk.fused_mea, fk.fused_bpp,
                              fk.fused_mea_shared})
@@ -1058,7 +1060,8 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
                 break;
             }
             case JOB_MFE:
-                CF_PHASE(0, (cf::k_viterbi64<<<grid, blk, smem, st>>>(A)));
+                if (P.ctas > 1) CF_PHASE(0, CF_CUDA(launch_lat(cf::k_viterbi_cluster64)));
+                else CF_PHASE(0, (cf::k_viterbi64<<<grid, blk, smem, st>>>(A)));
                 break;
             case JOB_SAMPLE: {
                 if (P.lat) CF_PHASE(0, CF_CUDA(launch_lat(lk.inside_acc)));

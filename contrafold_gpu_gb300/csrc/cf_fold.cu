@@ -1,5 +1,5 @@
-// cf_fold.cu -- fold kernels: inside (FP32 / FP64 / Viterbi), outside,
-// posterior, MEA decode, Viterbi traceback.
+// cf_fold.cu -- fold kernels: inside (FP32 / FP64), outside, posterior, MEA
+// decode.
 //
 // Scheduling: a CTA owns a GROUP of sequences (group size 1 is the plain
 // one-sequence-per-block path of gpu.py:508; larger groups are the batched
@@ -95,8 +95,6 @@ template <>
 __device__ __forceinline__ LseAcc32 make_sr<LseAcc32>(const PolyTables*) { return LseAcc32{}; }
 template <>
 __device__ __forceinline__ Lse64 make_sr<Lse64>(const PolyTables*) { return Lse64{}; }
-template <>
-__device__ __forceinline__ Max64 make_sr<Max64>(const PolyTables*) { return Max64{}; }
 
 template <class S, class Team = CtaTeam>
 __device__ __forceinline__ void inside_group(SmemFold<typename S::Real>* sm, const FoldArgs& A, const Team tm = Team{}) {
@@ -333,164 +331,6 @@ const void* cta_kernel(int mode) {
         case kCtaLogZ: return (const void*)k_fold_cta<kCtaLogZ>;
         case kCtaMea: return (const void*)k_fold_cta<kCtaMea>;
         default: return (const void*)k_fold_cta<kCtaBpp>;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Viterbi: max-plus inside in FP64, then the reference's EPS first-match
-// traceback (cpu.py:396-501), one thread per sequence.
-// ---------------------------------------------------------------------------
-__device__ void viterbi_traceback(const SmemTabs<double>* tb, const SeqV& Q, const InTabs<double>& T,
-                                  int* st, char* out, int* status) {
-    const ParamView<double> P{tb->blob};
-    const int L = Q.L;
-    const double EPS = 1e-6, HALF = CF_HALF64;
-    const int cap = 4 * L + 16;
-    int *st_t = st, *st_i = st + cap, *st_j = st + 2 * cap;
-    int sp = 0;
-#define VPUSH(tt, ii, jj)                                   \
-    do {                                                    \
-        if (sp >= cap) { atomicExch(status, CF_EDEVICE); return; } \
-        st_t[sp] = (tt); st_i[sp] = (ii); st_j[sp] = (jj); ++sp; \
-    } while (0)
-    VPUSH(0, 0, L);
-    while (sp > 0) {
-        --sp;
-        const int typ = st_t[sp], i = st_i[sp], j = st_j[sp];
-        if (typ == 0) {
-            if (j == 0) continue;
-            const double val = T.F5[j];
-            bool done = false;
-            if (T.F5[j - 1] > HALF && fabs(__dadd_rn(__dadd_rn(T.F5[j - 1], P.eu()), -val)) <= EPS) {
-                VPUSH(0, 0, j - 1);
-                done = true;
-            }
-            if (!done) {
-                for (int k = 0; k < j; ++k) {
-                    if (!Q.pairable(k + 1, j)) continue;
-                    const double fcin = T.FC[T.at(k + 1, j - 1)];
-                    if (!(fcin > HALF) || !(T.F5[k] > HALF)) continue;
-                    const double jA = junctionA_rev<Max64>(P, L, Q, k, j);
-                    const double v = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(T.F5[k], fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[j])), jA);
-                    if (fabs(__dadd_rn(v, -val)) <= EPS) {
-                        out[k] = '(';
-                        out[j - 1] = ')';
-                        VPUSH(1, k + 1, j - 1);
-                        VPUSH(0, 0, k);
-                        break;
-                    }
-                }
-            }
-        } else if (typ == 1) {
-            const double val = T.FC[T.at(i, j)];
-            const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
-            const double jB = tb->jB(si, sj1, si1, sj);
-            const int d = j - i;
-            bool done = fabs(__dadd_rn(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP)), -val)) <= EPS;
-            if (!done) {
-                const int pmax = (i + CMAX < j) ? i + CMAX : j;
-                for (int p = i; p <= pmax && !done; ++p) {
-                    const int l1 = p - i;
-                    int qmin = p + 2;
-                    const int alt = l1 + j - CMAX;
-                    if (alt > qmin) qmin = alt;
-                    for (int q = j; q >= qmin; --q) {
-                        const int l2 = j - q;
-                        if (!Q.pairable(p + 1, q)) continue;
-                        const double inner = T.FC[T.at(p + 1, q - 1)];
-                        if (!(inner > HALF)) continue;
-                        double e;
-                        if (p == i && q == j) {
-                            e = __dadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
-                        } else {
-                            const double jB2 = tb->jB(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p]);
-                            double snuc = 0.0;
-                            if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
-                            else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);
-                            else if (l1 == 1 && l2 == 1) snuc = P.i11(si1, sj);
-                            e = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(P.cs(l1, l2), P.bp(Q.s[p + 1], Q.s[q])), jB), jB2), snuc);
-                        }
-                        if (fabs(__dadd_rn(__dadd_rn(e, inner), -val)) <= EPS) {
-                            out[p] = '(';
-                            out[q - 1] = ')';
-                            VPUSH(1, p + 1, q - 1);
-                            done = true;
-                            break;
-                        }
-                    }
-                }
-            }
-            if (!done) {
-                const double jA = junctionA<Max64>(P, L, Q, i, j);
-                for (int k = i + 1; k < j; ++k) {
-                    const double f1 = T.FM1[T.at(i, k)], fm = T.FM[T.at(k, j)];
-                    if (f1 > HALF && fm > HALF &&
-                        fabs(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f1, fm), jA), P.mp()), P.mb()), -val)) <= EPS) {
-                        VPUSH(3, i, k);
-                        VPUSH(2, k, j);
-                        break;
-                    }
-                }
-            }
-        } else if (typ == 2) {
-            const double val = T.FM[T.at(i, j)];
-            bool done = false;
-            for (int k = i + 1; k < j; ++k) {
-                const double f1 = T.FM1[T.at(i, k)], fm = T.FM[T.at(k, j)];
-                if (f1 > HALF && fm > HALF && fabs(__dadd_rn(__dadd_rn(f1, fm), -val)) <= EPS) {
-                    VPUSH(3, i, k);
-                    VPUSH(2, k, j);
-                    done = true;
-                    break;
-                }
-            }
-            const double prev = T.FM[T.at(i, j - 1)];
-            if (!done && prev > HALF && fabs(__dadd_rn(__dadd_rn(prev, P.mu()), -val)) <= EPS) {
-                VPUSH(2, i, j - 1);
-                done = true;
-            }
-            const double f1 = T.FM1[T.at(i, j)];
-            if (!done && f1 > HALF && fabs(__dadd_rn(f1, -val)) <= EPS) VPUSH(3, i, j);
-        } else {
-            const double val = T.FM1[T.at(i, j)];
-            bool done = false;
-            if (Q.pairable(i + 1, j)) {
-                const double fin = T.FC[T.at(i + 1, j - 1)];
-                if (fin > HALF) {
-                    const double jAji = junctionA_rev<Max64>(P, L, Q, i, j);
-                    const double v = __dadd_rn(__dadd_rn(__dadd_rn(fin, jAji), P.mp()), P.bp(Q.s[i + 1], Q.s[j]));
-                    if (fabs(__dadd_rn(v, -val)) <= EPS) {
-                        out[i] = '(';
-                        out[j - 1] = ')';
-                        VPUSH(1, i + 1, j - 1);
-                        done = true;
-                    }
-                }
-            }
-            const double ext = T.FM1[T.at(i + 1, j)];
-            if (!done && ext > HALF && fabs(__dadd_rn(__dadd_rn(ext, P.mu()), -val)) <= EPS) VPUSH(3, i + 1, j);
-        }
-    }
-#undef VPUSH
-}
-
-__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_viterbi64(FoldArgs A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    auto* sm = reinterpret_cast<SmemFold<double>*>(smem_raw);
-    setup_group(sm, A, A.blob64);
-    inside_group<Max64>(sm, A);
-    for (int g = 0; g < sm->n; ++g) {
-        const int L = sm->L[g];
-        char* out = A.structs + sm->soff[g];
-        for (int t = threadIdx.x; t < L; t += blockDim.x) out[t] = '.';
-    }
-    __syncthreads();
-    for (int g = tb_index(); g < sm->n; g += blockDim.x) {   // tracebacks dealt over the warps first
-        const SeqV Q = seq_v(sm, g);
-        const InTabs<double> T = in_view<double>(A, sm->ws[g], Q.L).T;
-        const Arena64 ar = arena64(Q.L);
-        int* st = reinterpret_cast<int*>(A.ws + sm->ws[g] + ar.stack);   // stack offset is in 4-byte words
-        viterbi_traceback(&sm->tabs, Q, T, st, A.structs + sm->soff[g], A.status);
     }
 }
 

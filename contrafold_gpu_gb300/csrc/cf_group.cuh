@@ -311,4 +311,52 @@ __device__ __forceinline__ void mea_group(SmemFold<float>* sm, const FoldArgs& A
     tm.sync();
 }
 
+// ---------------------------------------------------------------------------
+// One sequence on a team, warps taking items of unlike kinds (cf_latency.cu,
+// cf_viterbi.cu)
+// ---------------------------------------------------------------------------
+constexpr int kWindowMax = (CMAX + 1) * (CMAX + 2) / 2;   // interior loops of one cell at most
+
+__device__ __forceinline__ int warp_exclusive(int v, int lane, int& total) {
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    total = __shfl_sync(0xffffffffu, x, 31);
+    return x - v;
+}
+
+// The candidates of a cell in the order of its rows: every lane lists its
+// row's (mask msk, packed l1 | bit << 5, highest bit first) behind the rows
+// before it.  Returns how many.
+__device__ __forceinline__ int window_list(uint32_t msk, int l1, uint16_t* list, int lane) {
+    int total;
+    int at = warp_exclusive(__popc(msk), lane, total);
+    while (msk) {
+        const int bit = 31 - __clz(msk);
+        msk ^= 1u << bit;
+        list[at++] = (uint16_t)(l1 | bit << 5);
+    }
+    __syncwarp();
+    return total;
+}
+
+// Claims the items of one step: item() runs for every index of this CTA's share
+template <typename R, class Team, class Item>
+__device__ __forceinline__ void run_items(SmemFold<R>* sm, const Team& tm, int step, int total, Item item) {
+    int* ctr = &sm->step_ctr[step & 1];
+    if (threadIdx.x == 0) sm->step_ctr[(step & 1) ^ 1] = 0;
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(ctr, 1);
+        q = __shfl_sync(0xffffffffu, q, 0) * tm.size() + tm.rank();
+        if (q >= total) break;
+        item(q, lane);
+    }
+    tm.sync();
+}
+
 }  // namespace cf

@@ -63,7 +63,8 @@ LatKernels lat_kernels(bool cluster);   // kLatThreads threads; kFoldThreads in 
 int64_t lat_term_words(int L);
 constexpr int kLatStaticSmem = 18 * 1024;   // at most, beside the grouped kernels' dynamic shared memory
 __global__ void k_inside64(FoldArgs A);
-__global__ void k_viterbi64(FoldArgs A);
+__global__ void k_viterbi64(FoldArgs A);           // one sequence a CTA ...
+__global__ void k_viterbi_cluster64(FoldArgs A);   // ... or a cluster (cf_viterbi.cu)
 // log-domain logZ of the sequences listed in fails (cf_linear.cu)
 __global__ void k_inside_redo32(FoldArgs A, const int* fails);
 __global__ void k_inside_redo64(FoldArgs A, const int* fails);

@@ -22,7 +22,7 @@
 namespace cf {
 namespace {
 
-constexpr int kTermRows = (CMAX + 1) * (CMAX + 2) / 2;   // interior loops of one cell at most
+constexpr int kTermRows = kWindowMax;
 
 // Interior-loop terms of two diagonals: terms[parity][k][cell], counts[parity][cell]
 struct TermBuf {
@@ -154,32 +154,13 @@ __device__ __forceinline__ float fold_chain(const S& sr, float acc, int n, Src s
     return acc;
 }
 
-__device__ __forceinline__ int warp_exclusive(int v, int lane, int& total) {
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
-
-// The candidates of a cell in order: every lane lists its row's (packed
-// l1 | bit << 5, highest bit first) behind the rows before it, then the warp
-// takes them 32 at a time, so that all lanes evaluate and up to four loads a
-// lane are in flight (a row a lane, in place: 8,000 cycles a cell at 400 nt).
+// Evaluates a cell's candidates (window_list) 32 at a time, four loads a lane
+// in flight, and stores their terms in order.  (A row a lane, in place, cost
+// 8,000 cycles a cell at 400 nt, this 5,000.)
 template <class Val, class Term>
 __device__ __forceinline__ int eval_terms(uint32_t msk, int l1, uint16_t* list, float* out, int stride, int lane, Val val,
                                           Term term) {
-    int total;
-    int at = warp_exclusive(__popc(msk), lane, total);
-    while (msk) {
-        const int bit = 31 - __clz(msk);
-        msk ^= 1u << bit;
-        list[at++] = (uint16_t)(l1 | bit << 5);
-    }
-    __syncwarp();
+    const int total = window_list(msk, l1, list, lane);
     for (int k0 = lane; k0 < total; k0 += 128) {
         int c[4];
         float v[4];
@@ -307,22 +288,6 @@ __device__ __forceinline__ float exterior_sum(const S& sr, float acc, int n, flo
         __syncwarp();
     }
     return acc;
-}
-
-// Claims the items of one step: item() runs for every index of this CTA's share
-template <class Team, class Item>
-__device__ __forceinline__ void run_items(SmemFold<float>* sm, const Team& tm, int step, int total, Item item) {
-    int* ctr = &sm->step_ctr[step & 1];
-    if (threadIdx.x == 0) sm->step_ctr[(step & 1) ^ 1] = 0;
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        int q = 0;
-        if (lane == 0) q = atomicAdd(ctr, 1);
-        q = __shfl_sync(0xffffffffu, q, 0) * tm.size() + tm.rank();
-        if (q >= total) break;
-        item(q, lane);
-    }
-    tm.sync();
 }
 
 template <class S, class Team>

@@ -1,0 +1,322 @@
+// cf_viterbi.cu -- Viterbi: max-plus inside in FP64, then the reference's EPS
+// first-match traceback (cpu.py:302-501).
+//
+// A maximum does not depend on the order of its candidates, so nothing of a
+// cell is serial: per diagonal one warp takes the interior loops of a pairable
+// cell (candidates listed, 32 evaluated at a time, a butterfly), a warp takes a
+// sixth of the multiloop splits of 32 cells, one the exterior recurrence's next
+// step, and after a barrier a thread a cell joins them.  Each candidate is the
+// reference's sum, rounded as there, so tables are its tables.
+//
+// The FP64 pipe bounds the fold of a full device (two adds or compares a cycle
+// and SM): a window candidate is five adds and a compare, a split two.  The
+// grouped kernel evaluated windows in lockstep, a cell a lane, and kept 46 % of
+// the lanes busy there; a listed window keeps them all.
+#include "cf_group.cuh"
+
+namespace cf {
+namespace {
+
+constexpr int kVitParts = 6;   // of a cell's splits; their maxima lie in the traceback stack's place
+constexpr int kVitWarps = kFoldThreads / 32;
+
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Largest interior-loop candidate of cell (i, j) (inside_B's terms).
+__device__ __forceinline__ double window_max(const SmemTabs<double>* __restrict__ tb, const SeqV& Q,
+                                             const InTabs<double>& T, int i, int j, uint16_t* list, int lane) {
+    const ParamView<double> P{tb->blob};
+    const int m = T.m, d = j - i;
+    const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
+    const double jB = tb->jB(si, sj1, si1, sj);
+    // row l1: q from j - C(l1) to j
+    const int C0 = d - 2 < CMAX ? d - 2 : CMAX;
+    const uint32_t msk = lane <= C0 ? Q.window(i + lane + 1, j - C0 + lane, C0 - lane + 1) : 0u;
+    const int total = window_list(msk, lane, list, lane);
+    double best = CF_NEG64;
+    for (int k0 = lane; k0 < total; k0 += 128) {
+        int c[4];
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = list[min(k0 + 32 * u, total - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int l1 = c[u] & 31, l2 = C0 - l1 - (c[u] >> 5);
+            v[u] = T.FC[tri_off(d - 2 - l1 - l2, m) + i + l1 + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int l1 = c[u] & 31, l2 = C0 - l1 - (c[u] >> 5);
+            const JunctionEntry<double> b = tb->jb[Q.s.pair(j - l2) * 25 + Q.s.pair(i + l1)];
+            double e;
+            if (l1 + l2 == 0) {
+                e = __dadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
+            } else {
+                e = __dadd_rn(__dadd_rn(__dadd_rn(P.cs(l1, l2), b.bp), jB), b.jB);
+                if (l1 < 2 && l2 < 2)   // 1-nt bulges and 1x1 (the zero that other loops add changes no maximum)
+                    e = __dadd_rn(e, l1 == 0 ? P.b01(sj) : l2 == 0 ? P.b01(si1) : P.i11(si1, sj));
+            }
+            best = fmax(best, __dadd_rn(e, v[u]));
+        }
+    }
+    __syncwarp();
+    return warp_max(best);
+}
+
+// Warp 0's traceback: a state's candidates in the reference's order, 32 at a
+// time; the first that matches the state's value within EPS is taken.
+__device__ void viterbi_traceback(const SmemTabs<double>* tb, const SeqV& Q, const InTabs<double>& T, int* st, char* out,
+                                  int* status, int lane) {
+    const ParamView<double> P{tb->blob};
+    const int L = Q.L;
+    const double EPS = 1e-6, HALF = CF_HALF64;
+    const int cap = 4 * L + 16;
+    int *st_t = st, *st_i = st + cap, *st_j = st + 2 * cap;
+    int sp = 0;
+    bool full = false;
+    auto push = [&](int t, int i, int j) {
+        if (sp >= cap) {
+            full = true;
+            return;
+        }
+        if (lane == 0) {
+            st_t[sp] = t;
+            st_i[sp] = i;
+            st_j[sp] = j;
+        }
+        ++sp;
+    };
+    auto pair = [&](int a, int b) {
+        if (lane == 0) {
+            out[a - 1] = '(';
+            out[b - 1] = ')';
+        }
+    };
+    // first k in [lo, hi) whose candidate matches, or -1
+    auto first = [&](int lo, int hi, auto match) {
+        for (int k0 = lo; k0 < hi; k0 += 32) {
+            const int k = k0 + lane;
+            const unsigned hit = __ballot_sync(0xffffffffu, k < hi && match(k));
+            if (hit) return k0 + __ffs(hit) - 1;
+        }
+        return -1;
+    };
+    push(0, 0, L);
+    while (sp > 0 && !full) {
+        --sp;
+        __syncwarp();
+        const int typ = st_t[sp], i = st_i[sp], j = st_j[sp];
+        __syncwarp();
+        auto near = [&](double v, double val) { return fabs(__dadd_rn(v, -val)) <= EPS; };
+        if (typ == 0) {
+            if (j == 0) continue;
+            const double val = T.F5[j], prev = T.F5[j - 1];
+            if (prev > HALF && near(__dadd_rn(prev, P.eu()), val)) {
+                push(0, 0, j - 1);
+                continue;
+            }
+            const int k = first(0, j, [&](int k) {
+                if (!Q.pairable(k + 1, j)) return false;
+                const double fcin = T.FC[T.at(k + 1, j - 1)], f5k = T.F5[k];
+                if (!(fcin > HALF) || !(f5k > HALF)) return false;
+                const double jA = junctionA_rev<Max64>(P, L, Q, k, j);
+                return near(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[j])), jA), val);
+            });
+            if (k >= 0) {
+                pair(k + 1, j);
+                push(1, k + 1, j - 1);
+                push(0, 0, k);
+            }
+        } else if (typ == 1) {
+            const double val = T.FC[T.at(i, j)];
+            const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
+            const double jB = tb->jB(si, sj1, si1, sj);
+            const int d = j - i;
+            if (near(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP)), val)) continue;
+            bool done = false;
+            const int pmax = (i + CMAX < j) ? i + CMAX : j;
+            for (int p = i; p <= pmax && !done; ++p) {   // a row of the window: q = j - lane
+                const int l1 = p - i, q = j - lane, l2 = lane;
+                const int qmin = p + 2 > l1 + j - CMAX ? p + 2 : l1 + j - CMAX;
+                bool hit = false;
+                if (q >= qmin && Q.pairable(p + 1, q)) {
+                    const double inner = T.FC[T.at(p + 1, q - 1)];
+                    if (inner > HALF) {
+                        double e;
+                        if (l1 == 0 && l2 == 0) {
+                            e = __dadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
+                        } else {
+                            const double jB2 = tb->jB(Q.s[q], Q.s[p + 1], Q.s[q + 1], Q.s[p]);
+                            double snuc = 0.0;
+                            if (l1 == 0 && l2 == 1) snuc = P.b01(sj);
+                            else if (l1 == 1 && l2 == 0) snuc = P.b01(si1);
+                            else if (l1 == 1 && l2 == 1) snuc = P.i11(si1, sj);
+                            e = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(P.cs(l1, l2), P.bp(Q.s[p + 1], Q.s[q])), jB), jB2), snuc);
+                        }
+                        hit = near(__dadd_rn(e, inner), val);
+                    }
+                }
+                const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                if (hits) {
+                    const int b = j - (__ffs(hits) - 1);
+                    pair(p + 1, b);
+                    push(1, p + 1, b - 1);
+                    done = true;
+                }
+            }
+            if (done) continue;
+            const double jA = junctionA<Max64>(P, L, Q, i, j);
+            const int k = first(i + 1, j, [&](int k) {
+                const double f1 = T.FM1[T.at(i, k)], fm = T.FM[T.at(k, j)];
+                return f1 > HALF && fm > HALF &&
+                       near(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f1, fm), jA), P.mp()), P.mb()), val);
+            });
+            if (k >= 0) {
+                push(3, i, k);
+                push(2, k, j);
+            }
+        } else if (typ == 2) {
+            const double val = T.FM[T.at(i, j)];
+            const int k = first(i + 1, j, [&](int k) {
+                const double f1 = T.FM1[T.at(i, k)], fm = T.FM[T.at(k, j)];
+                return f1 > HALF && fm > HALF && near(__dadd_rn(f1, fm), val);
+            });
+            if (k >= 0) {
+                push(3, i, k);
+                push(2, k, j);
+                continue;
+            }
+            const double prev = T.FM[T.at(i, j - 1)], f1 = T.FM1[T.at(i, j)];
+            if (prev > HALF && near(__dadd_rn(prev, P.mu()), val)) push(2, i, j - 1);
+            else if (f1 > HALF && near(f1, val)) push(3, i, j);
+        } else {
+            const double val = T.FM1[T.at(i, j)];
+            if (Q.pairable(i + 1, j)) {
+                const double fin = T.FC[T.at(i + 1, j - 1)];
+                if (fin > HALF) {
+                    const double jAji = junctionA_rev<Max64>(P, L, Q, i, j);
+                    if (near(__dadd_rn(__dadd_rn(__dadd_rn(fin, jAji), P.mp()), P.bp(Q.s[i + 1], Q.s[j])), val)) {
+                        pair(i + 1, j);
+                        push(1, i + 1, j - 1);
+                        continue;
+                    }
+                }
+            }
+            const double ext = T.FM1[T.at(i + 1, j)];
+            if (ext > HALF && near(__dadd_rn(ext, P.mu()), val)) push(3, i + 1, j);
+        }
+    }
+    if (full && lane == 0) atomicExch(status, CF_EDEVICE);
+}
+
+template <class Team>
+__device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, int gi) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto* sm = reinterpret_cast<SmemFold<double>*>(smem_raw);
+    __shared__ uint16_t lists[kVitWarps][kWindowMax];
+    uint16_t* list = lists[threadIdx.x >> 5];
+    setup_group(sm, A, A.blob64, gi);
+    const SeqV Q = seq_v(sm, 0);
+    const InView<double> V = in_view<double>(A, sm->ws[0], Q.L);
+    const InTabs<double>& T = V.T;
+    const ParamView<double> P{sm->tabs.blob};
+    const int L = Q.L, m = T.m;
+    const double NEG = CF_NEG64, HALF = CF_HALF64;
+    int* stack = reinterpret_cast<int*>(A.ws + sm->ws[0] + arena64(L).stack);
+    double* parts = reinterpret_cast<double*>(stack);   // [kVitParts][L + 4]
+    double* wmax = V.FB;                                // [i]
+    const int ps = L + 4;
+    if (tm.rank() == 0) build_plist(Q, V.PLs);
+    if (threadIdx.x == 0) sm->step_ctr[0] = sm->step_ctr[1] = 0;
+    if (tm.rank() == 0 && threadIdx.x == 0) T.F5[0] = 0.0;
+    for (int t = tm.tid(); t < L; t += tm.nthreads()) A.structs[sm->soff[0] + t] = '.';
+    tm.sync();
+    for (int d = 0; d <= L; ++d) {
+        const int nE = d <= L - 2 ? V.PLs.poff[d + 1] - V.PLs.poff[d] : 0, oE = nE ? V.PLs.poff[d] : 0;
+        const int c = max(0, L - 1 - d);   // inner cells i = 1 .. c
+        const int nS = d >= 2 ? kVitParts * ((c + 31) >> 5) : 0;
+        run_items(sm, tm, d, 1 + nE + nS, [&](int q, int lane) {
+            if (q == 0) {   // F5[d]: FC of spans up to d - 2
+                if (d < 1) return;
+                double best = NEG;
+                for (int k = lane; k < d; k += 32) {
+                    if (!Q.pairable(k + 1, d)) continue;
+                    const double fcin = T.FC[T.at(k + 1, d - 1)], f5k = T.F5[k];
+                    if (!(fcin > HALF) || !(f5k > HALF)) continue;
+                    const double jA = junctionA_rev<Max64>(P, L, Q, k, d);
+                    best = fmax(best, __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[d])), jA));
+                }
+                best = fmax(warp_max(best), __dadd_rn(T.F5[d - 1], P.eu()));
+                if (lane == 0) T.F5[d] = best;
+            } else if (q <= nE) {
+                const int i = V.PLs.pl[oE + q - 1];
+                const double w = window_max(&sm->tabs, Q, T, i, i + d, list, lane);
+                if (lane == 0) wmax[i] = w;
+            } else {
+                const int u = q - 1 - nE, part = u % kVitParts, i = 1 + (u / kVitParts) * 32 + lane;
+                if (i > c) return;
+                constexpr int N = kVitParts, H = N * (N - 1) / 2;
+                int s = 1 + part;
+                int o1 = tri_off(s, m) + i, o2 = tri_off(d - s, m) + i + s;
+                int d1 = N * m - N * s - H, d2 = N * (d - s) - N * m - N * N + H + N;   // see cf_linear.cu, dot_tri
+                double best = NEG;
+#pragma unroll 4
+                for (; s < d; s += N) {
+                    best = fmax(best, __dadd_rn(T.FM1[o1], T.FM[o2]));
+                    o1 += d1;
+                    d1 -= N * N;
+                    o2 += d2;
+                    d2 -= N * N;
+                }
+                parts[part * ps + i] = best;
+            }
+        });
+        for (int i = tm.tid(); i + d <= L; i += tm.nthreads()) {
+            const int j = i + d, at = tri_off(d, m) + i;
+            double fc = NEG, fm1 = NEG, fm = NEG;
+            if (i > 0 && j < L) {
+                double fm2 = NEG;
+                if (d >= 2) {
+#pragma unroll
+                    for (int p = 0; p < kVitParts; ++p) fm2 = fmax(fm2, parts[p * ps + i]);
+                }
+                if (Q.pairable(i, j + 1)) {
+                    const double jB = sm->tabs.jB(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j]);
+                    fc = fmax(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP)), wmax[i]);
+                    if (fm2 > HALF)
+                        fc = fmax(fc, __dadd_rn(__dadd_rn(__dadd_rn(fm2, junctionA<Max64>(P, L, Q, i, j)), P.mp()), P.mb()));
+                }
+                if (d >= 2) {
+                    const double fin = T.FC[T.at(i + 1, j - 1)], ext = T.FM1[T.at(i + 1, j)], prev = T.FM[T.at(i, j - 1)];
+                    if (Q.pairable(i + 1, j) && fin > HALF)
+                        fm1 = __dadd_rn(__dadd_rn(__dadd_rn(fin, junctionA_rev<Max64>(P, L, Q, i, j)), P.mp()),
+                                        P.bp(Q.s[i + 1], Q.s[j]));
+                    if (ext > HALF) fm1 = fmax(fm1, __dadd_rn(ext, P.mu()));
+                    if (fm2 > HALF) fm = fm2;
+                    if (prev > HALF) fm = fmax(fm, __dadd_rn(prev, P.mu()));
+                    if (fm1 > HALF) fm = fmax(fm, fm1);
+                }
+            }
+            T.FC[at] = fc;
+            T.FM1[at] = fm1;
+            T.FM[at] = fm;
+        }
+        tm.sync();
+    }
+    if (tm.rank() == 0 && threadIdx.x < 32)
+        viterbi_traceback(&sm->tabs, Q, T, stack, A.structs + sm->soff[0], A.status, threadIdx.x);
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(kFoldThreads, 3) k_viterbi64(FoldArgs A) { viterbi_fold(A, CtaTeam{}, blockIdx.x); }
+__global__ void __launch_bounds__(kFoldThreads, 2) k_viterbi_cluster64(FoldArgs A) {
+    const int c = cluster_nctas();
+    viterbi_fold(A, ClusterTeam{cluster_ctarank(), c}, (int)blockIdx.x / c);
+}
+
+}  // namespace cf
