@@ -9,9 +9,10 @@
 // reference's sum, rounded as there, so tables are its tables.
 //
 // The FP64 pipe bounds the fold of a full device (two adds or compares a cycle
-// and SM): a window candidate is five adds and a compare, a split two.  The
-// grouped kernel evaluated windows in lockstep, a cell a lane, and kept 46 % of
-// the lanes busy there; a listed window keeps them all.
+// and SM: 81 % busy on 1,216 x 200 nt while 23 % of the issue slots are used),
+// so what need not be an FP64 add is none: maxima compare ordered integers (see
+// key), and cs + bp, a candidate's first sum, comes from a table.  That leaves
+// a window candidate three adds of six operations and a split one of two.
 #include "cf_group.cuh"
 
 namespace cf {
@@ -20,15 +21,50 @@ namespace {
 constexpr int kVitParts = 6;   // of a cell's splits; their maxima lie in the traceback stack's place
 constexpr int kVitWarps = kFoldThreads / 32;
 
-__device__ __forceinline__ double warp_max(double v) {
+// Doubles as integers in the same order (and back).
+__device__ __forceinline__ long long key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double unkey(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ long long warp_max(long long v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 
+// cs(l1, l2) + bp of the six pairs, the first sum of a window candidate
+struct LoopScores {
+    double v[6][kWindowMax];
+};
+// slot of (l1, l2), rows l1 ascending; and the pair (x, y)'s number
+__device__ __forceinline__ int loop_slot(int l1, int l2) { return l1 * (CMAX + 1) - ((l1 * (l1 - 1)) >> 1) + l2; }
+__device__ __forceinline__ int pair_number(int x, int y) {
+    constexpr unsigned long long N = 0ull << (4 * 3) | 1ull << (4 * 12) | 2ull << (4 * 6) | 3ull << (4 * 9) |
+                                     4ull << (4 * 11) | 5ull << (4 * 14);   // AU UA CG GC GU UG
+    return (int)(N >> (4 * (x * 4 + y))) & 7;
+}
+__device__ __forceinline__ void load_loop_scores(LoopScores* t, const SmemTabs<double>* tb) {
+    const ParamView<double> P{tb->blob};
+    const int x[6] = {0, 3, 1, 2, 2, 3}, y[6] = {3, 0, 2, 1, 3, 2};
+    for (int k = threadIdx.x; k < 6 * (CMAX + 1) * (CMAX + 1); k += blockDim.x) {
+        const int l1 = k / 6 / (CMAX + 1), l2 = k / 6 % (CMAX + 1);
+        if (l1 + l2 <= CMAX) {
+            double bp = 0.0;
+#pragma unroll
+            for (int n = 0; n < 6; ++n)
+                if (n == k % 6) bp = P.bp(x[n], y[n]);
+            t->v[k % 6][loop_slot(l1, l2)] = __dadd_rn(P.cs(l1, l2), bp);
+        }
+    }
+}
+
 // Largest interior-loop candidate of cell (i, j) (inside_B's terms).
-__device__ __forceinline__ double window_max(const SmemTabs<double>* __restrict__ tb, const SeqV& Q,
-                                             const InTabs<double>& T, int i, int j, uint16_t* list, int lane) {
+__device__ __forceinline__ long long window_max(const SmemTabs<double>* __restrict__ tb, const LoopScores* __restrict__ ls,
+                                                const SeqV& Q, const InTabs<double>& T, int i, int j, uint16_t* list,
+                                                int lane) {
     const ParamView<double> P{tb->blob};
     const int m = T.m, d = j - i;
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
@@ -37,7 +73,7 @@ __device__ __forceinline__ double window_max(const SmemTabs<double>* __restrict_
     const int C0 = d - 2 < CMAX ? d - 2 : CMAX;
     const uint32_t msk = lane <= C0 ? Q.window(i + lane + 1, j - C0 + lane, C0 - lane + 1) : 0u;
     const int total = window_list(msk, lane, list, lane);
-    double best = CF_NEG64;
+    long long best = key(CF_NEG64);
     for (int k0 = lane; k0 < total; k0 += 128) {
         int c[4];
         double v[4];
@@ -51,16 +87,17 @@ __device__ __forceinline__ double window_max(const SmemTabs<double>* __restrict_
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int l1 = c[u] & 31, l2 = C0 - l1 - (c[u] >> 5);
-            const JunctionEntry<double> b = tb->jb[Q.s.pair(j - l2) * 25 + Q.s.pair(i + l1)];
+            const int cq = Q.s.pair(j - l2), cp = Q.s.pair(i + l1);   // (s[q], s[q + 1]), (s[p], s[p + 1])
+            const int sq = (cq * 205) >> 10, sa = cp - 5 * ((cp * 205) >> 10);
             double e;
             if (l1 + l2 == 0) {
                 e = __dadd_rn(P.bp(si1, sj), P.stack(si, sj1, si1, sj));
             } else {
-                e = __dadd_rn(__dadd_rn(__dadd_rn(P.cs(l1, l2), b.bp), jB), b.jB);
+                e = __dadd_rn(__dadd_rn(ls->v[pair_number(sa, sq)][loop_slot(l1, l2)], jB), tb->jb[cq * 25 + cp].jB);
                 if (l1 < 2 && l2 < 2)   // 1-nt bulges and 1x1 (the zero that other loops add changes no maximum)
                     e = __dadd_rn(e, l1 == 0 ? P.b01(sj) : l2 == 0 ? P.b01(si1) : P.i11(si1, sj));
             }
-            best = fmax(best, __dadd_rn(e, v[u]));
+            best = max(best, key(__dadd_rn(e, v[u])));
         }
     }
     __syncwarp();
@@ -218,8 +255,10 @@ __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* sm = reinterpret_cast<SmemFold<double>*>(smem_raw);
     __shared__ uint16_t lists[kVitWarps][kWindowMax];
+    __shared__ LoopScores ls;
     uint16_t* list = lists[threadIdx.x >> 5];
     setup_group(sm, A, A.blob64, gi);
+    load_loop_scores(&ls, &sm->tabs);
     const SeqV Q = seq_v(sm, 0);
     const InView<double> V = in_view<double>(A, sm->ws[0], Q.L);
     const InTabs<double>& T = V.T;
@@ -227,8 +266,8 @@ __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, 
     const int L = Q.L, m = T.m;
     const double NEG = CF_NEG64, HALF = CF_HALF64;
     int* stack = reinterpret_cast<int*>(A.ws + sm->ws[0] + arena64(L).stack);
-    double* parts = reinterpret_cast<double*>(stack);   // [kVitParts][L + 4]
-    double* wmax = V.FB;                                // [i]
+    long long* parts = reinterpret_cast<long long*>(stack);   // [kVitParts][L + 4], keys
+    long long* wmax = reinterpret_cast<long long*>(V.FB);     // [i], keys
     const int ps = L + 4;
     if (tm.rank() == 0) build_plist(Q, V.PLs);
     if (threadIdx.x == 0) sm->step_ctr[0] = sm->step_ctr[1] = 0;
@@ -242,19 +281,19 @@ __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, 
         run_items(sm, tm, d, 1 + nE + nS, [&](int q, int lane) {
             if (q == 0) {   // F5[d]: FC of spans up to d - 2
                 if (d < 1) return;
-                double best = NEG;
+                long long best = key(NEG);
                 for (int k = lane; k < d; k += 32) {
                     if (!Q.pairable(k + 1, d)) continue;
                     const double fcin = T.FC[T.at(k + 1, d - 1)], f5k = T.F5[k];
                     if (!(fcin > HALF) || !(f5k > HALF)) continue;
                     const double jA = junctionA_rev<Max64>(P, L, Q, k, d);
-                    best = fmax(best, __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[d])), jA));
+                    best = max(best, key(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[d])), jA)));
                 }
-                best = fmax(warp_max(best), __dadd_rn(T.F5[d - 1], P.eu()));
-                if (lane == 0) T.F5[d] = best;
+                best = max(warp_max(best), key(__dadd_rn(T.F5[d - 1], P.eu())));
+                if (lane == 0) T.F5[d] = unkey(best);
             } else if (q <= nE) {
                 const int i = V.PLs.pl[oE + q - 1];
-                const double w = window_max(&sm->tabs, Q, T, i, i + d, list, lane);
+                const long long w = window_max(&sm->tabs, &ls, Q, T, i, i + d, list, lane);
                 if (lane == 0) wmax[i] = w;
             } else {
                 const int u = q - 1 - nE, part = u % kVitParts, i = 1 + (u / kVitParts) * 32 + lane;
@@ -263,10 +302,10 @@ __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, 
                 int s = 1 + part;
                 int o1 = tri_off(s, m) + i, o2 = tri_off(d - s, m) + i + s;
                 int d1 = N * m - N * s - H, d2 = N * (d - s) - N * m - N * N + H + N;   // see cf_linear.cu, dot_tri
-                double best = NEG;
+                long long best = key(NEG);
 #pragma unroll 4
                 for (; s < d; s += N) {
-                    best = fmax(best, __dadd_rn(T.FM1[o1], T.FM[o2]));
+                    best = max(best, key(__dadd_rn(T.FM1[o1], T.FM[o2])));
                     o1 += d1;
                     d1 -= N * N;
                     o2 += d2;
@@ -279,14 +318,15 @@ __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, 
             const int j = i + d, at = tri_off(d, m) + i;
             double fc = NEG, fm1 = NEG, fm = NEG;
             if (i > 0 && j < L) {
-                double fm2 = NEG;
+                long long k2 = key(NEG);
                 if (d >= 2) {
 #pragma unroll
-                    for (int p = 0; p < kVitParts; ++p) fm2 = fmax(fm2, parts[p * ps + i]);
+                    for (int p = 0; p < kVitParts; ++p) k2 = max(k2, parts[p * ps + i]);
                 }
+                const double fm2 = unkey(k2);
                 if (Q.pairable(i, j + 1)) {
                     const double jB = sm->tabs.jB(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j]);
-                    fc = fmax(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP)), wmax[i]);
+                    fc = unkey(max(key(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP))), wmax[i]));
                     if (fm2 > HALF)
                         fc = fmax(fc, __dadd_rn(__dadd_rn(__dadd_rn(fm2, junctionA<Max64>(P, L, Q, i, j)), P.mp()), P.mb()));
                 }
