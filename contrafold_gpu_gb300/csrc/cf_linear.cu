@@ -435,15 +435,14 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
 //               (l1, l2) of the warp's part the sum of g G over the sequence,
 //               84 running sums in each lane's registers (four cells a lane),
 //               and each cell's own sum for its close weight's count;
-//   all warps   split sums for m, o and FM2 (recomputed: same terms, same
-//               order for every checkpoint spacing), units of 32 cells;
+//   all warps   split sums for m and o, units of 32 cells;
 //   a thread a cell  the derivatives and the probability of each transition.
 //
 // Counts need no atomics: thread i takes the cells (i, .), so the bases on one
 // side of its pairs never change, and it adds into rows of its own, one for
 // each choice of the bases on the other side.  Every sum has a fixed order.
 // ---------------------------------------------------------------------------
-constexpr int kOutSplit = 3;    // parts of a split sum
+constexpr int kOutSplit = 4;    // parts of a split sum
 constexpr int kOutWarps = kLinOutThreads / 32;
 constexpr int kCsrRow = 36;
 enum { kRowClose = 0, kRowV01 = 10, kRowV11 = 15, kRowStack = 20, kRowMulti = 30, kRowOut = 40, kRowEnd = 50, kRows = 60 };
@@ -460,7 +459,7 @@ struct LinOutHead {
 };
 struct LinOutLayout {
     int gs, go, cs;
-    int G, g, O, Wp, Pm, Po, P2, f, m, o, F5o, sig, pd, rows, codes, total;
+    int G, g, O, Wp, Pm, Po, f, m, o, F5o, sig, pd, rows, codes, total;
     bool rows_shared;           // the kRowStack .. rows too
 };
 __host__ __device__ __forceinline__ LinOutLayout lin_out_layout(int L) {
@@ -476,7 +475,6 @@ __host__ __device__ __forceinline__ LinOutLayout lin_out_layout(int L) {
     Y.Wp = take(kParts * Y.cs);
     Y.Pm = take(kOutSplit * Y.cs);
     Y.Po = take(kOutSplit * Y.cs);
-    Y.P2 = take(kOutSplit * Y.cs);
     Y.f = take(4 * Y.cs);
     Y.m = take(2 * Y.cs);
     Y.o = take(4 * Y.cs);
@@ -580,7 +578,7 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
     const int L = D.L, m = L + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const LinOutLayout Y = lin_out_layout(L);
     auto at = [&](int o) { return reinterpret_cast<float*>(smem_raw + o); };
-    float *G = at(Y.G), *gr = at(Y.g), *O = at(Y.O), *Wp = at(Y.Wp), *Pm = at(Y.Pm), *Po = at(Y.Po), *P2 = at(Y.P2);
+    float *G = at(Y.G), *gr = at(Y.g), *O = at(Y.O), *Wp = at(Y.Wp), *Pm = at(Y.Pm), *Po = at(Y.Po);
     float *fr = at(Y.f), *mr = at(Y.m), *orr = at(Y.o), *F5o = at(Y.F5o), *sig = at(Y.sig), *pd = at(Y.pd),
           *rows = at(Y.rows);
     int8_t* s = reinterpret_cast<int8_t*>(smem_raw + Y.codes);
@@ -675,6 +673,12 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
     for (int k = 0; k < 12; ++k) cD[k] = 0.f;
     // this thread's sums over its cells
     float s_mu = 0.f, s_one = 0.f, s_multi = 0.f, s_ext = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, s_hp = 0.f, end_last = 0.f;
+    // of this thread's last pair: the row of its bases (-1: none), its hairpin and small loops, and what neither they
+    // nor its stack account for
+    struct {
+        int y;
+        float loops, rest;
+    } before = {-1, 0.f, 0.f};
     __syncthreads();
 
     for (int d = L - 2; d >= -1; --d) {
@@ -699,24 +703,22 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
         }
         if (d >= 2) {   // split sums, units of 32 cells dealt out as warps come free
             constexpr int N = kOutSplit, T = N * (N - 1) / 2;
-            const int units = 3 * N * ((c + 31) >> 5);
+            const int units = 2 * N * ((c + 31) >> 5);
             for (;;) {
                 int u = 0;
                 if (lane == 0) u = atomicAdd(&h->ctr[d & 1], 1);
                 u = __shfl_sync(0xffffffffu, u, 0);
                 if (u >= units) break;
-                const int kind = u % 3, q = (u / 3) % N, i = 1 + (u / (3 * N)) * 32 + lane, j = i + d, x = 1 + q;
+                const int kind = u % 2, q = (u / 2) % N, i = 1 + (u / (2 * N)) * 32 + lane, j = i + d, x = 1 + q;
                 if (i > c) continue;
                 if (kind == 0) {          // m: two(i - x, j) FM1(i - x, i)
                     Pm[q * cs + i - 1] = dot_tri<float, N>(two, tri_off(d + x, m) + i - x, N * m - N * (d + x) - T - N,
                                                            FM1, tri_off(x, m) + i - x, N * m - N * x - T - N,
                                                            part_terms<N>(i - 1, q));
-                } else if (kind == 1) {   // o: two(i, j + x) FM(j, j + x)
+                } else {                  // o: two(i, j + x) FM(j, j + x)
                     Po[q * cs + i - 1] = dot_tri<float, N>(two, tri_off(d + x, m) + i, N * m - N * (d + x) - T,
                                                            FM, tri_off(x, m) + j, N * m - N * x - T,
                                                            part_terms<N>(L - 1 - j, q));
-                } else {
-                    P2[q * cs + i - 1] = splits<float, N>(FM1, FM, m, d, i, q);
                 }
             }
         }
@@ -724,27 +726,31 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
         if (tid == 0) h->ctr[(d & 1) ^ 1] = 0;
         const float kd = scale_pow<float>(max(d, 0));
         const int i = 1 + tid;
-        // the loop sums of diagonal d + 1, for its close weights' counts
-        if (d + 1 >= 4 && i <= c - 1) {
-            const float g1 = gr[((d + 1) & (kRing - 1)) * go + i + 32];
-            if (g1 != 0.f) {
-                float win = 0.f;
+        // The loop sum of this thread's pair of diagonal d + 1, for its close weight's count.  What the pair's
+        // probability leaves after its stack, hairpin and interior loops is its multiloop's: FM2 is not needed again.
+        if (d + 1 >= 0 && i <= c - 1 && before.y >= 0) {
+            float win = 0.f;
+            if (d + 1 >= 4) {
 #pragma unroll
                 for (int p = 0; p < kParts; ++p) win += Wp[p * cs + i - 1];
-                rows[(kRowClose + side(s[i + d + 2]) * 5 + s[i + d + 1]) * cs + i] += g1 * win;
+                win *= gr[((d + 1) & (kRing - 1)) * go + i + 32];
+                const float v_multi = before.rest - win;
+                more[(kRowMulti - kOwnRows + before.y) * rs + i] += v_multi;
+                s_multi += v_multi;
             }
+            rows[(kRowClose + before.y) * cs + i] += before.loops + win;
         }
+        before.y = -1;
         float v_hp = 0.f;
         if (d >= 0 && i <= c) {
             const int j = i + d, off = tri_off(d, m);
             const bool inner = i >= 2 && j + 1 <= L - 1;   // the cell (i - 1, j + 1) exists
-            float mv = 0.f, ov = 0.f, f2 = 0.f;
+            float mv = 0.f, ov = 0.f;
             if (d >= 2) {
 #pragma unroll
                 for (int p = 0; p < kOutSplit; ++p) {
                     mv += Pm[p * cs + i - 1];
                     ov += Po[p * cs + i - 1];
-                    f2 += P2[p * cs + i - 1];
                 }
                 if (i <= c - 1) mv += mr[((d + 1) & 1) * cs + i] * muk;
                 if (i >= 2) ov += orr[((d + 1) & 3) * cs + i - 1] * muk;
@@ -781,7 +787,6 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
                 const float fm = fv * mm * w_multi(w, s, i, b);
                 tw += fm;
                 // probabilities of the transitions: as the outer pair ...
-                const float v_multi = fm * f2;
                 v_hp = gv * w.hp[d <= DHP ? d : DHP] * kd;
                 float v01 = 0.f, v10 = 0.f, v11 = 0.f, v_st = 0.f;
                 if (d >= 2) v_st = fv * w.stack[key] * Bt[tri_off(d - 2, m) + i + 1];
@@ -792,17 +797,18 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
                 }
                 if (d >= 4) v11 = gv * k2 * w.cs11 * w.i11[si1 * 5 + sj] * G[((d - 4) & (kRing - 1)) * gs + 2 + i + 2];
                 const int y1 = side(sb) * 5 + sj, y2 = side(sb) * 5 + sr;
-                rows[(kRowClose + y1) * cs + i] += v_hp + v01 + v10 + v11;
+                before.loops = v_hp + v01 + v10 + v11;
+                before.rest = P - v_st - before.loops;
+                before.y = y1;
                 rows[(kRowV01 + sj) * cs + i] += v01;
                 rows[(kRowV11 + sj) * cs + i] += v11;
                 more[(kRowStack - kOwnRows + y1) * rs + i] += v_st;
-                more[(kRowMulti - kOwnRows + y1) * rs + i] += v_multi;
                 // ... and as the inner one
                 more[(kRowOut - kOwnRows + y2) * rs + i] += dG * out * Bv;
                 const float v_one = e_one * Bv, v_ext = e_ext * Bv;
                 if (b == L) end_last = v_one + v_ext;   // no base on its right: once for each i
                 else more[(kRowEnd - kOwnRows + y2) * rs + i] += v_one + v_ext;
-                s_one += v_one; s_ext += v_ext; s_multi += v_multi;
+                s_one += v_one; s_ext += v_ext;
                 s01 += v01; s10 += v10; s11 += v11;
                 if (d >= DHP) s_hp += v_hp;
             }
