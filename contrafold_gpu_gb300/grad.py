@@ -21,6 +21,7 @@ feature of the parameter file (the loader's key-set fallbacks stay fixed).
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
@@ -79,8 +80,13 @@ def tying_jacobian(names: Optional[Sequence[str]] = None) -> np.ndarray:
 class GradResult:
     logz: np.ndarray
     d_blob: np.ndarray
-    d_theta: np.ndarray
     d_bonus: List[np.ndarray]
+    names: Sequence[str]
+
+    @functools.cached_property
+    def d_theta(self) -> np.ndarray:
+        """(n, n_features): d_blob through the loader's tying, made when it is first asked for."""
+        return self.d_blob @ tying_jacobian(self.names)
 
 
 def _engine_for_theta(theta, names, device):
@@ -131,9 +137,7 @@ def logz_grad(seqs: Sequence[str], theta=None, bonus=None, masks=None, names=Non
                                _p(unp, ctypes.c_double)))
     if own:
         eng.close()
-    J = tying_jacobian(names)
-    counts = counts[:B.n]
-    return GradResult(logz=logz[:B.n], d_blob=counts, d_theta=counts @ J,
+    return GradResult(logz=logz[:B.n], d_blob=counts[:B.n], names=names,
                       d_bonus=[unp[B.offsets[b]:B.offsets[b + 1]].copy() for b in range(B.n)])
 
 
@@ -155,7 +159,10 @@ def _torch_function():
                 bn = bonus.detach().float().cpu().numpy()
                 bl = [bn[b, :len(s)] for b, s in enumerate(seqs)]
             res = logz_grad(seqs, th, bl, masks)
-            ctx.d_theta = torch.from_numpy(res.d_theta)
+            # the sequences' counts; backward sums them before they go through the tying, one row instead of n
+            # (512 x 2,577 x 708: 3.2 ms of a training step)
+            ctx.d_blob = res.d_blob
+            ctx.names = res.names
             Lmax = max((len(s) for s in seqs), default=0)
             db = np.zeros((len(seqs), Lmax))
             for b, v in enumerate(res.d_bonus):
@@ -167,7 +174,7 @@ def _torch_function():
         @staticmethod
         def backward(ctx, g):
             g64 = g.detach().double().cpu()
-            gt = (g64[:, None] * ctx.d_theta).sum(0).to(torch.float64)
+            gt = torch.from_numpy((g64.numpy() @ ctx.d_blob) @ tying_jacobian(ctx.names))
             gb = (g64[:, None] * ctx.d_bonus) if ctx.has_bonus else None
             return gt, gb, None, None
 
