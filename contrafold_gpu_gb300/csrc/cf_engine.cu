@@ -620,7 +620,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
     if (P.lat || (job == JOB_MFE && batched && !eng->shared)) {
         P.ctas = P.cluster ? cf::kClusterCtas : 1;
         if (!P.cluster && P.Lmax > 128)
-            P.ctas = n * 8 <= 2 * sms ? 8 : n * 4 <= 2 * sms ? 4 : n * 2 <= sms ? 2 : 1;
+            P.ctas = n * 8 <= 2 * sms ? 8 : n * 4 <= 2 * sms ? 4 : 1;
     }
     if (P.lat) {   // no room for the longest sequence's terms or codes: the grouped kernels need less
         int dev_max = 0;

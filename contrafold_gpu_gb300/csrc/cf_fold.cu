@@ -216,7 +216,7 @@ __device__ __forceinline__ void outside_group(SmemFold<float>* sm, const FoldArg
             },
             [&](int g, int a) {   // phase A(t): FMo, FM1o, FM2o
                 const SeqV Q = seq_v(sm, g);
-                outside_A_merged<Team::kChainPF>(sr, &sm->tabs, Q, out_tabs(A, sm->ws[g], Q.L), a, a + t);
+                outside_A<Team::kChainPF>(sr, &sm->tabs, Q, out_tabs(A, sm->ws[g], Q.L), a, a + t);
             });
     }
 }
@@ -259,14 +259,14 @@ __global__ void __launch_bounds__(kFoldThreads, MODE == 0 ? kFoldMinBlocksMea : 
     auto* sm = reinterpret_cast<SmemFold<float>*>(smem_raw);
     setup_group(sm, A, A.blob32);
     if constexpr (MODE == 0 || MODE == 2) {
-        inside_group<Lse32>(sm, A, CtaTeamMea{});
-        outside_group(sm, A, CtaTeamMea{});
+        inside_group<Lse32>(sm, A);
+        outside_group(sm, A);
         __syncthreads();
         FoldArgs Ap = A;
         Ap.post_out = nullptr;
         Ap.logz = nullptr;
-        posterior_group(sm, Ap, CtaTeamMea{});
-        mea_group(sm, A, CtaTeamMea{});
+        posterior_group(sm, Ap);
+        mea_group(sm, A);
     } else {
         inside_group<Lse32>(sm, A);
         outside_group(sm, A);

@@ -86,17 +86,6 @@ struct CtaTeam {
     __device__ __forceinline__ void sync() const { __syncthreads(); }
 };
 
-// The fused MEA kernels' team: the chain pipeline one term shallower (fused MEA
-// at 4 CTAs per SM, 64 registers: depth 2 / 3 / 4 / 6 measured 33.1k / 33.9k /
-// 33.2k / 31.5k folds/s on 10,000 x 200 nt; the per-phase, BPP and sampling
-// kernels keep kChainPF).
-#ifndef CF_FUSED_MEA_CHAIN_PF
-#define CF_FUSED_MEA_CHAIN_PF 3
-#endif
-struct CtaTeamMea : CtaTeam {
-    static constexpr int kChainPF = CF_FUSED_MEA_CHAIN_PF;
-};
-
 struct ClusterTeam {
     static constexpr int kChainPF = CF_CLUSTER_CHAIN_PF;
     int r, c;   // rank of this CTA in the cluster, cluster size

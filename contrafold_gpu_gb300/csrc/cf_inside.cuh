@@ -150,8 +150,8 @@ __device__ __forceinline__ typename S::Real junctionA_rev(const ParamView<typena
 //     goes to the slot read at term k - 1, whose value the fold of term k - 1
 //     has already consumed.  The module defines CF_CHAIN_THREADS (its block
 //     size); float chains only.
-//   CF_CHAIN_PF = PF > 0: a rolling register pipeline of 2*PF terms (the
-//     default of the PFD template parameter; latency kernels pass a deeper one).
+//   CF_CHAIN_PF = PF > 0: a rolling register pipeline of 2*PF terms (fused MEA
+//     of 10,000 x 200 nt with PF 3, 4, 6: 241, 236, 240 ms; PF is the default of the PFD template parameter; latency kernels pass a deeper one).
 //   both 0: load, then fold.
 // ---------------------------------------------------------------------------
 #ifndef CF_CHAIN_PF
@@ -183,6 +183,30 @@ __device__ __forceinline__ void cp_async_wait() {
 // ring[slot][operand][thread]: consecutive threads use consecutive words
 __shared__ float cf_chain_ring[CF_CHAIN_ASYNC + 1][2][CF_CHAIN_THREADS];
 #endif
+
+// A walk through a table, whose step becomes one smaller with every cell.
+template <typename R>
+struct DiagPtr {
+    int step;
+#ifdef CF_CHECK
+    CF_TAB(R) t;
+    int at;
+    __device__ DiagPtr(CF_TAB(R) tab, int o, int s) : step(s), t(tab), at(o) {}
+    __device__ const R* next() {
+        const R* q = t + at;
+        at += step--;
+        return q;
+    }
+#else
+    const R* p;
+    __device__ __forceinline__ DiagPtr(const R* tab, int o, int s) : step(s), p(tab + o) {}
+    __device__ __forceinline__ const R* next() {
+        const R* q = p;
+        p += step--;
+        return q;
+    }
+#endif
+};
 
 template <typename R, int PFD = kChainPF, class Ld, class Step>
 __device__ __forceinline__ void prefetched_chain(int n, Ld ld, Step step) {
@@ -280,47 +304,51 @@ __device__ __forceinline__ void prefetched_chain(int n, Ld ld, Step step) {
     }
 }
 
-// What a window's candidate loads ahead of its use: its table value and the
-// pair code of its position.
-template <typename R>
-struct Candidate {
-    R v;
-    int code;
-};
-
-// One row of a lockstep window walk (see inside_B): every lane of the group
-// runs `slots` iterations (the largest candidate count among them) and takes
-// the set bits of its own mask, highest first (HI) or lowest first; the
-// table value of the next candidate, `ld(bit)`, is loaded before the current
-// one is used, `use(bit, v)`.  (Two to eight loads ahead measured slower, in
-// the batched and in the cluster kernels alike.)
-template <bool HI, typename V, class Ld, class Use>
-__device__ __forceinline__ void lockstep_row(uint32_t msk, int slots, Ld ld, Use use) {
-    auto take = [&](int& bit) -> bool {
-        if (msk == 0u) return false;
-        if constexpr (HI) {
-            bit = 31 - __clz(msk);
-            msk ^= 1u << bit;
-        } else {
-            bit = __ffs(msk) - 1;
-            msk &= msk - 1u;
+// The rows of a window, four at a time: a lane goes on to the next of the four
+// as soon as its own is used up, so a warp takes as many turns as its fullest
+// lane has candidates in the four rows.  (Cells of 200-nt sequences have 120
+// candidates on average; a warp needs 228 turns row by row, 174 by fours, 143
+// if every lane fetches its next row when it likes, but the fetch then costs
+// every turn 40 instructions, where the fours' masks wait in registers.  The
+// folds are bound by instruction issue: 10,000 x 200 nt MEA 267 ms row by row,
+// 256 with free rows, 241 by fours; 25 samples of 1,024 x 40-400 nt 56, 55, 48.)
+//
+// row(k) is the mask of the lane's k-th row (k < rows, which all lanes share),
+// its candidates from bit 31 downwards; ld(k, u) prepares the candidate of bit
+// 31 - u of that row one turn before use() folds it, or not, if use()'s second
+// argument says that there was none.
+template <class Cand, class Row, class Ld, class Use>
+__device__ __forceinline__ void queue_rows(unsigned lanes, int rows, Row row, Ld ld, Use use) {
+    Cand cur{};
+    bool has = false;
+    for (int k0 = 0; k0 < rows; k0 += 4) {
+        uint32_t m0 = row(k0), m1 = k0 + 1 < rows ? row(k0 + 1) : 0u;
+        uint32_t m2 = k0 + 2 < rows ? row(k0 + 2) : 0u, m3 = k0 + 3 < rows ? row(k0 + 3) : 0u;
+        // an empty row between others takes a turn
+        int turns = __popc(m0) + max(__popc(m1), 1) + max(__popc(m2), 1) + __popc(m3);
+        turns = __reduce_max_sync(lanes, (m0 | m1 | m2 | m3) != 0u ? turns : 0);
+        int k = k0;
+        for (int t = 0; t < turns; ++t) {
+            if (m0 == 0u) {
+                m0 = m1;
+                m1 = m2;
+                m2 = m3;
+                m3 = 0u;
+                ++k;
+            }
+            Cand nx = cur;
+            const bool more = m0 != 0u;
+            if (more) {
+                const int u = __clz(m0);
+                m0 &= 0x7fffffffu >> u;
+                nx = ld(k, u);
+            }
+            use(cur, has);
+            cur = nx;
+            has = more;
         }
-        return true;
-    };
-    int bit = 0;
-    V v{};
-    bool h = take(bit);
-    if (h) v = ld(bit);
-    for (int k = 0; k < slots; ++k) {
-        int bn = 0;
-        V vn{};
-        const bool hn = take(bn);
-        if (hn) vn = ld(bn);
-        if (h) use(bit, v);
-        h = hn;
-        bit = bn;
-        v = vn;
     }
+    use(cur, has);
 }
 
 // ---------------------------------------------------------------------------
@@ -356,18 +384,13 @@ __device__ __forceinline__ typename S::Real inside_A(const S& sr, const SmemTabs
     R fm2 = NEG;
     if (fm_region) {
         // term k = i+1 .. j-1: FM1[i][k] (span s1 = k-i), FM[k][j] (span s2 = j-k)
-        int o1 = tri_off(1, m) + i;          // FM1[i][i+1]
-        int o2 = tri_off(d - 1, m) + i + 1;  // FM[i+1][j]
-        int s1 = 1, s2 = d - 1;
+        DiagPtr<R> x1(T.FM1, tri_off(1, m) + i, m - 1);              // FM1[i][i+1]; span s to s+1: m - s cells on
+        DiagPtr<R> x2(T.FM, tri_off(d - 1, m) + i + 1, d - 1 - m);   // FM[i+1][j]; span s to s-1, one position right
         prefetched_chain<R, CPF>(
             d - 1,
             [&](const R*& x, const R*& y) {
-                x = T.FM1 + o1;
-                y = T.FM + o2;
-                o1 += m - s1;
-                o2 += s2 - m;           // FM[k+1][j]: span s2-1, one position right
-                ++s1;
-                --s2;
+                x = x1.next();
+                y = x2.next();
             },
             [&](int, R x, R y) {
                 // Terms with an operand at the zero sentinel are skipped by the
@@ -413,12 +436,9 @@ __device__ __forceinline__ typename S::Real inside_A(const S& sr, const SmemTabs
 // order -- so only valid candidates cost work.
 //
 // `lanes` names the lanes of the warp that evaluate cells together (all of
-// them call inside_B with the same mask).  They walk the window in lockstep:
-// row by row (the rows and each row's q range depend only on d = j - i), and
-// within a row for as many slots as the lane with the most candidates has.  A
-// lane with fewer candidates idles in the remaining slots, so the warp never
-// splits into per-lane paths; each lane still folds exactly its own
-// candidates in the reference's order.
+// them call inside_B with the same mask).  They walk the window four rows at a
+// time (queue_rows), so the warp never splits into per-lane paths; each lane
+// still folds exactly its own candidates in the reference's order.
 template <class S, class QV>
 __device__ __forceinline__ void inside_B(const S& sr, const SmemTabs<typename S::Real>* __restrict__ tb,
                                          const QV& Q, const InTabs<typename S::Real>& T, int i, int j,
@@ -430,50 +450,58 @@ __device__ __forceinline__ void inside_B(const S& sr, const SmemTabs<typename S:
     const int si = Q.s[i], sj1 = Q.s[j + 1], si1 = Q.s[i + 1], sj = Q.s[j];
     const R jB = tb->jB(si, sj1, si1, sj);
     R acc = sr.plus(NEG, S::add(jB, P.hp(d <= DHP ? d : DHP)));
-    const int nrows = (d < CMAX ? d : CMAX) + 1;
-    // row p = i + l1; q range [j - C, j] with C = min(d - 2, 30) - l1, so that
-    // candidate `bit` has l2 = C - bit.  FC[p + 1][q - 1] has span x - l2, x =
-    // d - 2 - l1: tri_off(x - l2) = tri_off(x) - l2 (2 (m - x) + 1 + l2) / 2.
-    // `near` rows (l1 < 2) hold the stacking pair and the 1-nt bulge and 1x1
-    // terms; the reference adds a zero for those in the other rows too, which
-    // is skipped: x + 0 is x except that -0 becomes +0, which no comparison,
-    // log-sum-exp or max can see and later sums keep only in the sign of a zero
-    // (the Viterbi is bound by the FP64 pipe: one add of six per candidate).
-    auto row = [&](int l1, auto near) {
-        const int p = i + l1, C = (d - 2 < CMAX ? d - 2 : CMAX) - l1, x = d - 2 - l1;
-        uint32_t msk = l1 < nrows ? Q.window(p + 1, j - C, C + 1) : 0u;
-        const int slots = __reduce_max_sync(lanes, __popc(msk));
-        if (slots == 0) return;
-        const int at2 = 2 * (tri_off(x, m) + p + 1), step = 2 * (m - x) + 1;
-        const JunctionEntry<R>* jb = tb->jb + (l1 < nrows ? Q.s.pair(p) : 0);
-        const uint8_t* code = Q.s.p + j - C;
-        const R* cs = tb->blob + CF_OFF_CS + l1 * 31;
-        lockstep_row<true, Candidate<R>>(
-            msk, slots,
-            [&](int bit) -> Candidate<R> {
-                const int l2 = C - bit;
-                return {T.FC[(at2 - l2 * (step + l2)) >> 1], code[bit]};
-            },
-            [&](int bit, const Candidate<R>& c) {
-                // no zero-threshold test on the value: a visited candidate is
-                // a pairable cell, whose FC always holds its hairpin term, and
-                // acc (likewise) is finite, so a sub-threshold value would
-                // leave acc unchanged in any case
-                const int l2 = C - bit;
-                const JunctionEntry<R> b = jb[c.code * 25];
-                R e = S::add(S::add(S::add(cs[l2], b.bp), jB), b.jB);
-                if constexpr (near) {
-                    if (l1 == 0)
-                        e = l2 == 0 ? S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj)) : S::add(e, l2 == 1 ? P.b01(sj) : R(0));
-                    else
-                        e = S::add(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sj) : R(0)));
-                }
-                acc = sr.plus(acc, S::add(e, c.v));
-            });
+    // row p = i + l1 holds q = j - l2 for l1 + l2 <= C; its partner bits are
+    // taken with bit 31 at q = j.  FC[p + 1][q - 1] has span x = d - 2 - l1 - l2.
+    // The stacking pair, the 1-nt bulges and the 1x1 loop are the first two
+    // candidates of the rows 0 and 1 and are folded on their own; the reference
+    // adds a zero in the place of their extra term to all others, which is
+    // skipped: x + 0 is x except that -0 becomes +0, which no comparison,
+    // log-sum-exp or max can see and later sums keep only in the sign of a zero.
+    // There is no zero-threshold test on the values: a candidate is a pairable
+    // cell, whose FC always holds its hairpin term, and acc (likewise) is finite,
+    // so a sub-threshold value would leave acc unchanged in any case.
+    const int C = d - 2 < CMAX ? d - 2 : CMAX;
+    const int rows = __reduce_max_sync(lanes, C + 1);
+    const uint32_t* pb = Q.PB + ((j - 31) >> 5);   // (before the first word only where C masks it)
+    const uint8_t* codep = Q.s.p + i;
+    const uint8_t* codeq = Q.s.p + j;
+    const R* cs = tb->blob + CF_OFF_CS;
+    auto row = [&](int l1) -> uint32_t {
+        if (l1 > C) return 0u;
+        const int c = Q.pc[i + l1 + 1];
+        const uint32_t* w = pb + (c & 3) * Q.W;
+        const uint32_t x = __funnelshift_r(w[0], w[1], (j - 31) & 31) & (uint32_t)((int)0x80000000 >> (C - l1));
+        return c < 4 ? x : 0u;
     };
-    const int nr = __reduce_max_sync(lanes, nrows);
-    for (int l1 = 0; l1 < 2 && l1 < nr; ++l1) row(l1, std::true_type{});
-    for (int l1 = 2; l1 < nr; ++l1) row(l1, std::false_type{});
+    struct Cand {
+        R e, v;
+    };
+    auto cand = [&](int l1, int l2) -> Cand {
+        const int x = d - 2 - l1 - l2;
+        const R v = T.FC[((x * (2 * m + 1 - x)) >> 1) + i + 1 + l1];
+        const JunctionEntry<R> b = tb->jb[codep[l1] + codeq[-l2] * 25];
+        return {S::add(S::add(S::add(cs[l1 * 31 + l2], b.bp), jB), b.jB), v};
+    };
+    for (int part = 0; part < 2; ++part) {   // row 0, then the other rows
+        if (part >= rows) break;
+        const uint32_t near = row(part);
+        if (near & 0x80000000u) {
+            const Cand c = cand(part, 0);
+            const R e = part == 0 ? S::add(P.bp(si1, sj), P.stack(si, sj1, si1, sj)) : S::add(c.e, P.b01(si1));
+            acc = sr.plus(acc, S::add(e, c.v));
+        }
+        if (near & 0x40000000u) {
+            const Cand c = cand(part, 1);
+            acc = sr.plus(acc, S::add(S::add(c.e, part == 0 ? P.b01(sj) : P.i11(si1, sj)), c.v));
+        }
+        queue_rows<Cand>(
+            lanes, part == 0 ? 1 : rows - 1, [&](int k) { return row(part + k) & (k == 0 ? 0x3fffffffu : ~0u); },
+            [&](int k, int l2) { return cand(part + k, l2); },
+            [&](const Cand& c, bool has) {
+                const R r = sr.plus(acc, S::add(c.e, c.v));
+                acc = has ? r : acc;
+            });
+    }
     if (fm2 > HALF) {
         const R jA = junctionA<S>(P, L, Q, i, j);
         acc = sr.plus(acc, S::add(S::add(S::add(fm2, jA), P.mp()), P.mb()));

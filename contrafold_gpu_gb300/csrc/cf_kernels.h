@@ -14,8 +14,7 @@ constexpr int kFoldThreads = 256;       // threads per fold CTA
 #endif
 constexpr int kFoldMinBlocks = CF_FOLD_MIN_BLOCKS;   // resident CTAs per SM the register budget targets
 // ... and for the fused grouped MEA kernel alone (GB300, 10,000 x 200 nt MEA:
-// 3 -> 31.9k, 4 -> 33.2k folds/s, 40-400 nt 14.4k -> 16.3k; 4 slowed the
-// per-phase kernels, the fused BPP kernel and the sampler's inside 1.5-2.5x)
+// 3, 4, 5 -> 250, 236, 250 ms, with the chain depth best for each)
 #ifndef CF_FOLD_MIN_BLOCKS_MEA
 #define CF_FOLD_MIN_BLOCKS_MEA 4
 #endif

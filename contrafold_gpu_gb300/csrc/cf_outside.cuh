@@ -89,64 +89,20 @@ __device__ __forceinline__ void exterior_outside_warp(const Lse32& sr, const Sme
 }
 
 // Phase A of outside cell (a, b), 0 <= a <= b <= L: FMo, FM1o, FM2o.
-__device__ __forceinline__ void outside_A(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
-                                          const SeqV& Q, const OutTabs& T, int a, int b) {
-    const ParamView<float> P{tb->blob};
-    const int L = Q.L, m = T.m, t = b - a;
-    const int at = tri_off(t, m) + a;
-    const bool fm_region = (0 < a) && (a + 2 <= b) && (b < L);
-
-    // FMo[a][b]: FM2o distribution of sources (i, b), i = 1 .. a-1 ascending,
-    // k = a (cpu.py:753-758); then block 1 of source (a, b+1):
-    // FMo[a][b] (+)= FMo[a][b+1] + mu (cpu.py:705).
-    float fmo = CF_NEG32, fm1o = CF_NEG32;
-    if (fm_region) {
-        float acc = CF_NEG32;
-        // i = a - u, u = a-1 .. 1: FM2o[i][b] at span t+u, FM1[i][a] at span u
-        for (int u = a - 1; u >= 1; --u) {
-            const float src = T.FM2o[tri_off(t + u, m) + a - u];
-            const float f1 = T.FM1[tri_off(u, m) + a - u];
-            if (src > CF_HALF32 && f1 > CF_HALF32) acc = sr.plus(acc, __fadd_rn(src, f1));
-        }
-        if (b + 1 < L) acc = sr.plus(acc, __fadd_rn(T.FMo[tri_off(t + 1, m) + a], P.mu()));
-        fmo = acc;
-
-        // FM1o[a][b]: block 2 of source (a-1, b): FM1o[a-1][b] + mu (cpu.py:715);
-        // FM2o distribution of sources (a, j), j = L-1 .. b+1, k = b (cpu.py:756);
-        // block 1 of source (a, b): (+)= FMo[a][b] (cpu.py:706).
-        acc = CF_NEG32;
-        if (a >= 2) acc = sr.plus(acc, __fadd_rn(T.FM1o[tri_off(t + 1, m) + a - 1], P.mu()));
-        // j = b + v, v = L-1-b .. 1: FM2o[a][j] at span t+v, FM[b][j] at span v
-        for (int v = L - 1 - b; v >= 1; --v) {
-            const float src = T.FM2o[tri_off(t + v, m) + a];
-            const float fmk = T.FM[tri_off(v, m) + b];
-            if (src > CF_HALF32 && fmk > CF_HALF32) acc = sr.plus(acc, __fadd_rn(src, fmk));
-        }
-        fm1o = sr.plus(acc, fmo);
-    }
-    T.FMo[at] = fmo;
-    T.FM1o[at] = fm1o;
-
-    // FM2o[a][b] (cpu.py:702-704, 746-751); FCo[a][b] came from phase B.
-    float fm2o = CF_NEG32;
-    if (fm_region) fm2o = sr.plus(fm2o, fmo);
-    if (0 < a && b < L && Q.pairable(a, b + 1)) {
-        const float fco = T.FCo[at];
-        if (fco > CF_HALF32) {
-            const float jA = junctionA<Lse32>(P, L, Q, a, b);
-            fm2o = sr.plus(fm2o, __fadd_rn(__fadd_rn(__fadd_rn(fco, jA), P.mp()), P.mb()));
-        }
-    }
-    T.FM2o[at] = fm2o;
-}
-
-// Phase A as one loop: the FMo chain (a-1 terms) and the FM1o chain (L-1-b
-// terms) run back to back in a single loop of (a-1) + (L-1-b) = L-2-t
-// iterations, which is the same for every cell of diagonal t -- lanes of a
-// warp working on one diagonal stay converged.  Each chain keeps the
-// reference's order (see outside_A).
+//
+// FMo[a][b]: FM2o distribution of sources (i, b), i = 1 .. a-1 ascending, k = a
+// (cpu.py:753-758); then block 1 of source (a, b+1): FMo[a][b] (+)= FMo[a][b+1]
+// + mu (cpu.py:705).  FM1o[a][b]: block 2 of source (a-1, b): FM1o[a-1][b] + mu
+// (cpu.py:715); FM2o distribution of sources (a, j), j = L-1 .. b+1, k = b
+// (cpu.py:756); block 1 of source (a, b): (+)= FMo[a][b] (cpu.py:706).
+// FM2o[a][b]: cpu.py:702-704, 746-751, FCo[a][b] from phase B.
+//
+// The FMo chain (a-1 terms) and the FM1o chain (L-1-b terms) run back to back
+// in a single loop of (a-1) + (L-1-b) = L-2-t iterations, which is the same for
+// every cell of diagonal t -- lanes of a warp working on one diagonal stay
+// converged.
 template <int CPF = kChainPF>
-__device__ __forceinline__ void outside_A_merged(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
+__device__ __forceinline__ void outside_A(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
                                                  const SeqV& Q, const OutTabs& T, int a, int b) {
     const ParamView<float> P{tb->blob};
     const int L = Q.L, m = T.m, t = b - a;
@@ -155,43 +111,49 @@ __device__ __forceinline__ void outside_A_merged(const Lse32& sr, const SmemTabs
     float fmo = CF_NEG32, fm1o = CF_NEG32;
     if (fm_region) {
         const int n1 = a - 1, n2 = L - 1 - b, K = n1 + n2;
-        float acc = CF_NEG32;
-        auto switch_chain = [&]() {
-            if (b + 1 < L) acc = sr.plus(acc, __fadd_rn(T.FMo[tri_off(t + 1, m) + a], P.mu()));
-            fmo = acc;
-            acc = CF_NEG32;
-            if (a >= 2) acc = sr.plus(acc, __fadd_rn(T.FM1o[tri_off(t + 1, m) + a - 1], P.mu()));
-        };
-        // loader: phase 1 (k < n1) reads FM2o[a-w][b], FM1[a-w][a] with w = n1-k;
-        // phase 2 reads FM2o[a][b+w], FM[b][b+w] with w = n2-(k-n1)
-        int kl = 0, w = n1;
-        int addr1 = tri_off(t + n1, m) + a - n1, addr2 = tri_off(n1, m) + a - n1;
-        const float* tab2 = T.FM1;
-        int first = 1;
+        const float* fmo_next = T.FMo + (tri_off(t + 1, m) + a);   // FMo[a][b + 1]
+        float first = CF_NEG32;   // FM1o[a - 1][b] opens the FM1o chain
+        if (a >= 2) first = sr.plus(first, __fadd_rn(T.FM1o[tri_off(t + 1, m) + a - 1], P.mu()));
+        float acc = CF_NEG32, acc1 = CF_NEG32;
+        // terms k < n1: FM2o[a-w][b], FM1[a-w][a] with w = n1-k; then
+        // FM2o[a][b+w], FM[b][b+w] with w = n2-(k-n1).  Every lane of a warp
+        // changes over at another k: it does so by selections (a branch, taken by
+        // one lane after the other, cost 65 instead of 45 instructions a term; 10,000 x
+        // 200 nt MEA 256 -> 246 ms).  One index for both FM and FM1, which lies fm1 cells on.
+        const int fm1 = (int)(static_cast<const float*>(T.FM1) - static_cast<const float*>(T.FM));
+        int x = tri_off(t + n1, m) + a - n1, y = fm1 + tri_off(n1, m) + a - n1, dx = n1 + t - m, dy = n1 - m;
+        const int x2 = tri_off(t + n2, m) + a, y2 = tri_off(n2, m) + b;
+        int kl = 0;
         prefetched_chain<float, CPF>(
             K,
-            [&](const float*& x, const float*& y) {
-                if (kl == n1) {
-                    w = n2;
-                    addr1 = tri_off(t + n2, m) + a;
-                    addr2 = tri_off(n2, m) + b;
-                    tab2 = T.FM;
-                    first = 0;
-                }
-                x = T.FM2o + addr1;
-                y = tab2 + addr2;
-                addr1 -= (m - t - w + 1) - first;
-                addr2 -= (m - w + 1) - first;
-                --w;
+            [&](const float*& px, const float*& py) {
+                const bool over = kl == n1;
+                x = over ? x2 : x;
+                y = over ? y2 : y;
+                dx = over ? n2 - 1 + t - m : dx;
+                dy = over ? n2 - 1 - m : dy;
+                px = T.FM2o + x;
+#ifdef CF_CHECK
+                py = y >= fm1 ? T.FM1 + (y - fm1) : T.FM + y;
+#else
+                py = T.FM + y;
+#endif
+                x += dx--;
+                y += dy--;
                 ++kl;
             },
-            [&](int k, float x, float y) {
-                if (k == n1) switch_chain();
+            [&](int k, float vx, float vy) {
+                acc1 = k == n1 ? acc : acc1;
+                acc = k == n1 ? first : acc;
                 // unguarded fold: a sentinel operand makes the term <= NEG, which
                 // Fast_LogPlusEquals discards (it returns the larger argument)
-                acc = sr.plus(acc, __fadd_rn(x, y));
+                acc = sr.plus(acc, __fadd_rn(vx, vy));
             });
-        if (K == n1) switch_chain();
+        if (n2 == 0) {
+            acc1 = acc;
+            acc = first;
+        }
+        fmo = b + 1 < L ? sr.plus(acc1, __fadd_rn(*fmo_next, P.mu())) : acc1;
         fm1o = sr.plus(acc, fmo);
     }
     T.FMo[at] = fmo;
@@ -216,7 +178,7 @@ __device__ __forceinline__ void outside_A_merged(const Lse32& sr, const SmemTabs
 //     each row walks the partner mask of position i over j+1 = b+2 ..
 //     b+2+(30-l1), highest bit first.  Source (a-1, b+1) first contributes
 //     through FM1o (block 2, cpu.py:708-714), then through block 3.
-// `lanes`: the lanes evaluating cells together, walked in lockstep as in
+// `lanes`: the lanes evaluating cells together, walked together as in
 // inside_B (rows from the largest l1max among them, per row as many slots as
 // the lane with the most candidates).
 __device__ __forceinline__ void outside_B(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
@@ -237,50 +199,66 @@ __device__ __forceinline__ void outside_B(const Lse32& sr, const SmemTabs<float>
     // jB of the inner pair (p+1, q) = (a, b+1): hc[s[q]][s[p+1]] + tm[s[q]][s[p+1]][s[q+1]][s[p]]
     const float jB2 = tb->jB(sb1, sa, Q.s[b + 2], Q.s[a - 1]);
     const int l1max = (a - 2 < CMAX) ? a - 2 : CMAX;   // i = a-1-l1 >= 1
-    // row l1: sources (i, j) = (a - 1 - l1, b + 1 + l2), l2 the mask's bit;
-    // FCo[i][j] has span x + l2, x = t + 2 + l1: tri_off(x + l2) = tri_off(x) +
-    // l2 (2 (m - x) + 1 - l2) / 2.  `near` rows as in inside_B.
+    // row l1: sources (i, j) = (a - 1 - l1, b + 1 + l2), l1 + l2 <= 30, the
+    // partner bits (zero beyond L) with l2 = 30 - l1 at bit 31.  FCo[i][j] has
+    // span x = t + 2 + l1 + l2.  The last two sources of the rows 1 and 0 have an
+    // extra term and are folded on their own (the others': as in inside_B).
     const int sb2 = Q.s[b + 2];
-    uint32_t m0 = 0u;
-    auto row = [&](int l1, auto near) {
-        const int i = a - 1 - l1, x = t + 2 + l1;
-        const int jmax = (b + 1 + CMAX - l1 < L - 1) ? b + 1 + CMAX - l1 : L - 1;
-        const bool mine = l1 <= l1max;
-        uint32_t msk = mine ? Q.window(i, b + 2, jmax - b) : 0u;
-        if (near && l1 == 0) {
-            m0 = msk;
-            msk &= ~1u;   // the stacking source comes after the FM1o term
-        }
-        const int slots = __reduce_max_sync(lanes, __popc(msk));
-        if (slots == 0) return;
-        const int at2 = 2 * (tri_off(x, m) + i), step = 2 * (m - x) + 1;
-        const JunctionEntry<float>* jb = tb->jb + (mine ? Q.s.pair(i) * 25 : 0);
-        const uint8_t* code = Q.s.p + b + 1;
-        const float* cs = tb->blob + CF_OFF_CS + l1 * 31;
-        const int si1 = near && mine ? Q.s[a - l1] : 4;
-        lockstep_row<true, Candidate<float>>(
-            msk, slots,
-            [&](int l2) -> Candidate<float> { return {T.FCo[(at2 + l2 * (step - l2)) >> 1], code[l2]}; },
-            [&](int l2, const Candidate<float>& c) {
-                if (!(c.v > CF_HALF32)) return;
-                float e = __fadd_rn(__fadd_rn(__fadd_rn(cs[l2], bp_ab), jb[c.code].jB), jB2);
-                if constexpr (near) {
-                    if (l1 == 0) e = __fadd_rn(e, l2 == 1 ? P.b01(sb2) : 0.0f);
-                    else e = __fadd_rn(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sb2) : 0.0f));
-                }
-                acc = sr.plus(acc, __fadd_rn(c.v, e));
-            });
+    const uint32_t* pb = Q.PB + ((b + 2) >> 5);
+    const uint8_t* codep = Q.s.p + a - 1;
+    const uint8_t* codeq = Q.s.p + b + 1;
+    const float* cs = tb->blob + CF_OFF_CS;
+    auto row = [&](int l1) -> uint32_t {
+        if (l1 > l1max) return 0u;
+        const int c = Q.pc[a - 1 - l1];
+        const uint32_t* w = pb + (c & 3) * Q.W;
+        const uint32_t x = __funnelshift_r(w[0], w[1], (b + 2) & 31) << (l1 + 1);
+        return c < 4 ? x : 0u;
     };
-    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
-    for (int l1 = lm; l1 >= 2; --l1) row(l1, std::false_type{});
-    for (int l1 = lm < 1 ? lm : 1; l1 >= 0; --l1) row(l1, std::true_type{});
+    struct Cand {
+        float e, v;
+    };
+    auto cand = [&](int l1, int l2) -> Cand {
+        const int x = t + 2 + l1 + l2;
+        const float v = T.FCo[((x * (2 * m + 1 - x)) >> 1) + a - 1 - l1];
+        return {__fadd_rn(__fadd_rn(__fadd_rn(cs[l1 * 31 + l2], bp_ab), tb->jb[codep[-l1] * 25 + codeq[l2]].jB), jB2), v};
+    };
+    auto fold = [&](float v, float e, bool has) {
+        const float r = sr.plus(acc, __fadd_rn(v, e));
+        acc = has && v > CF_HALF32 ? r : acc;
+    };
+    const int lm = __reduce_max_sync(lanes, l1max);
+    uint32_t near = 0u;
+    for (int part = lm < 1 ? lm : 1; part >= 0; --part) {   // the rows lm .. 1, then row 0
+        near = row(part) >> (part + 1);
+        queue_rows<Cand>(
+            lanes, part == 0 ? 1 : lm,
+            [&](int k) -> uint32_t {
+                const int l1 = part == 0 ? k : lm - k;
+                const uint32_t x = row(l1);
+                return l1 == part ? x & ~(6u << part) : x;   // l1 = part: bits part + 1 and part + 2 are l2 = 0 and 1
+            },
+            [&](int k, int u) {
+                const int l1 = part == 0 ? k : lm - k;
+                return cand(l1, 30 - l1 - u);
+            },
+            [&](const Cand& c, bool has) { fold(c.v, c.e, has); });
+        if (near & 2u) {
+            const Cand c = cand(part, 1);
+            fold(c.v, __fadd_rn(c.e, part == 0 ? P.b01(sb2) : P.i11(Q.s[a - 1], sb2)), true);
+        }
+        if (part == 1 && near & 1u) {
+            const Cand c = cand(1, 0);
+            fold(c.v, __fadd_rn(c.e, P.b01(Q.s[a - 1])), true);
+        }
+    }
     if (l1max >= 0) {
         if (b + 1 < L) {
             const float v = T.FM1o[tri_off(t + 2, m) + a - 1];
             const float jAji = junctionA_rev<Lse32>(P, L, Q, a - 1, b + 1);
             acc = sr.plus(acc, __fadd_rn(__fadd_rn(__fadd_rn(v, jAji), P.mp()), bp_ab));
         }
-        if (m0 & 1u) {   // the stacking source (a - 1, b + 1)
+        if (near & 1u) {   // the stacking source (a - 1, b + 1)
             const float v = T.FCo[tri_off(t + 2, m) + a - 1];
             if (v > CF_HALF32)
                 acc = sr.plus(acc, __fadd_rn(v, __fadd_rn(bp_ab, P.stack(Q.s[a - 1], sb2, sa, sb1))));
@@ -295,7 +273,7 @@ __device__ __forceinline__ void outside_B(const Lse32& sr, const SmemTabs<float>
 // each iff pairable(i, j+1) and its outside value is live; source (a-1, b)
 // adds its multiloop (FM1o) term right after its stacking term; the exterior
 // term comes last.  Returns the clipped value.
-// `lanes`: the lanes evaluating pairs together, walked in lockstep as in
+// `lanes`: the lanes evaluating pairs together, walked together as in
 // inside_B.
 __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restrict__ tb, const PolyTables* pt,
                                                 const SeqV& Q, const OutTabs& T, float Z, int a, int b,
@@ -310,60 +288,67 @@ __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restric
     const float jB2 = tb->jB(sb, sa, Q.s[b + 1], Q.s[a - 1]);
     float post = 0.0f;
     const int l1max = live ? ((a - 2 < CMAX) ? a - 2 : CMAX) : -1;   // i = a-1-l1 >= 1
-    // row l1: sources (i, j) = (a - 1 - l1, b + l2), l2 the mask's bit; FCo[i][j]
-    // has span x + l2, x = b - a + 1 + l1 (addresses as in outside_B)
+    // row l1: sources (i, j) = (a - 1 - l1, b + l2), l1 + l2 <= 30, the partner
+    // bits (zero beyond L) with l2 = 0 at bit 31.  FCo[i][j] has span
+    // x = b - a + 1 + l1 + l2.  The first two sources of the rows 0 and 1 have an
+    // extra term and are added on their own (the others': as in inside_B).
     const int sb1 = Q.s[b + 1];
-    auto rowmask = [&](int l1) -> uint32_t {
-        const int jmax = (b + CMAX - l1 < L - 1) ? b + CMAX - l1 : L - 1;
-        return Q.window(a - 1 - l1, b + 1, jmax - b + 1);
+    const uint32_t* pb = Q.PB + ((b + 1) >> 5);
+    const uint8_t* codep = Q.s.p + a - 1;
+    const uint8_t* codeq = Q.s.p + b;
+    const float* cs = tb->blob + CF_OFF_CS;
+    auto row = [&](int l1) -> uint32_t {
+        if (l1 > l1max) return 0u;
+        const int c = Q.pc[a - 1 - l1];
+        const uint32_t* w = pb + (c & 3) * Q.W;
+        const uint32_t x = __brev(__funnelshift_r(w[0], w[1], (b + 1) & 31)) & (uint32_t)((int)0x80000000 >> (CMAX - l1));
+        return c < 4 ? x : 0u;
     };
-    // row 0: the stacking source (a-1, b), its multiloop term, then j ascending
-    uint32_t m0 = 0u;
-    if (l1max >= 0) {
-        m0 = rowmask(0);
-        if (m0 & 1u) {
-            const float out = __fsub_rn(T.FCo[tri_off(b - a + 1, m) + a - 1], Z);
-            if (out > CF_HALF32)
-                post = __fadd_rn(post, fexp32(pt, __fadd_rn(__fadd_rn(__fadd_rn(out, bp_ab), P.stack(Q.s[a - 1], sb1, sa, sb)), fcin)));
-        }
-        if (b < L) {
-            const float v = T.FM1o[tri_off(b - a + 1, m) + a - 1];
-            if (v > CF_HALF32) {
-                const float jAji = junctionA_rev<Lse32>(P, L, Q, a - 1, b);
-                const float x = __fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(v, fcin), jAji), P.mp()), bp_ab), Z);
-                post = __fadd_rn(post, fexp32(pt, x));
+    struct Cand {
+        float v, jB, cs;
+    };
+    auto cand = [&](int l1, int l2) -> Cand {
+        const int x = b - a + 1 + l1 + l2;
+        return {T.FCo[((x * (2 * m + 1 - x)) >> 1) + a - 1 - l1], tb->jb[codep[-l1] * 25 + codeq[l2]].jB, cs[l1 * 31 + l2]};
+    };
+    auto term = [&](const Cand& c) {
+        return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(c.v, Z), c.jB), c.cs), fcin), bp_ab), jB2);
+    };
+    auto add = [&](const Cand& c, float e) {
+        if (__fsub_rn(c.v, Z) > CF_HALF32) post = __fadd_rn(post, fexp32(pt, e));
+    };
+    const int lm = __reduce_max_sync(lanes, l1max);
+    for (int part = 0; part < 2 && part <= lm; ++part) {   // row 0, then the other rows
+        const uint32_t near = row(part);
+        if (part == 0) {   // the stacking source (a-1, b) and its multiloop term
+            if (near & 0x80000000u) {
+                const float out = __fsub_rn(T.FCo[tri_off(b - a + 1, m) + a - 1], Z);
+                if (out > CF_HALF32)
+                    post = __fadd_rn(post, fexp32(pt, __fadd_rn(__fadd_rn(__fadd_rn(out, bp_ab), P.stack(Q.s[a - 1], sb1, sa, sb)), fcin)));
             }
-        }
-        m0 &= ~1u;
-    }
-    auto row = [&](int l1, auto near) {
-        const int i = a - 1 - l1, x = b - a + 1 + l1;
-        const bool mine = l1 <= l1max;
-        const uint32_t msk = l1 == 0 ? m0 : mine ? rowmask(l1) : 0u;
-        const int slots = __reduce_max_sync(lanes, __popc(msk));
-        if (slots == 0) return;
-        const int at2 = 2 * (tri_off(x, m) + i), step = 2 * (m - x) + 1;
-        const JunctionEntry<float>* jb = tb->jb + (mine ? Q.s.pair(i) * 25 : 0);
-        const uint8_t* code = Q.s.p + b;
-        const float* cs = tb->blob + CF_OFF_CS + l1 * 31;
-        const int si1 = near && mine ? Q.s[a - l1] : 4;
-        lockstep_row<false, Candidate<float>>(
-            msk, slots,
-            [&](int l2) -> Candidate<float> { return {T.FCo[(at2 + l2 * (step - l2)) >> 1], code[l2]}; },
-            [&](int l2, const Candidate<float>& c) {
-                const float outside = __fsub_rn(c.v, Z);
-                if (!(outside > CF_HALF32)) return;
-                float e = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(outside, jb[c.code].jB), cs[l2]), fcin), bp_ab), jB2);
-                if constexpr (near) {
-                    if (l1 == 0) e = __fadd_rn(e, l2 == 1 ? P.b01(sb1) : 0.0f);
-                    else e = __fadd_rn(e, l2 == 0 ? P.b01(si1) : (l2 == 1 ? P.i11(si1, sb1) : 0.0f));
+            if (l1max >= 0 && b < L) {
+                const float v = T.FM1o[tri_off(b - a + 1, m) + a - 1];
+                if (v > CF_HALF32) {
+                    const float jAji = junctionA_rev<Lse32>(P, L, Q, a - 1, b);
+                    const float x = __fsub_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(v, fcin), jAji), P.mp()), bp_ab), Z);
+                    post = __fadd_rn(post, fexp32(pt, x));
                 }
-                post = __fadd_rn(post, fexp32(pt, e));
+            }
+        } else if (near & 0x80000000u) {
+            const Cand c = cand(1, 0);
+            add(c, __fadd_rn(term(c), P.b01(Q.s[a - 1])));
+        }
+        if (near & 0x40000000u) {
+            const Cand c = cand(part, 1);
+            add(c, __fadd_rn(term(c), part == 0 ? P.b01(sb1) : P.i11(Q.s[a - 1], sb1)));
+        }
+        queue_rows<Cand>(
+            lanes, part == 0 ? 1 : lm, [&](int k) { return row(part + k) & (k == 0 ? 0x3fffffffu : ~0u); },
+            [&](int k, int l2) { return cand(part + k, l2); },
+            [&](const Cand& c, bool has) {
+                if (has) add(c, term(c));
             });
-    };
-    const int lm = __reduce_max_sync(lanes, l1max + 1) - 1;
-    for (int l1 = 0; l1 <= lm && l1 < 2; ++l1) row(l1, std::true_type{});
-    for (int l1 = 2; l1 <= lm; ++l1) row(l1, std::false_type{});
+    }
     if (!live) return 0.0f;
     const float outside = __fsub_rn(T.F5o[b], Z);
     const float f5k = T.F5[a - 1];

@@ -381,7 +381,7 @@ struct QueueCtx {
         const int L = Q.L, m = L + 1;
         if (stage == kIn || stage == kOut) {
             const int nbc = St.nb_chunks;
-            if (chunk < nbc) {   // B items: pairable cells of diagonal t - 1, walked in lockstep
+            if (chunk < nbc) {   // B items: pairable cells of diagonal t - 1, walked together
                 const int k = chunk * 32 + lane;
                 const int nb = St.nb;
                 const unsigned lanes = __ballot_sync(0xffffffffu, k < nb);
@@ -409,7 +409,7 @@ struct QueueCtx {
                     else
                         fb[i] = inside_A<Lse32>(Lse32{&sm->poly}, &sm->tabs, Q, in_tabs(s, L), i, i + t);
                 } else {
-                    outside_A_merged(Lse32{&sm->poly}, &sm->tabs, Q, out_tabs(s, L), i, i + t);
+                    outside_A(Lse32{&sm->poly}, &sm->tabs, Q, out_tabs(s, L), i, i + t);
                 }
             }
             return;

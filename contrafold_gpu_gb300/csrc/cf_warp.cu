@@ -167,7 +167,7 @@ __device__ __forceinline__ void fold_one(const WarpArgs& A, const WarpSmemHead* 
                 outside_B(sr, &sm->tabs, Q, O, a, a + dB, lanes);
             }
         }
-        for (int a = lane; a <= L - t; a += 32) outside_A_merged(sr, &sm->tabs, Q, O, a, a + t);
+        for (int a = lane; a <= L - t; a += 32) outside_A(sr, &sm->tabs, Q, O, a, a + t);
         __syncwarp();
     }
 
