@@ -146,10 +146,10 @@ __host__ __device__ __forceinline__ Arena64 arena64(int L) {
 // segments.  The evaluation order ((c0*d + c1)*d + c2)*d + c3 is the
 // reference's.
 //
-// Segment lookup: bin = floor(d) in 0..11 holds at most one boundary (the
+// Segment lookup: bin = floor(d) holds at most one boundary (the
 // boundaries 0.66, 1.63, 2.49, 3.38, 4.43, 5.79, 7.82 fall in distinct unit
 // intervals), so seg = (boundaries below the bin) + (d >= the boundary inside
-// the bin), read from a 12-entry table -- the same count as comparing d with
+// the bin), read from a 16-entry table -- the same count as comparing d with
 // all seven.  Fast_Exp uses the same scheme on u = -x over its five
 // boundaries (0.67, 1.48, 2.49, 3.84, 5.86: distinct unit intervals too).
 // ---------------------------------------------------------------------------
@@ -169,14 +169,23 @@ __host__ __device__ __forceinline__ Arena64 arena64(int L) {
 #define FEXP_T4 ((float)-1.4805375919)
 #define FEXP_T5 ((float)-0.6725053211)
 
-constexpr int kLseBins = 12;    // unit bins of d over [0, 12)
-constexpr int kFexpBins = 10;   // unit bins of -x over [0, 10)
+// Unit bins of d and of -x over [0, 16): four bits of 2^20 + d rounded towards
+// zero, whatever d is.  (From 16 on the bin is any of them and the cubic's value
+// anything, but the cutoff, 11.86 and 9.91, has decided the result then.)
+constexpr int kLseBins = 16;
+constexpr int kFexpBins = 16;
+__device__ __forceinline__ const float2& unit_bin(const float2* bins, float d) {
+    // 8 floor(d), the bin's byte offset.  (A float-to-integer conversion runs at
+    // an eighth of the rate and waits some 20 cycles more.)
+    const int at = __float_as_int(__fadd_rz(d, 1048576.0f)) & 0x78;
+    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(bins) + at);
+}
 
 struct PolyTables {
     float4 lse[8];
     float4 fexp[6];
     float2 lse_bin[kLseBins];     // {boundary inside the bin or +FLT_MAX, int bits: boundaries below, in bytes of lse}
-    float2 fexp_bin[kFexpBins];   // {-boundary inside the bin or -FLT_MAX, int bits: boundaries above}
+    float2 fexp_bin[kFexpBins];   // {-boundary inside the bin or -FLT_MAX, int bits: boundaries above, in bytes of fexp}
 };
 
 __device__ __forceinline__ void load_poly_tables(PolyTables* t) {
@@ -225,7 +234,7 @@ __device__ __forceinline__ void load_poly_tables(PolyTables* t) {
                 if (U[i] >= hi) ++base;
                 else if (U[i] >= lo) inner = U[i];
             }
-            t->fexp_bin[b] = make_float2(inner, __int_as_float(base));
+            t->fexp_bin[b] = make_float2(inner, __int_as_float(base * (int)sizeof(float4)));
         }
     }
 }
@@ -288,11 +297,7 @@ __device__ __forceinline__ float lse32(const PolyTables* __restrict__ pt, float 
     const float hi = fmaxf(a, b);
     const float lo = fminf(a, b);
     const float d = fabsf(__fsub_rn(a, b));
-    // 8 floor(d) for d < 12, the bin's byte offset: 2^20 + d rounded towards
-    // zero holds floor(8 d) in its low bits.  (A float-to-integer conversion
-    // runs at an eighth of the rate and waits some 20 cycles more.)
-    const int at = __float_as_int(__fadd_rz(fminf(d, 11.5f), 1048576.0f)) & 0x78;
-    const float2 e = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(pt->lse_bin) + at);
+    const float2 e = unit_bin(pt->lse_bin, d);
     const int seg = __float_as_int(e.y) + (d >= e.x ? (int)sizeof(float4) : 0);
     const float r = cubic(*reinterpret_cast<const float4*>(reinterpret_cast<const char*>(pt->lse) + seg), d);
     const float res = __fadd_rn(lo, r);
@@ -304,6 +309,15 @@ __device__ __forceinline__ float lse32(const PolyTables* __restrict__ pt, float 
 #endif
 }
 
+// Fast_Exp of x < 0 (of other x: some number)
+__device__ __forceinline__ float fexp32_below(const PolyTables* __restrict__ pt, float x) {
+    const float u = -x;   // x >= T_k  <=>  u <= -T_k
+    const float2 e = unit_bin(pt->fexp_bin, u);
+    const int seg = __float_as_int(e.y) + (u <= e.x ? (int)sizeof(float4) : 0);
+    const float r = cubic(*reinterpret_cast<const float4*>(reinterpret_cast<const char*>(pt->fexp) + seg), x);
+    return x < FEXP_T0 ? 0.0f : r;
+}
+
 // exp(x), CONTRAfold Fast_Exp (RealT = float).  For x >= 0 the reference
 // evaluates exp in double precision and rounds (cpu.py:578-580).
 __device__ __forceinline__ float fexp32(const PolyTables* __restrict__ pt, float x) {
@@ -311,11 +325,7 @@ __device__ __forceinline__ float fexp32(const PolyTables* __restrict__ pt, float
         if (x > (float)46.052) return (float)1e20;
         return (float)exp((double)x);
     }
-    const float u = -x;   // x < 0: x >= T_k  <=>  u <= -T_k
-    const float2 e = pt->fexp_bin[min(__float2int_rz(u), kFexpBins - 1)];
-    const int seg = __float_as_int(e.y) + (u <= e.x);
-    const float r = cubic(pt->fexp[seg], x);
-    return x < FEXP_T0 ? 0.0f : r;
+    return fexp32_below(pt, x);
 }
 
 // FP64 log-sum-exp with exact log1p/exp (cpu.py:154-162).

@@ -67,8 +67,8 @@ struct Lse32Chain {
     static __device__ __forceinline__ float add(float x, float y) { return __fadd_rn(x, y); }
     __device__ __forceinline__ float plus(float a, float x) const {
         const float d = fabsf(__fsub_rn(a, x));   // = larger - smaller, the same rounding
-        // floor(d) for d < 12: 2^23 + d rounded towards zero
-        const int k = __float_as_int(__fadd_rz(fminf(d, 11.5f), 8388608.0f)) & 15;
+        // floor(d): 2^23 + d rounded towards zero (any bin from 16 on, as in unit_bin)
+        const int k = __float_as_int(__fadd_rz(d, 8388608.0f)) & 15;
         const float4 lo = c->below[k], hi = c->above[k];
         const bool up = d >= c->edge[k];
         const float4 q = make_float4(up ? hi.x : lo.x, up ? hi.y : lo.y, up ? hi.z : lo.z, up ? hi.w : lo.w);

@@ -314,8 +314,12 @@ __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restric
     auto term = [&](const Cand& c) {
         return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(c.v, Z), c.jB), c.cs), fcin), bp_ab), jB2);
     };
-    auto add = [&](const Cand& c, float e) {
-        if (__fsub_rn(c.v, Z) > CF_HALF32) post = __fadd_rn(post, fexp32(pt, e));
+    auto add = [&](const Cand& c, float e, bool has) {
+        has = has && __fsub_rn(c.v, Z) > CF_HALF32;
+        float x = fexp32_below(pt, e);
+        if (has && e >= 0.0f) x = fexp32(pt, e);
+        const float sum = __fadd_rn(post, x);
+        post = has ? sum : post;
     };
     const int lm = __reduce_max_sync(lanes, l1max);
     for (int part = 0; part < 2 && part <= lm; ++part) {   // row 0, then the other rows
@@ -336,18 +340,16 @@ __device__ __forceinline__ float posterior_pair(const SmemTabs<float>* __restric
             }
         } else if (near & 0x80000000u) {
             const Cand c = cand(1, 0);
-            add(c, __fadd_rn(term(c), P.b01(Q.s[a - 1])));
+            add(c, __fadd_rn(term(c), P.b01(Q.s[a - 1])), true);
         }
         if (near & 0x40000000u) {
             const Cand c = cand(part, 1);
-            add(c, __fadd_rn(term(c), part == 0 ? P.b01(sb1) : P.i11(Q.s[a - 1], sb1)));
+            add(c, __fadd_rn(term(c), part == 0 ? P.b01(sb1) : P.i11(Q.s[a - 1], sb1)), true);
         }
         queue_rows<Cand>(
             lanes, part == 0 ? 1 : lm, [&](int k) { return row(part + k) & (k == 0 ? 0x3fffffffu : ~0u); },
             [&](int k, int l2) { return cand(part + k, l2); },
-            [&](const Cand& c, bool has) {
-                if (has) add(c, term(c));
-            });
+            [&](const Cand& c, bool has) { add(c, term(c), has); });
     }
     if (!live) return 0.0f;
     const float outside = __fsub_rn(T.F5o[b], Z);
