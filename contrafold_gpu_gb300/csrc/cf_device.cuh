@@ -405,24 +405,6 @@ __device__ __forceinline__ void encode_seq(const uint8_t* __restrict__ seqs, con
     }
 }
 
-// Shared-memory header common to the FP32 kernels.
-struct SmemHead32 {
-    PolyTables poly;
-    float blob[CF_BLOB_LEN + 3];   // +3 pads to 16 bytes
-    float jB[625];                 // hc[a][b] + tm[a][b][c][d] (cpu.py:191,211-212)
-};
-
-// Load the FP32 blob and derived tables.  jB = hc + tm is the same float add
-// the reference does inline, so precomputing it keeps the bits.
-__device__ __forceinline__ void load_head32(SmemHead32* h, const float* __restrict__ gblob) {
-    load_poly_tables(&h->poly);
-    for (int t = threadIdx.x; t < CF_BLOB_LEN; t += blockDim.x) h->blob[t] = gblob[t];
-    for (int t = threadIdx.x; t < 625; t += blockDim.x) {
-        const int a = t / 125, c = (t / 25) % 5;
-        h->jB[t] = __fadd_rn(gblob[CF_OFF_HC + a * 5 + c], gblob[CF_OFF_TM + t]);
-    }
-}
-
 __device__ __forceinline__ int idx4(int a, int b, int c, int d) { return ((a * 5 + b) * 5 + c) * 5 + d; }
 
 }  // namespace cf

@@ -598,12 +598,14 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         P.warp = false;   // not even one CTA of warp slots fits: per-sequence kernels, sliced
     }
     // The latency kernels: a sequence on a cluster or, one after another on an SM, on CTAs of their own.  They win until
-    // the grouped kernels' CTAs fill the device (GB300, MEA, ms, latency / grouped: 200 nt n = 300 20 / 32, 450 29 / 34,
-    // 600 39 / 38; 40-400 nt n = 300 37 / 83, 800 71 / 90, 1,024 89 / 97).  Not on a shared device: a 512-thread CTA
-    // waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
+    // the grouped kernels' CTAs fill the device (GB300, ms, latency / grouped, MEA and 1 sample: 200 nt n = 304 19 / 24
+    // and 10 / 13, 456 29 / 26 and 15 / 13; 100 nt n = 456 8.8 / 9.3 and 5.9 / 5.4; 320 nt n = 304 46 / 53, 456 70 / 59;
+    // 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA).  Not on a shared device: a
+    // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
     int sms = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
-    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= (uniform ? 7 * sms / 2 : 6 * sms) &&
+    const int cut = uniform ? (P.Lmax <= 128 ? 3 : 2) : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
+    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= cut * sms &&
                           (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE));
     P.slice_begin.clear();
     P.slice_words.clear();
