@@ -783,7 +783,7 @@ int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S) {
     const bool fp64 = job == JOB_LOGZ64, train = job == JOB_GRAD;
     int classes = 0;
     for (size_t k = P.n_fold; k < P.descs.size(); ++classes) {
-        const int L = P.descs[k].L, rc = raise_smem_limit((const void*)cf::lin_inside_kernel(L, fp64, train).fn, eng->device,
+        const int L = P.descs[k].L, rc = raise_smem_limit((const void*)cf::lin_inside_kernel(L, fp64, train, eng->shared).fn, eng->device,
                                                           std::max<size_t>(cf::lin_inside_smem_bytes(L, fp64), 48 * 1024));
         if (rc) return rc;
         while (k < P.descs.size() && cf::lin_class_end(P.descs[k].L, fp64) == cf::lin_class_end(L, fp64)) ++k;
@@ -795,14 +795,14 @@ int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S) {
 // length class, on side streams beside st but for the first.  A launch of all
 // of them would give every CTA the longest one's shared memory (1,024 x 50-500
 // nt on GB300: one CTA an SM, 15.0 ms).
-int launch_lin_inside(const Plan& P, const cf::LinArgs& A, int k0, int k1, bool fp64, bool train, LinStreams* S,
+int launch_lin_inside(cf_engine* eng, const Plan& P, const cf::LinArgs& A, int k0, int k1, bool fp64, bool train, LinStreams* S,
                       cudaStream_t st, int& launches) {
     int used = 0;
     for (int k = k0; k < k1;) {
         const int L = P.descs[k].L, end = cf::lin_class_end(L, fp64);
         int q = k;
         while (q < k1 && cf::lin_class_end(P.descs[q].L, fp64) == end) ++q;
-        const cf::LinKernel K = cf::lin_inside_kernel(L, fp64, train);
+        const cf::LinKernel K = cf::lin_inside_kernel(L, fp64, train, eng->shared);
         cudaStream_t on = st;
         if (k > k0) {
             on = S->side[used];
@@ -859,7 +859,7 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         CF_CUDA(cudaMemsetAsync(X.fails, 0, sizeof(int), st));
         cudaEvent_t stop = nullptr;
         if (X.timer && (rc = X.timer->begin(0, st, &stop))) return rc;
-        if ((rc = launch_lin_inside(P, La, k0, k1, fp64, false, X.lin_streams, st, X.launches))) return rc;
+        if ((rc = launch_lin_inside(eng, P, La, k0, k1, fp64, false, X.lin_streams, st, X.launches))) return rc;
         if (fp64) cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
         else cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
         ++X.launches;
@@ -1530,7 +1530,7 @@ extern "C" int cf_grad(cf_engine* e, const uint8_t* seqs, const int64_t* offsets
         La.fails = e->fails.p;
         CF_CUDA(cudaMemsetAsync(e->fails.p, 0, sizeof(int), st));
         int launches = 0;
-        if ((rc = launch_lin_inside(P, La, P.lin_begin[sl], P.lin_begin[sl + 1], false, true, &e->lin_streams, st, launches)))
+        if ((rc = launch_lin_inside(e, P, La, P.lin_begin[sl], P.lin_begin[sl + 1], false, true, &e->lin_streams, st, launches)))
             return rc;
         cf::k_lin_outside32<<<A.n, cf::kLinOutThreads, out_smem, st>>>(La);
         adjoint(A, e->fails.p);

@@ -984,9 +984,10 @@ __global__ void __launch_bounds__(256, 2) k_lin_inside64(LinArgs A) { lin_inside
 
 // Threads by length: as many as keep an SM at about 1,024 threads with the
 // CTAs its shared memory holds (49 KB at 128 nt, 74 KB at 235, 113 KB at 395).
-LinKernel lin_inside_kernel(int L, bool fp64, bool train) {
+// On a shared device no more than other kernels' CTAs have (narrow).
+LinKernel lin_inside_kernel(int L, bool fp64, bool train, bool narrow) {
     if (fp64) return {k_lin_inside64, 256};
-    if (L <= 235) return {train ? k_lin_inside32<true, 256> : k_lin_inside32<false, 256>, 256};
+    if (L <= 235 || narrow) return {train ? k_lin_inside32<true, 256> : k_lin_inside32<false, 256>, 256};
     if (L <= 395) return {train ? k_lin_inside32<true, 512> : k_lin_inside32<false, 512>, 512};
     return {train ? k_lin_inside32<true, 1024> : k_lin_inside32<false, 1024>, 1024};
 }

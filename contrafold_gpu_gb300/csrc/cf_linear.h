@@ -62,7 +62,7 @@ struct LinKernel {
     int threads;
 };
 // the inside of sequences of up to L nt; train: with bonuses, and the tables the derivatives need
-LinKernel lin_inside_kernel(int L, bool fp64, bool train);
+LinKernel lin_inside_kernel(int L, bool fp64, bool train, bool narrow);   // narrow: 256 threads at most
 int lin_class_end(int L, bool fp64);   // sequences up to this length share the launch of an L-nt one
 size_t lin_inside_smem_bytes(int Lmax, bool fp64);
 // gradients: the derivatives, after lin_inside_kernel(train)

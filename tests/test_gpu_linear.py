@@ -86,3 +86,17 @@ def test_logz_follows_the_parameters(engine, P, oracle):
         plan.close()
     finally:
         eng.close()
+
+
+def test_shared_device_same_sums(engine, P):
+    """A shared device's launches have fewer threads from 236 nt up; sums and their order are the same."""
+    from contrafold_gpu_gb300.engine import Batch, Engine
+    rng = np.random.default_rng(23)
+    B = Batch(["".join(rng.choice(list("ACGU"), L)) for L in (60, 235, 236, 257, 395, 396, 511, 512)], None)
+    engine.set_mode("batched")
+    eng = Engine(P)
+    try:
+        eng.set_shared(True)
+        assert np.asarray(eng.logz(B)).tobytes() == np.asarray(engine.logz(B)).tobytes()
+    finally:
+        eng.close()
