@@ -133,10 +133,9 @@ struct TuneRow {
 };
 
 // The built-in table (GB300, contrafold_gpu_gb300/autotune.py sweeps):
-//  * small batches of long sequences fold on a thread-block cluster each (one
-//    600-nt MEA fold 172 -> 144 ms, 1,000 nt 450 -> 297 ms; 64 x 300 nt stays
-//    grouped: 69 vs 125 ms): every sequence >= 512 nt and at most two
-//    clusters' CTAs per SM (38 sequences on 152 SMs);
+//  * small batches of long sequences fold on a thread-block cluster of 8 each:
+//    every sequence >= 512 nt and at most two of the clusters' CTAs per SM (38
+//    sequences on 152 SMs; 4 x 801 nt MEA 181 ms grouped, 65 ms so);
 //  * large batches of mixed short lengths take the warp-per-sequence kernel
 //    (200 nt: n=1024 warp 8.7k vs grouped 10.2k MEA folds/s, n=2048 15.1k vs
 //    13.3k; 60 nt: n=2048 172k vs 186k, n=4096 238k vs 191k);
@@ -308,7 +307,7 @@ struct cf_engine {
     size_t smem_optin = 0;
     std::vector<TuneRow> tuning = default_tuning();   // schedule table of the automatic path
     int grad_ckpt = 0;   // FM2 checkpoint spacing of cf_grad (0 = automatic by the longest sequence)
-    bool shared = false; // the device is shared with other engines' launches: no wide CTAs, no clusters
+    bool shared = false; // the device is shared with other engines' launches: CTAs of 256 threads, no clusters
 };
 
 namespace {

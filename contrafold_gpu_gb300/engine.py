@@ -237,7 +237,7 @@ class Engine:
         self._check(self.lib.cf_engine_set_priority(self._h, int(bool(high))))
 
     def set_shared(self, on: bool):
-        """The device is shared with other engines' launches: no 512-thread CTAs, no clusters."""
+        """The device is shared with other engines' launches: CTAs of at most 256 threads, no clusters."""
         self._check(self.lib.cf_engine_set_shared(self._h, int(bool(on))))
 
     def set_group(self, group: int = 0):

@@ -9,7 +9,9 @@ enough that a full-section capture ends in a minute or two:
   group    k_fold_group32<MEA>: 2,432 x 200 nt drawn as the MEA workload (10 % mask)
   viterbi  k_viterbi64: 1,216 x 200 nt drawn as the MEA workload
   sample   k_inside32acc + k_sample32: 1,024 sequences drawn as the sampling workload x 10 samples
-  adj      k_adj_inside + k_adj_outside: 152 x 300 nt drawn as the gradient workload
+  adj      k_lin_inside32 + k_lin_outside32: 152 x 300 nt drawn as the gradient workload
+  logz     k_lin_inside32: 1,000 x 128 nt, no mask
+  latency  k_fold_cluster32: the inside of 4 x 997 nt
 """
 from __future__ import annotations
 
@@ -36,12 +38,16 @@ def run(case: str) -> None:
             s4, bonus = workloads.grad_300(152, 300)
             for _ in range(2):
                 grad.logz_grad(s4, None, list(bonus), engine=eng)
+        elif case in ("logz", "latency"):
+            B = Batch(workloads.as_strings(workloads.mea_200(*((1000, 128) if case == "logz" else (4, 997)))[0]))
+            for _ in range(2):
+                eng.logz(B)
         elif case == "group":
             B = Batch(seqs, masks)
             for _ in range(2):
                 eng.mea(B, 6.0)
         else:
-            raise SystemExit(f"unknown case {case!r}: group, viterbi, sample or adj")
+            raise SystemExit(f"unknown case {case!r}: group, viterbi, sample, adj, logz or latency")
     finally:
         eng.close()
 

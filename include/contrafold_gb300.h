@@ -93,11 +93,12 @@ int cf_engine_set_budget(cf_engine* eng, size_t bytes);
 int cf_engine_set_mode(cf_engine* eng, int mode);
 /* Batched-path schedule (the tuner's knob): kind 0 = automatic by length,
  * 1 = persistent warp-per-sequence kernel, 2 = persistent CTA-per-sequence
- * fused kernel, 3 = length-grouped per-phase kernels, 4 = cluster: each
- * sequence (or group, cf_engine_set_group) folded by the 8 CTAs of a
- * thread-block cluster on 8 SMs -- the latency of long sequences, for logZ,
- * BPP, MEA and sampling (kind 0 follows the schedule table,
- * cf_engine_load_tuning); ctas_per_sm caps the residency of the persistent
+ * fused kernel, 3 = length-grouped kernels (a sequence a CTA or cluster where
+ * the batch leaves most of the device idle), 4 = cluster: each sequence
+ * folded by the 8 CTAs of a thread-block cluster -- the latency of long
+ * sequences, for logZ, BPP, MEA and sampling (kind 0 follows the schedule
+ * table, cf_engine_load_tuning).  logZ of up to 512 nt, FP64 logZ of up to 416
+ * and Viterbi have kernels of their own on every kind; ctas_per_sm caps the residency of the persistent
  * CTA kernels (0 = automatic).  Results are identical for every choice.
  * Kind 5 (the queue schedule, cf_queue.cu) is disabled and returns
  * CF_EINVAL: its kernel did not finish in two GPU test runs. */
@@ -111,8 +112,9 @@ int cf_engine_set_schedule(cf_engine* eng, int kind, int ctas_per_sm);
  * counterpart. */
 int cf_engine_set_priority(cf_engine* eng, int high);
 /* on != 0: the device runs other engines' launches at the same time (the
- * serving loop's workers).  The engine then launches no 512-thread CTAs and
- * no thread-block clusters (the cluster schedule folds grouped instead):
+ * serving loop's workers).  The engine then folds in CTAs of at most 256
+ * threads and no thread-block clusters (the cluster schedule folds grouped
+ * instead; gradients keep theirs):
  * such a launch waits until a whole SM, or 8 SMs of one GPC, have room at
  * once, and between other engines' steady launches of smaller CTAs that took
  * seconds.  Results are identical.  No reference counterpart. */
