@@ -1673,7 +1673,9 @@ size_t cf_plan_arena_bytes(const cf_plan* p) { return p ? p->arena.cap * sizeof(
 
 int cf_plan_run(cf_plan* p, const uint8_t* d_seqs, const uint8_t* d_mask, float gamma, void* d_out, void* stream) {
     if (!p) return fail(CF_EINVAL, "plan is NULL");
-    if (p->n > 0 && (!d_out || (!d_seqs && p->P.Lmax > 0))) return fail(CF_EINVAL, "NULL device buffer");
+    // both parts of the plan: Lmax is 0 where every sequence takes the sum-of-products kernels
+    if (p->n > 0 && (!d_out || (!d_seqs && std::max(p->P.Lmax, p->P.lin_Lmax) > 0)))
+        return fail(CF_EINVAL, "NULL device buffer");
     if (p->job == JOB_MEA && !(gamma > 0.0f)) return fail(CF_EINVAL, "gamma must be > 0");
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : p->eng->stream;
     Exec X;

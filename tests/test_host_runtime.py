@@ -1,0 +1,69 @@
+"""The engine's host code over a CUDA runtime without a device (native/fake_cudart.cpp): what it refuses before a
+launch, what it copies and when, and the streams it makes.  Each check is a program of its own, with the fake runtime
+loaded before the library."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+REPO = os.path.dirname(HERE)
+
+PRELUDE = """
+import ctypes, os, sys
+import numpy as np
+fake = ctypes.CDLL(os.environ["LD_PRELOAD"])
+from contrafold_gpu_gb300 import params
+from contrafold_gpu_gb300.engine import *
+from contrafold_gpu_gb300.engine import Plan, Batch, Engine
+P = params.load()
+rng = np.random.default_rng(1)
+def seqs(*lens):
+    return ["".join(rng.choice(list("ACGU"), L)) for L in lens]
+eng = Engine(P)
+"""
+
+
+@pytest.fixture(scope="session")
+def run(tmp_path_factory):
+    from contrafold_gpu_gb300 import build
+    gxx = shutil.which("g++")
+    try:
+        cuda = os.path.dirname(os.path.dirname(build.nvcc()))
+        build.build()
+    except RuntimeError:
+        cuda = None
+    if not gxx or not cuda:
+        pytest.skip("compilers not available")
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.check_call([gxx, "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(cuda, "include"), "-o", so,
+                           os.path.join(HERE, "native", "fake_cudart.cpp")])
+
+    def go(body):
+        env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=REPO)
+        env.pop("CONTRAFOLD_GB300_LIB", None)
+        r = subprocess.run([sys.executable, "-c", PRELUDE + body], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+    return go
+
+
+def test_plan_run_refuses_null_buffers(run):
+    """Plans whose sequences take the sums of products alone, the other kernels alone, or both."""
+    run("""
+for lens in ((20, 40), (600,), (600, 40)):
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    for job in (CF_JOB_LOGZ, CF_JOB_LOGZ64, CF_JOB_BPP, CF_JOB_MEA, CF_JOB_MFE):
+        plan = Plan(eng, job, offs)
+        for graph, d_seqs, d_out in ((False, 0, 4096), (False, 4096, 0), (True, 0, 4096), (True, 4096, 0)):
+            plan.set_graph(graph)
+            try:
+                plan.run(d_seqs, 0, d_out)
+            except EngineError as e:
+                assert e.code == CF_EINVAL
+            else:
+                raise SystemExit(f"accepted: {lens}, job {job}")
+assert fake.fake_launches() == 0
+""")
