@@ -364,25 +364,23 @@ size_t budget_bytes(const cf_engine* eng) {
     return fr / 2;
 }
 
-// Weights of the sum-of-products kernels on the device.
-int ensure_weights(cf_engine* e, bool fp64) {
-    if (fp64) {
-        if (e->lin64.p) return CF_OK;
-        int rc = e->lin64.ensure(1);
-        if (rc) return rc;
-        cf::LinWeights<double> w;
-        cf::lin_weights(e->host64.data(), &w);
-        CF_CUDA(cudaMemcpyAsync(e->lin64.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
-    } else {
-        if (e->lin32.p) return CF_OK;
-        int rc = e->lin32.ensure(1);
-        if (rc) return rc;
-        cf::LinWeights<float> w;
-        cf::lin_weights(e->host64.data(), &w);
-        CF_CUDA(cudaMemcpyAsync(e->lin32.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
-    }
-    CF_CUDA(cudaStreamSynchronize(e->stream));   // once per parameter set: readable on every stream after it
+// Weights of the sum-of-products kernels, made of the parameters and copied to
+// the device.  Synchronises: the copy may read w until then, and the weights
+// are readable on every stream after it (once per parameter set).
+template <typename R>
+int upload_weights(cf_engine* e, DevBuf<cf::LinWeights<R>>& to, const double* params64) {
+    const int rc = to.ensure(1);
+    if (rc) return rc;
+    cf::LinWeights<R> w;
+    cf::lin_weights(params64, &w);
+    CF_CUDA(cudaMemcpyAsync(to.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
+    CF_CUDA(cudaStreamSynchronize(e->stream));
     return CF_OK;
+}
+
+int ensure_weights(cf_engine* e, bool fp64) {
+    if (fp64) return e->lin64.p ? CF_OK : upload_weights(e, e->lin64, e->host64.data());
+    return e->lin32.p ? CF_OK : upload_weights(e, e->lin32, e->host64.data());
 }
 
 int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<int> order, Plan& P);
@@ -1303,16 +1301,8 @@ int cf_engine_set_params(cf_engine* e, const float* params32, const double* para
     CF_CUDA(cudaMemcpyAsync(e->blob64.p, params64, sizeof(double) * CF_BLOB_LEN, cudaMemcpyHostToDevice, e->stream));
     e->host64.assign(params64, params64 + CF_BLOB_LEN);
     // weights made of the parameters before these: again, in place (plans and their graphs read them there)
-    if (e->lin32.p) {
-        cf::LinWeights<float> w;
-        cf::lin_weights(params64, &w);
-        CF_CUDA(cudaMemcpyAsync(e->lin32.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
-    }
-    if (e->lin64.p) {
-        cf::LinWeights<double> w;
-        cf::lin_weights(params64, &w);
-        CF_CUDA(cudaMemcpyAsync(e->lin64.p, &w, sizeof w, cudaMemcpyHostToDevice, e->stream));
-    }
+    if (e->lin32.p && (rc = upload_weights(e, e->lin32, params64))) return rc;
+    if (e->lin64.p && (rc = upload_weights(e, e->lin64, params64))) return rc;
     CF_CUDA(cudaStreamSynchronize(e->stream));
     return CF_OK;
 }

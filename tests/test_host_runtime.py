@@ -67,3 +67,17 @@ for lens in ((20, 40), (600,), (600, 40)):
                 raise SystemExit(f"accepted: {lens}, job {job}")
 assert fake.fake_launches() == 0
 """)
+
+
+def test_copied_parameters_live_until_the_copy(run):
+    """A host-to-device copy may read its source as late as the stream's next synchronisation."""
+    run("""
+B = Batch(seqs(30, 40))
+eng.logz(B)
+eng.logz64(B)        # both sets of weights exist from here on: set_params copies them again
+for k in range(3):
+    Q = {k: P[k] for k in params.TABLES + params.SCALARS}
+    Q["ep"] = Q["ep"] + 0.5 * k
+    eng.set_params(Q)
+assert fake.fake_changed_sources() == 0, fake.fake_changed_sources()
+""")
