@@ -304,7 +304,6 @@ struct cf_engine {
     int sched = 0;       // batched schedule: 0 auto, 1 warp-persistent, 2 CTA-persistent, 3 grouped, 4 cluster
     int ctas_per_sm = 0; // CTA-persistent occupancy cap (0 = auto)
     int group = 0;       // sequences per CTA of the grouped kernels (0 = auto)
-    size_t smem_optin = 0;
     std::vector<TuneRow> tuning = default_tuning();   // schedule table of the automatic path
     int grad_ckpt = 0;   // FM2 checkpoint spacing of cf_grad (0 = automatic by the longest sequence)
     bool shared = false; // the device is shared with other engines' launches: CTAs of 256 threads, no clusters
@@ -321,7 +320,7 @@ int group_for_length(int L) {
     return 1;
 }
 
-int ensure_smem(cf_engine* eng, size_t bytes);
+int ensure_smem(cf_engine* eng, size_t bytes, const std::vector<const void*>& kernels);
 
 struct Plan {
     bool plain = false;           // reference launch shape (mode 0): cf_plain.cu kernels for BPP/MEA
@@ -523,7 +522,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         const int mode = job == JOB_LOGZ ? cf::kQueueLogZ : job == JOB_MEA ? cf::kQueueMea
                        : job == JOB_BPP ? cf::kQueueBpp : cf::kQueueSample;
         const size_t smem = cf::queue_smem_bytes(P.Lmax, seats, mode);
-        int rc = ensure_smem(eng, smem);
+        int rc = ensure_smem(eng, smem, {cf::queue_kernel(mode)});
         if (rc) return rc;
         int per_sm = 0, sms = 0;
         CF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf::queue_kernel(mode), cf::kQueueThreads, smem));
@@ -547,7 +546,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
     if (P.cta) {
         const int mode = job == JOB_LOGZ ? cf::kCtaLogZ : job == JOB_MEA ? cf::kCtaMea : cf::kCtaBpp;
         const size_t smem = cf::fold_smem_bytes(P.Lmax, 1, false);
-        int rc = ensure_smem(eng, smem);
+        int rc = ensure_smem(eng, smem, {cf::cta_kernel(mode)});
         if (rc) return rc;
         int per_sm = 0, sms = 0;
         CF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf::cta_kernel(mode), cf::kFoldThreads, smem));
@@ -575,7 +574,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         const int mode = job == JOB_LOGZ ? cf::kWarpLogZ : job == JOB_MEA ? cf::kWarpMea
                        : job == JOB_BPP ? cf::kWarpBpp : cf::kWarpSample;
         const size_t smem = cf::warp_smem_bytes(P.Lmax);
-        int rc = ensure_smem(eng, smem);
+        int rc = ensure_smem(eng, smem, {cf::warp_kernel(mode)});
         if (rc) return rc;
         int per_sm = 0, sms = 0;
         CF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf::warp_kernel(mode), cf::kWarpThreads, smem));
@@ -664,30 +663,42 @@ int check_batch(cf_engine* eng, const uint8_t* seqs, const int64_t* offsets, int
     return CF_OK;
 }
 
-int ensure_smem(cf_engine* eng, size_t bytes) {
-    // set even below 48 KB: static shared memory (the cp.async chain ring)
-    // counts against the same 48 KB default limit
-    if (eng->smem_optin != 0 && bytes <= eng->smem_optin) return CF_OK;
+// Before a launch: the dynamic shared-memory limit of the kernels that will
+// run, and of no other (a kernel with static shared memory of its own cannot be
+// raised as far).  Set even below 48 KB: static shared memory (the cp.async
+// chain ring) counts against the same 48 KB default limit.
+int ensure_smem(cf_engine* eng, size_t bytes, const std::vector<const void*>& kernels) {
     bytes = std::max<size_t>(bytes, 48 * 1024);
     int dev_max = 0;
     CF_CUDA(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, eng->device));
     if ((size_t)dev_max < bytes) return fail(CF_EINVAL, "sequence too long for shared-memory staging");
-    std::vector<const void*> ks = {(const void*)cf::k_plain_inside32, (const void*)cf::k_plain_outside32,
-                                   (const void*)cf::k_plain_posterior32, (const void*)cf::k_plain_mea32,
-                                   (const void*)cf::k_inside64, (const void*)cf::k_viterbi64,
-                                   (const void*)cf::k_viterbi_cluster64};
-    const cf::FoldKernels fk = cf::fold_kernels();
-    for (cf::FoldKernel k : {fk.inside, fk.inside_acc, fk.outside, fk.posterior, fk.mea, fk.fused_mea, fk.fused_bpp,
-                             fk.fused_mea_shared})
-        ks.push_back((const void*)k);
-    for (int mode = 0; mode < 4; ++mode) ks.push_back(cf::warp_kernel(mode));
-    for (int mode = 0; mode < 3; ++mode) ks.push_back(cf::cta_kernel(mode));
-    for (const void* k : ks) {
+    for (const void* k : kernels) {
         const int rc = raise_smem_limit(k, eng->device, bytes);
         if (rc) return rc;
     }
-    eng->smem_optin = bytes;
     return CF_OK;
+}
+
+// The kernels of a batch of slices (no persistent or latency kernel): fused ones, and the per-phase ones of a timed run.
+std::vector<const void*> slice_kernels(Job job, const Plan& P) {
+    const cf::FoldKernels fk = cf::fold_kernels();
+    std::vector<const void*> ks;
+    auto add = [&](std::initializer_list<cf::FoldKernel> more) {
+        for (cf::FoldKernel k : more) ks.push_back((const void*)k);
+    };
+    switch (job) {
+        case JOB_LOGZ64: add({cf::k_inside64}); break;
+        case JOB_MFE: add({P.ctas > 1 ? cf::k_viterbi_cluster64 : cf::k_viterbi64}); break;
+        case JOB_BPP:
+        case JOB_MEA:
+            if (P.plain) ks = {(const void*)cf::k_plain_inside32, (const void*)cf::k_plain_outside32,
+                               (const void*)cf::k_plain_posterior32, (const void*)cf::k_plain_mea32};
+            else if (job == JOB_BPP) add({fk.fused_bpp, fk.inside, fk.outside, fk.posterior});
+            else add({fk.fused_mea, fk.fused_mea_shared, fk.inside, fk.outside, fk.posterior, fk.mea});
+            break;
+        default: add({fk.inside_acc});
+    }
+    return ks;
 }
 
 int ensure_lat_smem(cf_engine* eng, const Plan& P) {
@@ -895,7 +906,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         A.status = X.status;
         const int mode = job == JOB_LOGZ ? cf::kCtaLogZ : job == JOB_MEA ? cf::kCtaMea : cf::kCtaBpp;
         const size_t smem = cf::fold_smem_bytes(P.Lmax, 1, false);
-        if ((rc = ensure_smem(eng, smem))) return rc;
+        if ((rc = ensure_smem(eng, smem, {cf::cta_kernel(mode)}))) return rc;
         CF_CUDA(cudaMemsetAsync(X.status + 1, 0, sizeof(int), st));
         int* counter = X.status + 1;
         int64_t slot_words = P.slot_words;
@@ -929,7 +940,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         const int mode = job == JOB_LOGZ ? cf::kQueueLogZ : job == JOB_MEA ? cf::kQueueMea
                        : job == JOB_BPP ? cf::kQueueBpp : cf::kQueueSample;
         const size_t smem = cf::queue_smem_bytes(P.Lmax, P.seats, mode);
-        if ((rc = ensure_smem(eng, smem))) return rc;
+        if ((rc = ensure_smem(eng, smem, {cf::queue_kernel(mode)}))) return rc;
         CF_CUDA(cudaMemsetAsync(X.status + 1, 0, sizeof(int), st));
         void* args[] = {&Q};
         CF_PHASE(0, (cudaLaunchKernel(cf::queue_kernel(mode), dim3(P.wgrid), dim3(cf::kQueueThreads), args, smem, st)));
@@ -960,7 +971,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         const int mode = job == JOB_LOGZ ? cf::kWarpLogZ : job == JOB_MEA ? cf::kWarpMea
                        : job == JOB_BPP ? cf::kWarpBpp : cf::kWarpSample;
         const size_t smem = cf::warp_smem_bytes(P.Lmax);
-        if ((rc = ensure_smem(eng, smem))) return rc;
+        if ((rc = ensure_smem(eng, smem, {cf::warp_kernel(mode)}))) return rc;
         CF_CUDA(cudaMemsetAsync(X.status + 1, 0, sizeof(int), st));
         void* args[] = {&W};
         CF_PHASE(0, (cudaLaunchKernel(cf::warp_kernel(mode), dim3(P.wgrid), dim3(cf::kWarpThreads), args, smem, st)));
@@ -968,7 +979,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
     }
     const bool fp64 = job == JOB_LOGZ64 || job == JOB_MFE;
     const size_t smem = cf::fold_smem_bytes(P.Lmax, P.group, fp64);
-    if ((rc = ensure_smem(eng, std::max(smem, cf::plain_smem_bytes(P.Lmax))))) return rc;
+    if ((rc = ensure_smem(eng, std::max(smem, cf::plain_smem_bytes(P.Lmax)), slice_kernels(job, P)))) return rc;
     if (P.lat && (rc = ensure_lat_smem(eng, P))) return rc;
 
     for (size_t s = 0; s + 1 < P.slice_begin.size(); ++s) {
@@ -1564,29 +1575,28 @@ namespace {
 // Shared memory run_device will ask for: set before a stream capture, which
 // then records kernel launches only.
 int plan_prepare_smem(cf_engine* e, Job job, const Plan& P, LinStreams* S) {
-    size_t bytes;
     if (!P.lin_begin.empty()) {
         const int rc = prepare_linear(e, job, P, S);
         if (rc) return rc;
         if (P.n_fold == 0) return CF_OK;
     }
-    if (P.cta) {
-        bytes = cf::fold_smem_bytes(P.Lmax, 1, false);
-    } else if (P.warp) {
-        bytes = cf::warp_smem_bytes(P.Lmax);
-    } else if (P.queue) {
-        const int mode = job == JOB_LOGZ ? cf::kQueueLogZ : job == JOB_MEA ? cf::kQueueMea
-                       : job == JOB_BPP ? cf::kQueueBpp : cf::kQueueSample;
-        bytes = cf::queue_smem_bytes(P.Lmax, P.seats, mode);
-    } else {
-        const bool fp64 = job == JOB_LOGZ64 || job == JOB_MFE;
-        bytes = std::max(cf::fold_smem_bytes(P.Lmax, P.group, fp64), cf::plain_smem_bytes(P.Lmax));
-        if (P.lat) {
-            const int rc = ensure_lat_smem(e, P);
-            if (rc) return rc;
-        }
+    if (P.cta)
+        return ensure_smem(e, cf::fold_smem_bytes(P.Lmax, 1, false),
+                           {cf::cta_kernel(job == JOB_LOGZ ? cf::kCtaLogZ : job == JOB_MEA ? cf::kCtaMea : cf::kCtaBpp)});
+    if (P.warp)
+        return ensure_smem(e, cf::warp_smem_bytes(P.Lmax),
+                           {cf::warp_kernel(job == JOB_LOGZ ? cf::kWarpLogZ : job == JOB_MEA ? cf::kWarpMea : cf::kWarpBpp)});
+    if (P.queue) {
+        const int mode = job == JOB_LOGZ ? cf::kQueueLogZ : job == JOB_MEA ? cf::kQueueMea : cf::kQueueBpp;
+        return ensure_smem(e, cf::queue_smem_bytes(P.Lmax, P.seats, mode), {cf::queue_kernel(mode)});
     }
-    return ensure_smem(e, bytes);
+    if (P.lat) {
+        const int rc = ensure_lat_smem(e, P);
+        if (rc) return rc;
+    }
+    const bool fp64 = job == JOB_LOGZ64 || job == JOB_MFE;
+    return ensure_smem(e, std::max(cf::fold_smem_bytes(P.Lmax, P.group, fp64), cf::plain_smem_bytes(P.Lmax)),
+                       slice_kernels(job, P));
 }
 
 }  // namespace
@@ -1771,7 +1781,7 @@ namespace cf {
 int engine_device(const cf_engine* e) { return e->device; }
 cudaStream_t engine_stream(const cf_engine* e) { return e->stream; }
 const float* engine_blob32(const cf_engine* e) { return e->blob32.p; }
-int engine_ensure_smem(cf_engine* e, size_t bytes) { return ensure_smem(e, bytes); }
+int engine_ensure_smem(cf_engine* e, size_t bytes, const void* kernel) { return ensure_smem(e, bytes, {kernel}); }
 int engine_fail(int code, const char* msg) { return fail(code, msg); }
 
 }  // namespace cf

@@ -176,7 +176,7 @@ extern "C" int cf_mea_scratch(cf_engine* e, const uint8_t* seqs, const int64_t* 
 
     const int mode = cf::kWarpMea;
     const size_t smem = cf::warp_smem_bytes(Lmax);
-    int rc = cf::engine_ensure_smem(e, smem);
+    int rc = cf::engine_ensure_smem(e, smem, cf::warp_kernel(mode));
     if (rc) return rc;
     int per_sm = 0, sms = 0;
     CF_CUDA_S(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf::warp_kernel(mode), cf::kWarpThreads, smem));
