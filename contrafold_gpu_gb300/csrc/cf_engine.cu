@@ -1618,12 +1618,12 @@ int cf_plan_create(cf_engine* e, int32_t job, const int64_t* offsets, int32_t n,
     p->n = n;
     rc = make_plan(e, p->job, offsets, n, p->P);
     if (!rc && n > 0 && p->P.n_fold == 0) {
-        // every sequence takes the sum-of-products kernels: the schedule the batch is tuned to is still what
-        // cf_plan_schedule and cf_plan_group report
+        // Every sequence takes the sum-of-products kernels.  What cf_plan_schedule and cf_plan_group report is still
+        // the schedule the batch is tuned to; where that one has no room, it is the default.
         Plan S;
         std::vector<int> all(n);
         std::iota(all.begin(), all.end(), 0);
-        if (!(rc = make_fold_plan(e, p->job, offsets, std::move(all), S))) {
+        if (make_fold_plan(e, p->job, offsets, std::move(all), S) == CF_OK) {
             p->P.plain = S.plain; p->P.cta = S.cta; p->P.warp = S.warp; p->P.cluster = S.cluster; p->P.group = S.group;
         }
     }

@@ -81,3 +81,26 @@ for k in range(3):
     eng.set_params(Q)
 assert fake.fake_changed_sources() == 0, fake.fake_changed_sources()
 """)
+
+
+def test_plan_of_sums_needs_no_room_for_other_kernels(run):
+    """A budget that holds what the plan launches is enough, whatever the schedule it reports would need; one that
+    does not hold the longest sequence is refused, as by the call itself."""
+    run("""
+B = Batch(seqs(*[120] * 64))
+eng.set_schedule("group")
+eng.set_group(32)
+eng.set_budget(1 << 20)                  # one sequence's tables are 100 KB
+eng.logz(B)
+plan = Plan(eng, CF_JOB_LOGZ, B.offsets)
+assert plan.schedule == "group", plan.schedule
+plan.run(4096, 0, 8192)
+eng.set_budget(1 << 14)
+for call in (lambda: eng.logz(B), lambda: Plan(eng, CF_JOB_LOGZ, B.offsets)):
+    try:
+        call()
+    except EngineError as e:
+        assert e.code == CF_ENOMEM
+    else:
+        raise SystemExit("accepted")
+""")
