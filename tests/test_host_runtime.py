@@ -104,3 +104,17 @@ for call in (lambda: eng.logz(B), lambda: Plan(eng, CF_JOB_LOGZ, B.offsets)):
     else:
         raise SystemExit("accepted")
 """)
+
+
+def test_gradient_result_is_a_plain_record(run):
+    """Positional construction, asdict and replace; d_theta is the counts through the tying."""
+    run("""
+import dataclasses
+from contrafold_gpu_gb300 import grad
+assert [f.name for f in dataclasses.fields(grad.GradResult)] == ["logz", "d_blob", "d_theta", "d_bonus"]
+r = grad.logz_grad(seqs(20, 30), engine=eng)
+assert set(dataclasses.asdict(r)) == {"logz", "d_blob", "d_theta", "d_bonus"}
+assert np.array_equal(r.d_theta, r.d_blob @ grad.tying_jacobian()) and r.d_theta.shape[0] == 2
+assert dataclasses.replace(r, logz=None).d_theta is r.d_theta
+assert grad.GradResult(1, 2, 3, 4).d_bonus == 4
+""")
