@@ -236,20 +236,26 @@ const TuneRow* match_tuning(const std::vector<TuneRow>& rows, Job job, int n, in
 namespace {
 // Side streams of the sum-of-products inside: its length classes run at the
 // same time, each with its own shared memory.  Made at the first batch of
-// several classes; every owner (an engine's calls, a plan) has its own, so
+// several classes, with the priority of the stream they work beside, and again
+// when that changes; every owner (an engine's calls, a plan) has its own, so
 // runs of different plans never share an event.
 struct LinStreams {
     static constexpr int kSide = 4;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork = nullptr, join[kSide] = {};
-    int ensure() {
-        if (fork) return CF_OK;
+    int priority = 0;
+    int ensure(cudaStream_t beside) {
+        int now = 0;
+        CF_CUDA(cudaStreamGetPriority(beside, &now));
+        if (fork && now == priority) return CF_OK;
+        release();   // (work in flight on a destroyed stream completes)
+        priority = now;
         cudaEvent_t f = nullptr;
-        CF_CUDA(cudaEventCreateWithFlags(&f, cudaEventDisableTiming));
         for (int k = 0; k < kSide; ++k) {
-            if (!side[k]) CF_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
-            if (!join[k]) CF_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
+            CF_CUDA(cudaStreamCreateWithPriority(&side[k], cudaStreamNonBlocking, priority));
+            CF_CUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
         }
+        CF_CUDA(cudaEventCreateWithFlags(&f, cudaEventDisableTiming));
         fork = f;
         return CF_OK;
     }
@@ -787,7 +793,7 @@ struct Exec {
 
 // Before the launches of a plan (and outside a stream capture): shared-memory
 // limits and side streams of its sum-of-products inside.
-int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S) {
+int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S, cudaStream_t st) {
     const bool fp64 = job == JOB_LOGZ64, train = job == JOB_GRAD;
     int classes = 0;
     for (size_t k = P.n_fold; k < P.descs.size(); ++classes) {
@@ -796,7 +802,7 @@ int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S) {
         if (rc) return rc;
         while (k < P.descs.size() && cf::lin_class_end(P.descs[k].L, fp64) == cf::lin_class_end(L, fp64)) ++k;
     }
-    return classes > 1 ? S->ensure() : CF_OK;
+    return classes > 1 ? S->ensure(st) : CF_OK;
 }
 
 // The inside of descs [k0, k1), sorted by falling length: a launch for each
@@ -837,7 +843,7 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
                float* d_logz, double* d_logz64, cudaStream_t st) {
     int rc;
     const bool fp64 = job == JOB_LOGZ64;
-    if ((rc = prepare_linear(eng, job, P, X.lin_streams))) return rc;
+    if ((rc = prepare_linear(eng, job, P, X.lin_streams, st))) return rc;
     const size_t redo = cf::fold_smem_bytes(P.lin_Lmax, 1, fp64);
     int sms = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
@@ -1487,7 +1493,7 @@ extern "C" int cf_grad(cf_engine* e, const uint8_t* seqs, const int64_t* offsets
     if ((rc = e->arena.ensure((size_t)P.arena_words()))) return rc;
     const size_t smem = cf::adj_smem_bytes(std::max(P.Lmax, P.lin_Lmax));
     const size_t out_smem = cf::lin_outside_smem_bytes(P.lin_Lmax);
-    if ((rc = prepare_linear(e, JOB_GRAD, P, &e->lin_streams))) return rc;
+    if ((rc = prepare_linear(e, JOB_GRAD, P, &e->lin_streams, st))) return rc;
     {
         int dev_max = 0;
         CF_CUDA(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
@@ -1574,9 +1580,9 @@ namespace {
 
 // Shared memory run_device will ask for: set before a stream capture, which
 // then records kernel launches only.
-int plan_prepare_smem(cf_engine* e, Job job, const Plan& P, LinStreams* S) {
+int plan_prepare_smem(cf_engine* e, Job job, const Plan& P, LinStreams* S, cudaStream_t st) {
     if (!P.lin_begin.empty()) {
-        const int rc = prepare_linear(e, job, P, S);
+        const int rc = prepare_linear(e, job, P, S, st);
         if (rc) return rc;
         if (P.n_fold == 0) return CF_OK;
     }
@@ -1694,7 +1700,7 @@ int cf_plan_run(cf_plan* p, const uint8_t* d_seqs, const uint8_t* d_mask, float 
         const bool hit = p->gexec != nullptr && p->g_seqs == d_seqs && p->g_mask == d_mask && p->g_out == d_out &&
                          p->g_gamma == gamma;
         if (!hit) {   // (re)capture the launches of one run
-            int rc = plan_prepare_smem(p->eng, p->job, p->P, &p->lin_streams);
+            int rc = plan_prepare_smem(p->eng, p->job, p->P, &p->lin_streams, st);
             if (rc) return rc;
             if (p->gexec) {
                 CF_CUDA(cudaGraphExecDestroy(p->gexec));

@@ -48,6 +48,11 @@ extern "C" {
 int fake_changed_sources() { return changed; }
 int fake_launches() { return launches; }
 int fake_streams_of(int priority) { return made[-priority]; }   // created so far with this priority
+void* fake_stream(int priority) {
+    cudaStream_t s;
+    make_stream(&s, priority);
+    return s;
+}
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }

@@ -15,6 +15,7 @@ PRELUDE = """
 import ctypes, os, sys
 import numpy as np
 fake = ctypes.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_stream.restype = ctypes.c_void_p
 from contrafold_gpu_gb300 import params
 from contrafold_gpu_gb300.engine import *
 from contrafold_gpu_gb300.engine import Plan, Batch, Engine
@@ -117,4 +118,32 @@ assert set(dataclasses.asdict(r)) == {"logz", "d_blob", "d_theta", "d_bonus"}
 assert np.array_equal(r.d_theta, r.d_blob @ grad.tying_jacobian()) and r.d_theta.shape[0] == 2
 assert dataclasses.replace(r, logz=None).d_theta is r.d_theta
 assert grad.GradResult(1, 2, 3, 4).d_bonus == 4
+""")
+
+
+def test_side_streams_have_the_callers_priority(run):
+    """Length classes beside the first one run at the priority of the stream that the call or the run is on."""
+    run("""
+offs = Batch(seqs(20, 120, 220, 380, 500)).offsets
+B = Batch(seqs(20, 120, 220, 380, 500))
+LEAST, GREATEST = 0, -5
+def made():
+    return fake.fake_streams_of(LEAST), fake.fake_streams_of(GREATEST)
+least, greatest = made()
+eng.logz(B)
+assert made()[0] > least and made()[1] == greatest == 0
+eng.set_priority(True)                   # the engine's own high-priority stream, then its side streams
+least = made()[0]
+own = made()[1]
+eng.logz(B)
+assert made()[0] == least and made()[1] > own
+greatest = made()[1]
+eng.logz(B)
+assert made() == (least, greatest)       # kept between calls
+plan = Plan(eng, CF_JOB_LOGZ, offs)
+for graph in (False, True):
+    plan.set_graph(graph)
+    stream = fake.fake_stream(-3)
+    plan.run(4096, 0, 8192, 6.0, stream)
+    assert fake.fake_streams_of(-3) > 1
 """)
