@@ -247,12 +247,14 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
     const int gs = Y.gs, cs = Y.cs;
     constexpr int SP = kSplitParts<R>;
 
-    // tables in the arena: FM and FM1 by diagonals, E by rows, for gradients the pairs by diagonals
+    // tables in the arena: FM and FM1 by diagonals, then the pairs' ends E by rows; for gradients FM2 and the pairs
+    // by diagonals instead (E is their product with the end weights)
     R* base = reinterpret_cast<R*>(A.ws + D.ws_off);
     const int64_t tri = pad32(tri_size(L));
     R* FM = base;
     R* FM1 = base + tri;
     R* E = base + 2 * tri;
+    R* F2 = base + 2 * tri;
     R* Bt = base + 3 * tri;
 
     {   // weights
@@ -354,8 +356,12 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
             Gd[i] = gg;
             Bd[i] = b;
             Md[i] = mm1;
-            if constexpr (TRAIN) Bt[off + i] = b;
-            E[e_row(i, L) + d] = mm1;   // b - a - 1 = d
+            if constexpr (TRAIN) {
+                F2[off + i] = f2;
+                Bt[off + i] = b;
+            } else {
+                E[e_row(i, L) + d] = mm1;   // b - a - 1 = d
+            }
         }
         if constexpr (sizeof(R) == 8) {   // pairable cells of the next diagonal
             if (warp == (NT / 32) - 1) {
@@ -378,7 +384,11 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
     R acc0 = R(0), acc1 = R(0), f = R(1);
     const int j0 = tid + 1, j1 = tid + 1 + NT;   // NT >= 256, L <= 512
     const R euk = w.eu * R(CF_LIN_SCALE);
-    auto row = [&](int a, int j) -> R { return (a < L && j > a && j <= L) ? E[e_row(a, L) + j - a - 1] : R(0); };
+    auto row = [&](int a, int j) -> R {
+        if (a >= L || j <= a || j > L) return R(0);
+        return TRAIN ? Bt[tri_off(j - a - 1, m) + a] : E[e_row(a, L) + j - a - 1];
+    };
+    auto ended = [&](R v, int a, int j) -> R { return TRAIN && v != R(0) ? v * w_end(w, s, L, a, j) : v; };
     R n0[4], n1[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -391,7 +401,7 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
         for (int u = 0; u < 4; ++u) {
             const int k = k0 + u;
             if (k < L) {   // uniform over the CTA
-                const R e0 = n0[u], e1 = n1[u];
+                const R e0 = ended(n0[u], k + 1, j0), e1 = ended(n1[u], k + 1, j1);
                 n0[u] = row(k + 5, j0);
                 if (L > NT) n1[u] = row(k + 5, j1);
                 const R fe = f * w.ep;
@@ -589,7 +599,7 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
     const int64_t tri = pad32(tri_size(L));
     const float* FM = base;
     const float* FM1 = base + tri;
-    float* E = base + 2 * tri;             // by rows; its place is taken by two (by diagonals) after the exterior pass
+    float* two = base + 2 * tri;           // FM2; a cell's derivative takes its place
     const float* Bt = base + 3 * tri;
     const float* F5 = base + 4 * tri;
     if (F5[L + 1] == 0.f) return;         // on the list already
@@ -631,7 +641,7 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
         const float invZ = 1.0f / F5[L];
         float acc = 0.f, f = invZ;
         if (tid == 0) F5o[L] = invZ;
-        auto col = [&](int j) -> float { return (j > tid + 1 && tid + 1 < L && j <= L) ? E[e_row(tid + 1, L) + j - tid - 2] : 0.f; };
+        auto col = [&](int j) -> float { return (j > tid + 1 && tid + 1 < L && j <= L) ? Bt[tri_off(j - tid - 2, m) + tid + 1] : 0.f; };
         float nx[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) nx[u] = col(L - u);
@@ -640,7 +650,7 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
             for (int u = 0; u < 4; ++u) {
                 const int j = j0 - u;   // F5o[j] = f known: to all earlier positions, then F5o[j - 1]
                 if (j >= 1) {
-                    const float e = nx[u];
+                    const float e = nx[u] != 0.f ? nx[u] * w_end(w, s, L, tid + 1, j) : 0.f;
                     nx[u] = col(j - 4);
                     acc = fmaf(f * w.ep, e, acc);
                     if (tid == j - 1) F5o[j - 1] = fmaf(f, euk, acc);
@@ -651,7 +661,6 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
         }
     }
     __syncthreads();
-    float* two = E;
 
     // G of the 32 longest diagonals
     auto load_G = [&](int r, int a) {
@@ -673,12 +682,10 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
     for (int k = 0; k < 12; ++k) cD[k] = 0.f;
     // this thread's sums over its cells
     float s_mu = 0.f, s_one = 0.f, s_multi = 0.f, s_ext = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, s_hp = 0.f, end_last = 0.f;
-    // of this thread's last pair: the row of its bases (-1: none), its hairpin and small loops, and what neither they
-    // nor its stack account for
-    struct {
+    struct {   // of this thread's last pair: the row of its bases (-1: none), its hairpin and small loops
         int y;
-        float loops, rest;
-    } before = {-1, 0.f, 0.f};
+        float loops;
+    } before = {-1, 0.f};
     __syncthreads();
 
     for (int d = L - 2; d >= -1; --d) {
@@ -726,17 +733,13 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
         if (tid == 0) h->ctr[(d & 1) ^ 1] = 0;
         const float kd = scale_pow<float>(max(d, 0));
         const int i = 1 + tid;
-        // The loop sum of this thread's pair of diagonal d + 1, for its close weight's count.  What the pair's
-        // probability leaves after its stack, hairpin and interior loops is its multiloop's: FM2 is not needed again.
+        // the loop sum of this thread's pair of diagonal d + 1, for its close weight's count
         if (d + 1 >= 0 && i <= c - 1 && before.y >= 0) {
             float win = 0.f;
             if (d + 1 >= 4) {
 #pragma unroll
                 for (int p = 0; p < kParts; ++p) win += Wp[p * cs + i - 1];
                 win *= gr[((d + 1) & (kRing - 1)) * go + i + 32];
-                const float v_multi = before.rest - win;
-                more[(kRowMulti - kOwnRows + before.y) * rs + i] += v_multi;
-                s_multi += v_multi;
             }
             rows[(kRowClose + before.y) * cs + i] += before.loops + win;
         }
@@ -796,10 +799,14 @@ __global__ void __launch_bounds__(kLinOutThreads, 1) k_lin_outside32(LinArgs A) 
                     v10 = gv * K1 * w.cs10 * w.b01[si1] * G3[i + 2];
                 }
                 if (d >= 4) v11 = gv * k2 * w.cs11 * w.i11[si1 * 5 + sj] * G[((d - 4) & (kRing - 1)) * gs + 2 + i + 2];
+                // (the multiloop as a product: what the other loops leave of P loses a rare one's digits, 9e-3 of the
+                // count at 20 nt, 4e-4 at 30)
+                const float v_multi = fm * two[off + i];
                 const int y1 = side(sb) * 5 + sj, y2 = side(sb) * 5 + sr;
                 before.loops = v_hp + v01 + v10 + v11;
-                before.rest = P - v_st - before.loops;
                 before.y = y1;
+                more[(kRowMulti - kOwnRows + y1) * rs + i] += v_multi;
+                s_multi += v_multi;
                 rows[(kRowV01 + sj) * cs + i] += v01;
                 rows[(kRowV11 + sj) * cs + i] += v11;
                 more[(kRowStack - kOwnRows + y1) * rs + i] += v_st;
