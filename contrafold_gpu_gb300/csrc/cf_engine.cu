@@ -347,6 +347,8 @@ struct Plan {
     int Lmax = 0;
     int n_fold = 0;               // descs [0, n_fold) take the kernels above; the rest, sorted by falling length,
     int lin_Lmax = 0;             // the sum-of-products kernels (longest length, arena slices)
+    int lin_redo = 1;             // what leaves their range: sequences a CTA at most,
+    bool lin_mixed = false;       // and whether lengths differ by more than 25 %
     std::vector<int> lin_begin;
     int64_t arena_words() const {
         int64_t w = 1;
@@ -415,6 +417,8 @@ int make_plan(cf_engine* eng, Job job, const int64_t* offsets, int n, Plan& P) {
     int rc = ensure_weights(eng, job == JOB_LOGZ64);
     if (rc) return rc;
     P.lin_Lmax = len(lin[0]);
+    P.lin_mixed = P.lin_Lmax > len(lin.back()) + len(lin.back()) / 4;
+    P.lin_redo = eng->mode != 1 ? 1 : P.lin_mixed ? group_for_length(len(lin[lin.size() / 2])) : cf::kMaxGroup;
     const int64_t most = (int64_t)(budget_bytes(eng) / 4);
     int64_t cur = 0, widest = 0;
     P.lin_begin.push_back(P.n_fold);
@@ -802,6 +806,11 @@ int prepare_linear(cf_engine* eng, Job job, const Plan& P, LinStreams* S, cudaSt
         if (rc) return rc;
         while (k < P.descs.size() && cf::lin_class_end(P.descs[k].L, fp64) == cf::lin_class_end(L, fp64)) ++k;
     }
+    if (classes > 0 && !train) {
+        const int rc = raise_smem_limit(fp64 ? (const void*)cf::k_inside_redo64 : (const void*)cf::k_inside_redo32, eng->device,
+                                        std::max<size_t>(cf::fold_smem_bytes(P.lin_Lmax, P.lin_redo, fp64), 48 * 1024));
+        if (rc) return rc;
+    }
     return classes > 1 ? S->ensure(st) : CF_OK;
 }
 
@@ -844,7 +853,6 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
     int rc;
     const bool fp64 = job == JOB_LOGZ64;
     if ((rc = prepare_linear(eng, job, P, X.lin_streams, st))) return rc;
-    const size_t redo = cf::fold_smem_bytes(P.lin_Lmax, 1, fp64);
     int sms = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
     for (size_t s = 0; s + 1 < P.lin_begin.size(); ++s) {
@@ -852,7 +860,7 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         cf::FoldArgs A{};
         A.descs = X.d_descs + k0;
         A.n = k1 - k0;
-        A.group = 1;
+        A.group = P.lin_redo;
         A.seqs = d_seqs;
         A.mask = d_mask;
         A.blob32 = eng->blob32.p;
@@ -874,8 +882,9 @@ int run_linear(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
         cudaEvent_t stop = nullptr;
         if (X.timer && (rc = X.timer->begin(0, st, &stop))) return rc;
         if ((rc = launch_lin_inside(eng, P, La, k0, k1, fp64, false, X.lin_streams, st, X.launches))) return rc;
-        if (fp64) cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
-        else cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails);
+        const size_t redo = cf::fold_smem_bytes(P.lin_Lmax, P.lin_redo, fp64);
+        if (fp64) cf::k_inside_redo64<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails, P.lin_mixed);
+        else cf::k_inside_redo32<<<rgrid, cf::kFoldThreads, redo, st>>>(A, X.fails, P.lin_mixed);
         ++X.launches;
         CF_CUDA(cudaGetLastError());
         if (X.timer && (rc = X.timer->end(stop, st))) return rc;

@@ -159,39 +159,51 @@ __global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside64(FoldA
 }
 
 // Sequences that the sum-of-products kernels left (fails[0] of them, descs
-// indices fails[1 ..]; usually none), one CTA each, in the log domain.
+// indices fails[1 ..]; usually none), in the log domain.  How many there are is
+// known here only, so each CTA takes as many of them together as the host's rule
+// gives a batch of that size, A.group at most: as few waves as that allows, or
+// two where lengths are mixed (GB300, the whole logZ call: 1,000 hairpins of 124
+// nt 20.2 ms with one a CTA in turn, 9.8 so; 500 of 304 nt 46.4, 35.3).
 template <class S>
-__device__ __forceinline__ void inside_redo(const FoldArgs& A, const int* fails, const typename S::Real* blob,
+__device__ __forceinline__ void inside_redo(const FoldArgs& A, const int* fails, bool mixed, const typename S::Real* blob,
                                             typename S::Real* out) {
     using R = typename S::Real;
-    const int n = fails[0];
-    if ((int)blockIdx.x >= n) return;
+    const int n = fails[0], slots = gridDim.x;
+    if (n == 0) return;
+    const int waves = (n + A.group * slots - 1) / (A.group * slots);
+    const int group = mixed ? min(A.group, max(1, (n + slots) / (2 * slots))) : (n + waves * slots - 1) / (waves * slots);
+    if ((int)blockIdx.x * group >= n) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* sm = reinterpret_cast<SmemFold<R>*>(smem_raw);
     load_tabs(&sm->tabs, blob);
     load_poly_tables(&sm->poly);
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    for (int k = blockIdx.x * group; k < n; k += slots * group) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            const SeqDesc D = A.descs[fails[1 + k]];
-            sm->L[0] = D.L;
-            sm->ws[0] = D.ws_off;
-            sm->soff[0] = D.seq_off;
-            sm->idx[0] = D.idx;
-            sm->n = sm->gcap = 1;
-            sm->Lmax = D.L;
+            sm->n = min(group, n - k);
+            sm->gcap = A.group;
+            sm->Lmax = 0;
+            for (int g = 0; g < sm->n; ++g) {
+                const SeqDesc D = A.descs[fails[1 + k + g]];
+                sm->L[g] = D.L;
+                sm->ws[g] = D.ws_off;
+                sm->soff[g] = D.seq_off;
+                sm->idx[g] = D.idx;
+                sm->Lmax = max(sm->Lmax, D.L);
+            }
         }
         __syncthreads();
         build_group_seqs(sm, A);
         inside_group<S>(sm, A);
-        if (threadIdx.x == 0) out[sm->idx[0]] = in_view<R>(A, sm->ws[0], sm->L[0]).T.F5[sm->L[0]];
+        for (int g = threadIdx.x; g < sm->n; g += blockDim.x)
+            out[sm->idx[g]] = in_view<R>(A, sm->ws[g], sm->L[g]).T.F5[sm->L[g]];
     }
 }
-__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo32(FoldArgs A, const int* fails) {
-    inside_redo<LseAcc32>(A, fails, A.blob32, A.logz);
+__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo32(FoldArgs A, const int* fails, bool mixed) {
+    inside_redo<LseAcc32>(A, fails, mixed, A.blob32, A.logz);
 }
-__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo64(FoldArgs A, const int* fails) {
-    inside_redo<Lse64>(A, fails, A.blob64, A.logz64);
+__global__ void __launch_bounds__(kFoldThreads, kFoldMinBlocks) k_inside_redo64(FoldArgs A, const int* fails, bool mixed) {
+    inside_redo<Lse64>(A, fails, mixed, A.blob64, A.logz64);
 }
 
 // ---------------------------------------------------------------------------

@@ -64,9 +64,9 @@ constexpr int kLatStaticSmem = 18 * 1024;   // at most, beside the grouped kerne
 __global__ void k_inside64(FoldArgs A);
 __global__ void k_viterbi64(FoldArgs A);           // one sequence a CTA ...
 __global__ void k_viterbi_cluster64(FoldArgs A);   // ... or a cluster (cf_viterbi.cu)
-// log-domain logZ of the sequences listed in fails (cf_linear.cu)
-__global__ void k_inside_redo32(FoldArgs A, const int* fails);
-__global__ void k_inside_redo64(FoldArgs A, const int* fails);
+// log-domain logZ of the sequences listed in fails (cf_linear.h), A.group at most on a CTA (cf_fold.cu)
+__global__ void k_inside_redo32(FoldArgs A, const int* fails, bool mixed);
+__global__ void k_inside_redo64(FoldArgs A, const int* fails, bool mixed);
 
 size_t fold_smem_bytes(int Lmax, int group, bool fp64);
 
