@@ -136,25 +136,30 @@ struct TuneRow {
 //  * small batches of long sequences fold on a thread-block cluster of 8 each:
 //    every sequence >= 512 nt and at most two of the clusters' CTAs per SM (38
 //    sequences on 152 SMs; 4 x 801 nt MEA 181 ms grouped, 65 ms so);
-//  * large batches of mixed short lengths take the warp-per-sequence kernel
-//    (200 nt: n=1024 warp 8.7k vs grouped 10.2k MEA folds/s, n=2048 15.1k vs
-//    13.3k; 60 nt: n=2048 172k vs 186k, n=4096 238k vs 191k);
 //  * sampling of large mixed batches up to 400 nt folds 4 sequences per CTA
 //    (4,096 x U{40..400} x 100 samples: 1.30M samples/s against 1.20M with
 //    the MEA-tuned length table's 2), where that leaves two waves of CTAs
-//    (3,648 sequences on 152 SMs);
+//    (3,648 sequences on 152 SMs); up to 256 nt from 1,900 on (10 samples,
+//    2 / 4 a CTA: 2,000 x 60-100 nt 13.8 / 10.0 ms, 2,000 x 100-200 nt 31 / 24),
+//    and 8 up to 128 nt (4 / 8: 3,648 x 60-100 nt 16.1 / 14.4, 6,000 27.8 / 22.7);
+//  * very many mixed short ones fold 16 per CTA instead of 8 (MEA of 30,000 x
+//    20-40 / 40-80 nt with 8, 16: 17.7, 15.5 / 63, 56 ms; posteriors alike);
 //  * everything else folds grouped (lengths within 25 %: one wave of full
-//    CTAs; mixed: several waves).
+//    CTAs; mixed: several waves).  The warp-per-sequence kernel, which large
+//    batches of mixed short lengths took, is slower there than groups (MEA,
+//    ms, warp / groups: 30,000 x 20-40 nt 37.7 / 17.7, 10,000 x 50-150 nt 87 /
+//    74, 4,096 x 100-256 nt 176 / 121; posteriors alike).
 std::vector<TuneRow> default_tuning() {
     const unsigned lbms = (1u << JOB_LOGZ) | (1u << JOB_BPP) | (1u << JOB_MEA) | (1u << JOB_SAMPLE);
-    const unsigned lbm = (1u << JOB_LOGZ) | (1u << JOB_BPP) | (1u << JOB_MEA);
     std::vector<TuneRow> t(5);
     t[0].min_len = 512; t[0].min_batch = 1; t[0].max_batch = 38; t[0].jobs = lbms; t[0].sched = 4;
-    t[1].max_len = 80; t[1].min_batch = 4096; t[1].uniform = 0; t[1].jobs = lbm; t[1].sched = 1;
-    t[2].max_len = 80; t[2].uniform = 0; t[2].jobs = lbm; t[2].sched = 3;
-    t[3].max_len = 256; t[3].min_batch = 2048; t[3].uniform = 0; t[3].jobs = lbm; t[3].sched = 1;
-    t[4].max_len = 400; t[4].min_batch = 3648; t[4].uniform = 0; t[4].jobs = 1u << JOB_SAMPLE; t[4].sched = 3;
-    t[4].group = 4;
+    auto mixed = [&](int row, int max_len, int min_batch, unsigned jobs, int group) {
+        t[row].max_len = max_len; t[row].min_batch = min_batch; t[row].uniform = 0; t[row].jobs = jobs; t[row].group = group;
+    };
+    mixed(1, 80, 16384, (1u << JOB_BPP) | (1u << JOB_MEA), 16);
+    mixed(2, 128, 3648, 1u << JOB_SAMPLE, 8);
+    mixed(3, 256, 1900, 1u << JOB_SAMPLE, 4);
+    mixed(4, 400, 3648, 1u << JOB_SAMPLE, 4);
     return t;
 }
 
@@ -453,13 +458,20 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         P.Lmax = std::max<int>(P.Lmax, (int)(offsets[b + 1] - offsets[b]));
         Lmin = std::min<int>(Lmin, (int)(offsets[b + 1] - offsets[b]));
     }
-    // lengths within 25 % of each other: the grouped kernels with whole waves
-    // of full CTAs beat the warp kernel (10,000 x 200 nt MEA: 27.7k vs 25.2k
-    // folds/s; 10,000 x 100 nt: 121k vs 109k); mixed lengths keep the warp
-    // kernel's per-sequence work queue (150-250 nt: 20.8k vs 15.1k)
+    // lengths within 25 % of each other
     const bool uniform = P.Lmax <= Lmin + Lmin / 4;
     const bool batched = eng->mode == 1 && job != JOB_GRAD;
     P.plain = !batched;
+    // Few enough for the latency kernels: a sequence on a cluster or, one after another on an SM, on CTAs of their own.
+    // They win until the grouped kernels' CTAs fill the device (GB300, ms, latency / grouped, MEA and 1 sample: 200 nt n =
+    // 304 19 / 24 and 10 / 13, 456 29 / 26 and 15 / 13; 100 nt n = 456 8.8 / 9.3 and 5.9 / 5.4; 320 nt n = 304 46 / 53, 456
+    // 70 / 59; 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA).  Not on a shared device: a
+    // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
+    int sms = 0;
+    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
+    const int cut = uniform ? (P.Lmax <= 128 ? 3 : 2) : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
+    const bool few = batched && !eng->shared && n <= cut * sms &&
+                     (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE);
     if (batched) {
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
             return offsets[x + 1] - offsets[x] > offsets[y + 1] - offsets[y];
@@ -471,10 +483,12 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         // per CTA); mixed lengths keep several waves so the long sequences' CTAs
         // do not set the end alone (40-400 nt: 11.8k with 2 per CTA, 6.5k with 9;
         // 25 samples of 1,024 / 2,048 x 40-400 nt with 1, 2, 4 per CTA: 60 / 117,
-        // 68 / 88, 92 / 118 ms; Viterbi 1,024 x 100-500 nt with 1, 2: 108, 139 ms)
+        // 68 / 88, 92 / 118 ms), but a short sequence leaves most of a CTA's
+        // threads without a cell, so at least as many go together as make two
+        // cells of a diagonal a thread, while every CTA has a group (MEA of 2,048
+        // x 15-25 nt with 1, 2, 4, 8: 2.0, 1.4, 1.2, 1.3 ms; 10 samples of 1,024 x
+        // 60-100 nt: 11.0, 7.5, 7.7, 8.3; 1,024 x 100-200 nt: 25.6, 17.4, 18.9, 26.4)
         const int Lmed = n ? (int)(offsets[order[n / 2] + 1] - offsets[order[n / 2]]) : 0;
-        int sms = 0;
-        CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
         // resident CTAs per SM of the kernel that will run: the fused MEA kernel
         // is built for more than the other grouped kernels
         const int slots =
@@ -482,9 +496,12 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         // whole waves: the fewest waves whose groups fit kMaxGroup sequences
         const int waves = std::max(1, (n + cf::kMaxGroup * slots - 1) / (cf::kMaxGroup * slots));
         const int wave_group = std::min(cf::kMaxGroup, std::max(1, (n + waves * slots - 1) / (waves * slots)));
-        const int wave2 = std::min(cf::kMaxGroup, std::max(1, n / (2 * slots)));   // two whole waves at least
+        // two waves: whole ones at least (MEA of 2,048 x 40-400 nt, 1.7 of two, with 1, 2: 135, 144 ms), for the inside
+        // alone about two (10 samples of 1,500 x 40-400 nt, 1.6 of two: 60, 53 ms)
+        const int wave2 = (n + (job == JOB_SAMPLE ? slots : 0)) / (2 * slots);
+        const int fill = few ? 1 : std::min(n / slots, 2 * cf::kFoldThreads / std::max(P.Lmax, 1));
         P.group = eng->group > 0 ? std::min(cf::kMaxGroup, eng->group)
-                                 : uniform ? wave_group : std::min(group_for_length(Lmed), wave2);
+                                 : uniform ? wave_group : std::min(group_for_length(Lmed), std::max({1, wave2, fill}));
     }
     for (int k = 0; k < n; ++k) {
         const int b = order[k];
@@ -603,16 +620,7 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         }
         P.warp = false;   // not even one CTA of warp slots fits: per-sequence kernels, sliced
     }
-    // The latency kernels: a sequence on a cluster or, one after another on an SM, on CTAs of their own.  They win until
-    // the grouped kernels' CTAs fill the device (GB300, ms, latency / grouped, MEA and 1 sample: 200 nt n = 304 19 / 24
-    // and 10 / 13, 456 29 / 26 and 15 / 13; 100 nt n = 456 8.8 / 9.3 and 5.9 / 5.4; 320 nt n = 304 46 / 53, 456 70 / 59;
-    // 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA).  Not on a shared device: a
-    // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
-    int sms = 0;
-    CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
-    const int cut = uniform ? (P.Lmax <= 128 ? 3 : 2) : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
-    P.lat = P.cluster || (batched && !eng->shared && P.group == 1 && n <= cut * sms &&
-                          (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE));
+    P.lat = P.cluster || (few && P.group == 1);
     P.slice_begin.clear();
     P.slice_words.clear();
     int64_t cur = 0;

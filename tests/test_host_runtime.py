@@ -147,3 +147,20 @@ for graph in (False, True):
     plan.run(4096, 0, 8192, 6.0, stream)
     assert fake.fake_streams_of(-3) > 1
 """)
+
+
+def test_groups_of_short_mixed_batches(run):
+    """Short sequences of mixed lengths fold several a CTA as soon as every CTA has a group (152 SMs here), long ones
+    only where two waves of CTAs remain; no batch takes the warp-per-sequence kernel on its own."""
+    run("""
+def plan(n, lo, hi, job=CF_JOB_MEA):
+    p = Plan(eng, job, Batch(seqs(*rng.integers(lo, hi + 1, n), lo, hi)).offsets)
+    return p.schedule, p.group
+eng.set_budget(1 << 30)
+assert plan(2046, 15, 25) == ("group", 3)        # 608 CTAs
+assert plan(10000, 20, 40) == ("group", 8)
+assert plan(3000, 100, 256) == ("group", 2)
+assert plan(2046, 40, 400) == ("group", 1)
+assert plan(700, 15, 25) == ("group", 1)         # the latency kernels
+assert plan(2046, 60, 70) == ("group", 4)        # lengths alike: one wave
+""")
