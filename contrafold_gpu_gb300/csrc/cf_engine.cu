@@ -467,8 +467,9 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
     // 304 19 / 24 and 10 / 13, 456 29 / 26 and 15 / 13; 100 nt n = 456 8.8 / 9.3 and 5.9 / 5.4; 320 nt n = 304 46 / 53, 456
     // 70 / 59; 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA).  Not on a shared device: a
     // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
-    int sms = 0;
+    int sms = 0, smem_optin = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
+    CF_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, eng->device));
     const int cut = uniform ? (P.Lmax <= 128 ? 3 : 2) : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
     const bool few = batched && !eng->shared && n <= cut * sms &&
                      (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE);
@@ -629,7 +630,6 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         const int64_t w = arena_words(job, P.descs[k].L, P.grad_ckpt);
         return P.lat ? cf::pad32(w) + cf::lat_term_words(P.descs[k].L) : w;
     };
-    if (job == JOB_MFE) P.group = 1;   // cf_viterbi.cu: a sequence a CTA, or a cluster
     // CTAs a sequence.  Two of a cluster's fit an SM; a cluster of two is only worth its barriers where it spreads over
     // two SMs.  (GB300, MEA, ms with 1 / 2 / 4 / 8: 1 x 60 nt 1.4 / 1.6 / 1.5 / 1.5, 1 x 400 nt 35 / 28 / 22 / 20, 48 x
     // 40-400 nt 33 / 27 / 22 / 20, 70 x 200 nt 9.3 / 9.3 / 8.8 / 15, 140 x 200 nt 9.8 / 11 / 17 / 31.)
@@ -638,10 +638,19 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
         if (!P.cluster && P.Lmax > 128)
             P.ctas = n * 8 <= 2 * sms ? 8 : n * 4 <= 2 * sms ? 4 : 1;
     }
+    if (job == JOB_MFE) {
+        // Viterbi folds a sequence a CTA (or a cluster); very short ones, whose diagonals hold fewer items than the CTA has
+        // warps, together, in whole waves (ms with 1, 2, 4, 8: 30,000 x 15-25 nt 11.1, 10.1, 9.3, 9.2; 3,000 x 20-40 nt
+        // 1.68, 1.59, 1.45, 1.92; 3,000 x 60 nt 4.4, 4.5, 4.5, 4.8; 3,000 x 100 nt 11.7, 12.2, 13.0, 13.7)
+        const int slots = cf::kFoldMinBlocks * sms, most = std::max(1, std::min(cf::kVitGroup, 176 / std::max(P.Lmax, 1)));
+        const int waves = (n + most * slots - 1) / (most * slots);
+        const int asked = eng->group > 0 ? eng->group : row_group;
+        P.group = P.ctas > 1 || !batched ? 1 : asked > 0 ? std::min(cf::kVitGroup, asked)
+                : 2 * n <= 3 * slots ? 1 : (n + waves * slots - 1) / (waves * slots);
+        while (P.group > 1 && cf::fold_smem_bytes(P.Lmax, P.group, true) + cf::kVitStaticSmem > (size_t)smem_optin) --P.group;
+    }
     if (P.lat) {   // no room for the longest sequence's terms or codes: the grouped kernels need less
-        int dev_max = 0;
-        CF_CUDA(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, eng->device));
-        bool fits = cf::fold_smem_bytes(P.Lmax, 1, false) + cf::kLatStaticSmem <= (size_t)dev_max;
+        bool fits = cf::fold_smem_bytes(P.Lmax, 1, false) + cf::kLatStaticSmem <= (size_t)smem_optin;
         for (int k = 0; k < n && fits; ++k) fits = words(k) <= budget_words;
         if (!fits) P.lat = P.cluster = false;
     }
@@ -706,7 +715,7 @@ std::vector<const void*> slice_kernels(Job job, const Plan& P) {
     };
     switch (job) {
         case JOB_LOGZ64: add({cf::k_inside64}); break;
-        case JOB_MFE: add({P.ctas > 1 ? cf::k_viterbi_cluster64 : cf::k_viterbi64}); break;
+        case JOB_MFE: add({P.ctas > 1 ? cf::k_viterbi_cluster64 : P.group > 1 ? cf::k_viterbi_group64 : cf::k_viterbi64}); break;
         case JOB_BPP:
         case JOB_MEA:
             if (P.plain) ks = {(const void*)cf::k_plain_inside32, (const void*)cf::k_plain_outside32,
@@ -1094,7 +1103,7 @@ int run_device(cf_engine* eng, Job job, const Plan& P, Exec& X, const uint8_t* d
             }
             case JOB_MFE:
                 if (P.ctas > 1) CF_PHASE(0, CF_CUDA(launch_lat(cf::k_viterbi_cluster64)));
-                else CF_PHASE(0, (cf::k_viterbi64<<<grid, blk, smem, st>>>(A)));
+                else CF_PHASE(0, ((P.group > 1 ? cf::k_viterbi_group64 : cf::k_viterbi64)<<<grid, blk, smem, st>>>(A)));
                 break;
             case JOB_SAMPLE: {
                 if (P.lat) CF_PHASE(0, CF_CUDA(launch_lat(lk.inside_acc)));

@@ -62,8 +62,12 @@ LatKernels lat_kernels(bool cluster);   // kLatThreads threads; kFoldThreads in 
 int64_t lat_term_words(int L);
 constexpr int kLatStaticSmem = 18 * 1024;   // at most, beside the grouped kernels' dynamic shared memory
 __global__ void k_inside64(FoldArgs A);
-__global__ void k_viterbi64(FoldArgs A);           // one sequence a CTA ...
-__global__ void k_viterbi_cluster64(FoldArgs A);   // ... or a cluster (cf_viterbi.cu)
+// Viterbi (cf_viterbi.cu): one sequence a CTA, up to kVitGroup, or one a cluster
+__global__ void k_viterbi64(FoldArgs A);
+__global__ void k_viterbi_group64(FoldArgs A);
+__global__ void k_viterbi_cluster64(FoldArgs A);
+constexpr int kVitGroup = 8;
+constexpr int kVitStaticSmem = 32 * 1024;   // at most, beside fold_smem_bytes
 // log-domain logZ of the sequences listed in fails (cf_linear.h), A.group at most on a CTA (cf_fold.cu)
 __global__ void k_inside_redo32(FoldArgs A, const int* fails, bool mixed);
 __global__ void k_inside_redo64(FoldArgs A, const int* fails, bool mixed);

@@ -250,110 +250,209 @@ __device__ void viterbi_traceback(const SmemTabs<double>* tb, const SeqV& Q, con
     if (full && lane == 0) atomicExch(status, CF_EDEVICE);
 }
 
+// A sequence's tables; parts ([kVitParts][L + 4]) lie in the traceback stack's
+// place, wmax ([i]) in the step buffers, both keys.
+struct VitSeq {
+    SeqV Q;
+    InView<double> V;
+    int* stack;
+    long long *parts, *wmax;
+};
+__device__ __forceinline__ VitSeq vit_seq(SmemFold<double>* sm, const FoldArgs& A, int g) {
+    VitSeq X;
+    X.Q = seq_v(sm, g);
+    X.V = in_view<double>(A, sm->ws[g], X.Q.L);
+    X.stack = reinterpret_cast<int*>(A.ws + sm->ws[g] + arena64(X.Q.L).stack);
+    X.parts = reinterpret_cast<long long*>(X.stack);
+    X.wmax = reinterpret_cast<long long*>(X.V.FB);
+    return X;
+}
+__device__ __forceinline__ int vit_pairs(const VitSeq& X, int d) {   // pairable cells of diagonal d
+    return d <= X.Q.L - 2 ? X.V.PLs.poff[d + 1] - X.V.PLs.poff[d] : 0;
+}
+__device__ __forceinline__ int vit_splits(int L, int d) {            // items of its splits
+    return d >= 2 ? kVitParts * ((max(0, L - 1 - d) + 31) >> 5) : 0;
+}
+
+// F5[d]: FC of spans up to d - 2
+__device__ __forceinline__ void vit_exterior(const SmemTabs<double>* tb, const VitSeq& X, int d, int lane) {
+    const ParamView<double> P{tb->blob};
+    const SeqV& Q = X.Q;
+    const InTabs<double>& T = X.V.T;
+    if (d < 1) return;
+    long long best = key(CF_NEG64);
+    for (int k = lane; k < d; k += 32) {
+        if (!Q.pairable(k + 1, d)) continue;
+        const double fcin = T.FC[T.at(k + 1, d - 1)], f5k = T.F5[k];
+        if (!(fcin > CF_HALF64) || !(f5k > CF_HALF64)) continue;
+        const double jA = junctionA_rev<Max64>(P, Q.L, Q, k, d);
+        best = max(best, key(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[d])), jA)));
+    }
+    best = max(warp_max(best), key(__dadd_rn(T.F5[d - 1], P.eu())));
+    if (lane == 0) T.F5[d] = unkey(best);
+}
+
+// Item u of the splits of diagonal d: a part of 32 inner cells'.
+__device__ __forceinline__ void vit_split(const VitSeq& X, int d, int u, int lane) {
+    const InTabs<double>& T = X.V.T;
+    const int L = X.Q.L, m = T.m, part = u % kVitParts, i = 1 + (u / kVitParts) * 32 + lane;
+    if (i > max(0, L - 1 - d)) return;
+    constexpr int N = kVitParts, H = N * (N - 1) / 2;
+    int s = 1 + part;
+    int o1 = tri_off(s, m) + i, o2 = tri_off(d - s, m) + i + s;
+    int d1 = N * m - N * s - H, d2 = N * (d - s) - N * m - N * N + H + N;   // see cf_linear.cu, dot_tri
+    long long best = key(CF_NEG64);
+#pragma unroll 4
+    for (; s < d; s += N) {
+        best = max(best, key(__dadd_rn(T.FM1[o1], T.FM[o2])));
+        o1 += d1;
+        d1 -= N * N;
+        o2 += d2;
+        d2 -= N * N;
+    }
+    X.parts[part * (L + 4) + i] = best;
+}
+
+// Joins the items of cell (i, i + d).
+__device__ __forceinline__ void vit_join(const SmemTabs<double>* tb, const VitSeq& X, int d, int i) {
+    const ParamView<double> P{tb->blob};
+    const SeqV& Q = X.Q;
+    const InTabs<double>& T = X.V.T;
+    const double NEG = CF_NEG64, HALF = CF_HALF64;
+    const int L = Q.L, ps = L + 4, j = i + d, at = tri_off(d, T.m) + i;
+    double fc = NEG, fm1 = NEG, fm = NEG;
+    if (i > 0 && j < L) {
+        long long k2 = key(NEG);
+        if (d >= 2) {
+#pragma unroll
+            for (int p = 0; p < kVitParts; ++p) k2 = max(k2, X.parts[p * ps + i]);
+        }
+        const double fm2 = unkey(k2);
+        if (Q.pairable(i, j + 1)) {
+            const double jB = tb->jB(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j]);
+            fc = unkey(max(key(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP))), X.wmax[i]));
+            if (fm2 > HALF)
+                fc = fmax(fc, __dadd_rn(__dadd_rn(__dadd_rn(fm2, junctionA<Max64>(P, L, Q, i, j)), P.mp()), P.mb()));
+        }
+        if (d >= 2) {
+            const double fin = T.FC[T.at(i + 1, j - 1)], ext = T.FM1[T.at(i + 1, j)], prev = T.FM[T.at(i, j - 1)];
+            if (Q.pairable(i + 1, j) && fin > HALF)
+                fm1 = __dadd_rn(__dadd_rn(__dadd_rn(fin, junctionA_rev<Max64>(P, L, Q, i, j)), P.mp()),
+                                P.bp(Q.s[i + 1], Q.s[j]));
+            if (ext > HALF) fm1 = fmax(fm1, __dadd_rn(ext, P.mu()));
+            if (fm2 > HALF) fm = fm2;
+            if (prev > HALF) fm = fmax(fm, __dadd_rn(prev, P.mu()));
+            if (fm1 > HALF) fm = fmax(fm, fm1);
+        }
+    }
+    T.FC[at] = fc;
+    T.FM1[at] = fm1;
+    T.FM[at] = fm;
+}
+
+// What a fold begins with: no pairs yet, the pair list, F5[0].
+template <class Team>
+__device__ __forceinline__ void vit_begin(SmemFold<double>* sm, const FoldArgs& A, const Team& tm, const VitSeq& X, int g) {
+    if (tm.rank() == 0) build_plist(X.Q, X.V.PLs);
+    if (tm.rank() == 0 && threadIdx.x == 0) X.V.T.F5[0] = 0.0;
+    for (int t = tm.tid(); t < X.Q.L; t += tm.nthreads()) A.structs[sm->soff[g] + t] = '.';
+}
+
+struct VitShared {
+    uint16_t lists[kVitWarps][kWindowMax];
+    LoopScores ls;
+};
+
 template <class Team>
 __device__ __forceinline__ void viterbi_fold(const FoldArgs& A, const Team& tm, int gi) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* sm = reinterpret_cast<SmemFold<double>*>(smem_raw);
-    __shared__ uint16_t lists[kVitWarps][kWindowMax];
-    __shared__ LoopScores ls;
-    uint16_t* list = lists[threadIdx.x >> 5];
+    __shared__ VitShared sh;
+    uint16_t* list = sh.lists[threadIdx.x >> 5];
     setup_group(sm, A, A.blob64, gi);
-    load_loop_scores(&ls, &sm->tabs);
-    const SeqV Q = seq_v(sm, 0);
-    const InView<double> V = in_view<double>(A, sm->ws[0], Q.L);
-    const InTabs<double>& T = V.T;
-    const ParamView<double> P{sm->tabs.blob};
-    const int L = Q.L, m = T.m;
-    const double NEG = CF_NEG64, HALF = CF_HALF64;
-    int* stack = reinterpret_cast<int*>(A.ws + sm->ws[0] + arena64(L).stack);
-    long long* parts = reinterpret_cast<long long*>(stack);   // [kVitParts][L + 4], keys
-    long long* wmax = reinterpret_cast<long long*>(V.FB);     // [i], keys
-    const int ps = L + 4;
-    if (tm.rank() == 0) build_plist(Q, V.PLs);
+    load_loop_scores(&sh.ls, &sm->tabs);
+    const VitSeq X = vit_seq(sm, A, 0);
+    const int L = X.Q.L;
     if (threadIdx.x == 0) sm->step_ctr[0] = sm->step_ctr[1] = 0;
-    if (tm.rank() == 0 && threadIdx.x == 0) T.F5[0] = 0.0;
-    for (int t = tm.tid(); t < L; t += tm.nthreads()) A.structs[sm->soff[0] + t] = '.';
+    vit_begin(sm, A, tm, X, 0);
     tm.sync();
     for (int d = 0; d <= L; ++d) {
-        const int nE = d <= L - 2 ? V.PLs.poff[d + 1] - V.PLs.poff[d] : 0, oE = nE ? V.PLs.poff[d] : 0;
-        const int c = max(0, L - 1 - d);   // inner cells i = 1 .. c
-        const int nS = d >= 2 ? kVitParts * ((c + 31) >> 5) : 0;
-        run_items(sm, tm, d, 1 + nE + nS, [&](int q, int lane) {
-            if (q == 0) {   // F5[d]: FC of spans up to d - 2
-                if (d < 1) return;
-                long long best = key(NEG);
-                for (int k = lane; k < d; k += 32) {
-                    if (!Q.pairable(k + 1, d)) continue;
-                    const double fcin = T.FC[T.at(k + 1, d - 1)], f5k = T.F5[k];
-                    if (!(fcin > HALF) || !(f5k > HALF)) continue;
-                    const double jA = junctionA_rev<Max64>(P, L, Q, k, d);
-                    best = max(best, key(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(f5k, fcin), P.ep()), P.bp(Q.s[k + 1], Q.s[d])), jA)));
-                }
-                best = max(warp_max(best), key(__dadd_rn(T.F5[d - 1], P.eu())));
-                if (lane == 0) T.F5[d] = unkey(best);
+        const int nE = vit_pairs(X, d), oE = nE ? X.V.PLs.poff[d] : 0;
+        run_items(sm, tm, d, 1 + nE + vit_splits(L, d), [&](int q, int lane) {
+            if (q == 0) {
+                vit_exterior(&sm->tabs, X, d, lane);
             } else if (q <= nE) {
-                const int i = V.PLs.pl[oE + q - 1];
-                const long long w = window_max(&sm->tabs, &ls, Q, T, i, i + d, list, lane);
-                if (lane == 0) wmax[i] = w;
+                const int i = X.V.PLs.pl[oE + q - 1];
+                const long long w = window_max(&sm->tabs, &sh.ls, X.Q, X.V.T, i, i + d, list, lane);
+                if (lane == 0) X.wmax[i] = w;
             } else {
-                const int u = q - 1 - nE, part = u % kVitParts, i = 1 + (u / kVitParts) * 32 + lane;
-                if (i > c) return;
-                constexpr int N = kVitParts, H = N * (N - 1) / 2;
-                int s = 1 + part;
-                int o1 = tri_off(s, m) + i, o2 = tri_off(d - s, m) + i + s;
-                int d1 = N * m - N * s - H, d2 = N * (d - s) - N * m - N * N + H + N;   // see cf_linear.cu, dot_tri
-                long long best = key(NEG);
-#pragma unroll 4
-                for (; s < d; s += N) {
-                    best = max(best, key(__dadd_rn(T.FM1[o1], T.FM[o2])));
-                    o1 += d1;
-                    d1 -= N * N;
-                    o2 += d2;
-                    d2 -= N * N;
-                }
-                parts[part * ps + i] = best;
+                vit_split(X, d, q - 1 - nE, lane);
             }
         });
-        for (int i = tm.tid(); i + d <= L; i += tm.nthreads()) {
-            const int j = i + d, at = tri_off(d, m) + i;
-            double fc = NEG, fm1 = NEG, fm = NEG;
-            if (i > 0 && j < L) {
-                long long k2 = key(NEG);
-                if (d >= 2) {
-#pragma unroll
-                    for (int p = 0; p < kVitParts; ++p) k2 = max(k2, parts[p * ps + i]);
-                }
-                const double fm2 = unkey(k2);
-                if (Q.pairable(i, j + 1)) {
-                    const double jB = sm->tabs.jB(Q.s[i], Q.s[j + 1], Q.s[i + 1], Q.s[j]);
-                    fc = unkey(max(key(__dadd_rn(jB, P.hp(d <= DHP ? d : DHP))), wmax[i]));
-                    if (fm2 > HALF)
-                        fc = fmax(fc, __dadd_rn(__dadd_rn(__dadd_rn(fm2, junctionA<Max64>(P, L, Q, i, j)), P.mp()), P.mb()));
-                }
-                if (d >= 2) {
-                    const double fin = T.FC[T.at(i + 1, j - 1)], ext = T.FM1[T.at(i + 1, j)], prev = T.FM[T.at(i, j - 1)];
-                    if (Q.pairable(i + 1, j) && fin > HALF)
-                        fm1 = __dadd_rn(__dadd_rn(__dadd_rn(fin, junctionA_rev<Max64>(P, L, Q, i, j)), P.mp()),
-                                        P.bp(Q.s[i + 1], Q.s[j]));
-                    if (ext > HALF) fm1 = fmax(fm1, __dadd_rn(ext, P.mu()));
-                    if (fm2 > HALF) fm = fm2;
-                    if (prev > HALF) fm = fmax(fm, __dadd_rn(prev, P.mu()));
-                    if (fm1 > HALF) fm = fmax(fm, fm1);
-                }
-            }
-            T.FC[at] = fc;
-            T.FM1[at] = fm1;
-            T.FM[at] = fm;
-        }
+        for (int i = tm.tid(); i + d <= L; i += tm.nthreads()) vit_join(&sm->tabs, X, d, i);
         tm.sync();
     }
     if (tm.rank() == 0 && threadIdx.x < 32)
-        viterbi_traceback(&sm->tabs, Q, T, stack, A.structs + sm->soff[0], A.status, threadIdx.x);
+        viterbi_traceback(&sm->tabs, X.Q, X.V.T, X.stack, A.structs + sm->soff[0], A.status, threadIdx.x);
+}
+
+// The same for a group of very short sequences on a CTA (rule: cf_engine.cu):
+// alone, each has fewer items a diagonal than the CTA has warps.
+__device__ __forceinline__ void viterbi_group(const FoldArgs& A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto* sm = reinterpret_cast<SmemFold<double>*>(smem_raw);
+    __shared__ VitShared sh;
+    __shared__ int npair[2][kVitGroup];   // pairable cells of a diagonal, by its parity
+    uint16_t* list = sh.lists[threadIdx.x >> 5];
+    const CtaTeam tm;
+    setup_group(sm, A, A.blob64);
+    load_loop_scores(&sh.ls, &sm->tabs);
+    const int ng = sm->n, tid = threadIdx.x;
+    if (tid == 0) sm->step_ctr[0] = sm->step_ctr[1] = 0;
+    for (int g = 0; g < ng; ++g) vit_begin(sm, A, tm, vit_seq(sm, A, g), g);
+    __syncthreads();
+    if (tid < ng) npair[0][tid] = vit_pairs(vit_seq(sm, A, tid), 0);
+    __syncthreads();
+    for (int d = 0; d <= sm->Lmax; ++d) {
+        auto items = [&](int g) { return d > sm->L[g] ? 0 : 1 + npair[d & 1][g] + vit_splits(sm->L[g], d); };
+        int total = 0, cells = 0;
+        for (int g = 0; g < ng; ++g) {
+            total += items(g);
+            cells += max(0, sm->L[g] + 1 - d);
+        }
+        run_items(sm, tm, d, total, [&](int q, int lane) {
+            int g = 0;
+            for (int n; q >= (n = items(g)); ++g) q -= n;
+            const VitSeq X = vit_seq(sm, A, g);
+            const int nE = npair[d & 1][g];
+            if (q == 0) {
+                vit_exterior(&sm->tabs, X, d, lane);
+            } else if (q <= nE) {
+                const int i = X.V.PLs.pl[X.V.PLs.poff[d] + q - 1];
+                const long long w = window_max(&sm->tabs, &sh.ls, X.Q, X.V.T, i, i + d, list, lane);
+                if (lane == 0) X.wmax[i] = w;
+            } else {
+                vit_split(X, d, q - 1 - nE, lane);
+            }
+        });
+        if (tid < ng) npair[(d + 1) & 1][tid] = vit_pairs(vit_seq(sm, A, tid), d + 1);
+        for (int c = tid; c < cells; c += kFoldThreads) {
+            int g = 0, i = c;
+            for (int n; i >= (n = max(0, sm->L[g] + 1 - d)); ++g) i -= n;
+            vit_join(&sm->tabs, vit_seq(sm, A, g), d, i);
+        }
+        __syncthreads();
+    }
+    for (int g = tid >> 5; g < ng; g += kVitWarps) {
+        const VitSeq X = vit_seq(sm, A, g);
+        viterbi_traceback(&sm->tabs, X.Q, X.V.T, X.stack, A.structs + sm->soff[g], A.status, tid & 31);
+    }
 }
 
 }  // namespace
 
 __global__ void __launch_bounds__(kFoldThreads, 3) k_viterbi64(FoldArgs A) { viterbi_fold(A, CtaTeam{}, blockIdx.x); }
+__global__ void __launch_bounds__(kFoldThreads, 3) k_viterbi_group64(FoldArgs A) { viterbi_group(A); }
 __global__ void __launch_bounds__(kFoldThreads, 2) k_viterbi_cluster64(FoldArgs A) {
     const int c = cluster_nctas();
     viterbi_fold(A, ClusterTeam{cluster_ctarank(), c}, (int)blockIdx.x / c);

@@ -27,3 +27,26 @@ def test_viterbi_ties(engine, oracle, P):
     from contrafold_gpu_gb300.engine import Batch
     seqs = ["GU" * 60, "GC" * 50, "GGGAAACCC" * 14, "A" * 40 + "U" * 40, "G" * 70 + "C" * 70]
     assert engine.mfe(Batch(seqs, None)) == oracle.batch(oracle.JOB_MFE, seqs, P, None)
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 8), (22, 22), (15, 40), (55, 60)])
+def test_viterbi_groups_equal_oracle(engine, oracle, P, lo, hi):
+    """Thousands of very short sequences fold several a CTA: whole groups, a last one that is not full, lengths alike and
+    mixed, with empty sequences."""
+    from contrafold_gpu_gb300.engine import Batch, Engine
+    rng = np.random.default_rng(40 + hi)
+    lens = rng.integers(lo, hi + 1, 3421)
+    seqs = ["".join(rng.choice(list("ACGUN"), p=[.24, .24, .24, .24, .04], size=L)) for L in lens]
+    masks = [(rng.random(L) < 0.1).astype(np.uint8) for L in lens]
+    want = oracle.batch(oracle.JOB_MFE, seqs, P, masks)
+    engine.set_mode("batched")
+    engine.set_schedule("auto")
+    B = Batch(seqs, masks)
+    assert engine.mfe(B) == want
+    eng = Engine(P)
+    try:
+        for group in (1, 3, 8):
+            eng.set_group(group)
+            assert eng.mfe(B) == want
+    finally:
+        eng.close()
