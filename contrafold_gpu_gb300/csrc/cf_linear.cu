@@ -990,7 +990,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lin_inside32(LinArgs A) { lin
 __global__ void __launch_bounds__(256, 2) k_lin_inside64(LinArgs A) { lin_inside<double, false, 256>(A); }
 
 // Threads by length: as many as keep an SM at about 1,024 threads with the
-// CTAs its shared memory holds (49 KB at 128 nt, 74 KB at 235, 113 KB at 395).
+// CTAs its shared memory holds (four of 256 up to 160 nt, three up to 235, two of
+// 512 up to 395; a few nt more would fit, but leave the splits no L1: 1,000 x 240
+// nt with three, two CTAs 4.7, 4.6 ms, 1,000 x 405 nt with two, one 18.1, 16.0).
 // On a shared device no more than other kernels' CTAs have (narrow).
 LinKernel lin_inside_kernel(int L, bool fp64, bool train, bool narrow) {
     if (fp64) return {k_lin_inside64, 256};
@@ -999,11 +1001,15 @@ LinKernel lin_inside_kernel(int L, bool fp64, bool train, bool narrow) {
     return {train ? k_lin_inside32<true, 1024> : k_lin_inside32<false, 1024>, 1024};
 }
 // Last length of the launch class of L: sequences of a class share a launch,
-// whose shared memory is its longest sequence's.
+// whose shared memory is its longest sequence's.  In float the classes end where
+// an SM holds a CTA less (see above; 2,000 x 130-180 nt in one class of 235, two:
+// 3.6, 3.4 ms).  In double the FP64 pipe, not the CTAs an SM holds, bounds all
+// but the short ones, and a class more is a last wave more (300 x 150-180 nt with
+// a class up to 160, up to 235: 5.2, 4.0 ms; 500 x 20-400 nt with these classes
+// and with float's: 13.6, 13.9).
 int lin_class_end(int L, bool fp64) {
-    for (int e : {60, 128, 235, 395})
-        if (L <= e) return e;
-    return fp64 ? kLinMaxLen64 : kLinMaxLen;
+    if (fp64) return L <= 96 ? 96 : L <= 235 ? 235 : kLinMaxLen64;
+    return L <= 160 ? 160 : L <= 235 ? 235 : L <= 395 ? 395 : kLinMaxLen;
 }
 
 size_t lin_inside_smem_bytes(int Lmax, bool fp64) {

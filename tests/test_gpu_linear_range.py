@@ -72,3 +72,28 @@ def test_slices_of_a_small_arena(P, oracle, engine):
         assert all(np.array_equal(a, b) for a, b in zip(got.d_bonus, counts.d_bonus))
     finally:
         eng.close()
+
+
+def test_length_classes(engine, oracle, P):
+    """Lengths on either side of the launch classes' ends: the result each has alone, in a launch of its own, on a shared
+    device, in float and in double (tolerance of test_gpu_linear.py)."""
+    from contrafold_gpu_gb300.engine import Batch, Engine
+    engine.set_mode("batched")
+    engine.set_schedule("auto")
+    rng = np.random.default_rng(4)
+    seqs = [_random(rng, L) for L in (1, 95, 96, 97, 159, 160, 161, 235, 236, 300, 395, 396, 415, 512)]
+    z, z64 = engine.logz(Batch(seqs)), engine.logz64(Batch(seqs[:-1]))
+    want = np.array(oracle.batch(oracle.JOB_LOGZ64, seqs, P, None))
+    L = np.array([len(s) for s in seqs])
+    assert np.all(np.abs(z - want) <= 16 * L * 2.0 ** -24 + 2.0 ** -23 * np.abs(want))
+    for k, s in enumerate(seqs):
+        assert engine.logz(Batch([s]))[0] == z[k]
+        if k < len(z64):
+            assert engine.logz64(Batch([s]))[0] == z64[k]
+    eng = Engine(P)
+    try:
+        eng.set_shared(True)
+        assert np.array_equal(eng.logz(Batch(seqs)), z)
+        assert np.array_equal(eng.logz64(Batch(seqs[:-1])), z64)
+    finally:
+        eng.close()
