@@ -5,7 +5,7 @@ then linked into one shared library that exports the C-ABI of
 include/contrafold_gb300.h.  `-fmad=false` keeps every float add and multiply
 separately rounded (the FP32 paths are bitwise parity targets).
 
-Extra nvcc flags (for example -DCF_FLAT_WALK=0 to compare a kernel variant)
+Extra nvcc flags (for example -DCF_CHAIN_PF=6 to compare a kernel variant)
 come from the environment variable CONTRAFOLD_GB300_NVCC_FLAGS; the flags of
 the last build are recorded next to the library, and a change rebuilds it.
 

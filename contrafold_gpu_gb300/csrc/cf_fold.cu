@@ -117,7 +117,7 @@ __device__ __forceinline__ void inside_group(SmemFold<typename S::Real>* sm, con
             [&](int g, int i) {   // phase A(t): FM2, FM1, FM
                 const SeqV Q = seq_v(sm, g);
                 const InView<R> V = in_view<R>(A, sm->ws[g], Q.L);
-                V.FB[(t & 1) * V.fbs + i] = inside_A<S, Team::kChainPF>(sr, &sm->tabs, Q, V.T, i, i + t);
+                V.FB[(t & 1) * V.fbs + i] = inside_A<S>(sr, &sm->tabs, Q, V.T, i, i + t);
             });
     }
     // exterior recurrence: one warp per sequence
@@ -228,7 +228,7 @@ __device__ __forceinline__ void outside_group(SmemFold<float>* sm, const FoldArg
             },
             [&](int g, int a) {   // phase A(t): FMo, FM1o, FM2o
                 const SeqV Q = seq_v(sm, g);
-                outside_A<Team::kChainPF>(sr, &sm->tabs, Q, out_tabs(A, sm->ws[g], Q.L), a, a + t);
+                outside_A(sr, &sm->tabs, Q, out_tabs(A, sm->ws[g], Q.L), a, a + t);
             });
     }
 }

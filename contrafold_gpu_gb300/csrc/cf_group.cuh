@@ -68,8 +68,8 @@ __device__ __forceinline__ void build_group_seqs(SmemFold<R>* sm, const FoldArgs
 
 // ---------------------------------------------------------------------------
 // Teams: the threads that fold one group together.  CtaTeam is one CTA (the
-// batched kernels); ClusterTeam is the C CTAs of a thread-block cluster, on C
-// SMs, folding the same group (the latency kernels).  Work of a diagonal step
+// batched kernels, which take no other); ClusterTeam is the C CTAs of a
+// thread-block cluster, on C SMs (the latency and the Viterbi kernels).  Work of a diagonal step
 // is split over tid() / nthreads(); sync() separates steps (a cluster barrier
 // with release / acquire semantics for ClusterTeam, so table cells written in
 // global memory by one CTA are read by the others after it).  Every sync() is
@@ -78,7 +78,6 @@ __device__ __forceinline__ void build_group_seqs(SmemFold<R>* sm, const FoldArgs
 // rank-0-only work sits between two syncs, not around one.
 // ---------------------------------------------------------------------------
 struct CtaTeam {
-    static constexpr int kChainPF = cf::kChainPF;   // bifurcation-chain register pipeline depth
     __device__ __forceinline__ int rank() const { return 0; }
     __device__ __forceinline__ int size() const { return 1; }
     __device__ __forceinline__ int tid() const { return threadIdx.x; }
@@ -87,7 +86,6 @@ struct CtaTeam {
 };
 
 struct ClusterTeam {
-    static constexpr int kChainPF = CF_CLUSTER_CHAIN_PF;
     int r, c;   // rank of this CTA in the cluster, cluster size
     __device__ __forceinline__ int rank() const { return r; }
     __device__ __forceinline__ int size() const { return c; }
@@ -277,7 +275,7 @@ __device__ __forceinline__ void mea_group(SmemFold<float>* sm, const FoldArgs& A
         const SeqV Q = seq_v(sm, g);
         const Arena32 ar = arena32(Q.L);
         float* base = A.ws + sm->ws[g];
-        mea_cell<Team::kChainPF>(Q, base + ar.FMo, base + ar.up, base + ar.FM2o, reinterpret_cast<int*>(base + ar.FM), Q.L, i, j);
+        mea_cell(Q, base + ar.FMo, base + ar.up, base + ar.FM2o, reinterpret_cast<int*>(base + ar.FM), Q.L, i, j);
     });
     for (int g = 0; g < sm->n; ++g) {
         const int L = sm->L[g];

@@ -151,7 +151,7 @@ __device__ __forceinline__ typename S::Real junctionA_rev(const ParamView<typena
 //     has already consumed.  The module defines CF_CHAIN_THREADS (its block
 //     size); float chains only.
 //   CF_CHAIN_PF = PF > 0: a rolling register pipeline of 2*PF terms (fused MEA
-//     of 10,000 x 200 nt with PF 3, 4, 6: 241, 236, 240 ms; PF is the default of the PFD template parameter; latency kernels pass a deeper one).
+//     of 10,000 x 200 nt with PF 3, 4, 6: 241, 236, 240 ms).
 //   both 0: load, then fold.
 // ---------------------------------------------------------------------------
 #ifndef CF_CHAIN_PF
@@ -363,7 +363,7 @@ __device__ __forceinline__ void queue_rows(unsigned lanes, int rows, Row row, Ld
 // Phase A of inside cell (i, j), 0 <= i <= j <= L.  Returns FM2[i][j] (the
 // semiring zero where the cell needs none).  Writes FM1, FM, and FC = zero
 // for cells that cannot close a pair (pairable cells get FC in phase B).
-template <class S, int CPF = kChainPF, class QV>
+template <class S, class QV>
 __device__ __forceinline__ typename S::Real inside_A(const S& sr, const SmemTabs<typename S::Real>* __restrict__ tb,
                                                      const QV& Q, const InTabs<typename S::Real>& T, int i, int j) {
     using R = typename S::Real;
@@ -386,7 +386,7 @@ __device__ __forceinline__ typename S::Real inside_A(const S& sr, const SmemTabs
         // term k = i+1 .. j-1: FM1[i][k] (span s1 = k-i), FM[k][j] (span s2 = j-k)
         DiagPtr<R> x1(T.FM1, tri_off(1, m) + i, m - 1);              // FM1[i][i+1]; span s to s+1: m - s cells on
         DiagPtr<R> x2(T.FM, tri_off(d - 1, m) + i + 1, d - 1 - m);   // FM[i+1][j]; span s to s-1, one position right
-        prefetched_chain<R, CPF>(
+        prefetched_chain<R>(
             d - 1,
             [&](const R*& x, const R*& y) {
                 x = x1.next();

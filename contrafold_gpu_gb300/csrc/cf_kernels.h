@@ -49,12 +49,9 @@ struct FoldKernels {
 };
 FoldKernels fold_kernels();
 // Latency kernels (cf_latency.cu): one sequence on one CTA of kLatThreads, or
-// on the 2 to kClusterCtas CTAs of a cluster.  They need
+// on the 4 or kClusterCtas CTAs of a cluster, of kFoldThreads each.  They need
 // lat_term_words(L) words behind the sequence's arena.
 constexpr int kClusterCtas = 8;   // the largest portable cluster
-#ifndef CF_CLUSTER_CHAIN_PF
-#define CF_CLUSTER_CHAIN_PF 8   // MEA decode's chain pipeline depth in the latency kernels
-#endif
 struct LatKernels {
     FoldKernel mea, bpp, inside_acc;
 };

@@ -1,5 +1,6 @@
 // cf_latency.cu -- fold kernels for batches that do not fill the device: one
-// sequence on one 512-thread CTA, or on the 8 CTAs of a thread-block cluster.
+// sequence on one 512-thread CTA, or on the 4 or 8 256-thread CTAs of a
+// thread-block cluster.
 //
 // Such a fold is bound by its longest serial chain, not by throughput: on each
 // diagonal the step's barrier waits for the cell that folds the most terms one
@@ -565,10 +566,6 @@ __device__ __forceinline__ void mea_lat(SmemFold<float>* sm, const FoldArgs& A, 
     }
 }
 
-struct LatTeam : CtaTeam {
-    static constexpr int kChainPF = CF_CLUSTER_CHAIN_PF;
-};
-
 // MODE 0: MEA, 1: BPP, 2: the inside with the accurate log-sum-exp alone
 // (logZ, and the tables the sampler draws from).
 template <int MODE, class Team>
@@ -607,7 +604,7 @@ __device__ __forceinline__ void fold_lat(const FoldArgs& A, const Team& tm, int 
 
 template <int MODE>
 __global__ void __launch_bounds__(kLatThreads, 1) k_fold_lat32(FoldArgs A) {
-    fold_lat<MODE>(A, LatTeam{}, blockIdx.x);
+    fold_lat<MODE>(A, CtaTeam{}, blockIdx.x);
 }
 template <int MODE>
 __global__ void __launch_bounds__(kFoldThreads, 2) k_fold_cluster32(FoldArgs A) {

@@ -56,7 +56,6 @@ struct LinHead {
     LinWeights<R> w;
     R kp[32];         // CF_LIN_SCALE^t
     int npair[2];     // double: pairable cells of the diagonal (by parity)
-    int bad;
 };
 
 static_assert(offsetof(LinHead<float>, w) % 16 == 0 && offsetof(LinWeights<float>, csf) % 16 == 0,
@@ -274,7 +273,7 @@ __device__ __forceinline__ void lin_inside(const LinArgs& A) {
     }
     for (int k = L + 2 + tid; k < 32; k += NT) h->kp[k] = R(0);   // loops longer than the sequence
     for (int k = tid; k < (kRing + 8) * gs; k += NT) G[k] = R(0);   // and B, M
-    if (tid == 0) h->bad = h->npair[0] = h->npair[1] = 0;
+    if (tid == 0) h->npair[0] = h->npair[1] = 0;
     encode_seq(A.seqs, A.mask, D.seq_off, L, s, pc);
     __syncthreads();
 
@@ -465,7 +464,6 @@ struct LinOutHead {
     float hp[31 * kOutWarps];
     float red[8 * kOutWarps];
     int ctr[2];
-    int bad;
 };
 struct LinOutLayout {
     int gs, go, cs;

@@ -101,7 +101,6 @@ __device__ __forceinline__ void exterior_outside_warp(const Lse32& sr, const Sme
 // in a single loop of (a-1) + (L-1-b) = L-2-t iterations, which is the same for
 // every cell of diagonal t -- lanes of a warp working on one diagonal stay
 // converged.
-template <int CPF = kChainPF>
 __device__ __forceinline__ void outside_A(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
                                                  const SeqV& Q, const OutTabs& T, int a, int b) {
     const ParamView<float> P{tb->blob};
@@ -124,7 +123,7 @@ __device__ __forceinline__ void outside_A(const Lse32& sr, const SmemTabs<float>
         int x = tri_off(t + n1, m) + a - n1, y = fm1 + tri_off(n1, m) + a - n1, dx = n1 + t - m, dy = n1 - m;
         const int x2 = tri_off(t + n2, m) + a, y2 = tri_off(n2, m) + b;
         int kl = 0;
-        prefetched_chain<float, CPF>(
+        prefetched_chain<float>(
             K,
             [&](const float*& px, const float*& py) {
                 const bool over = kl == n1;
@@ -179,8 +178,7 @@ __device__ __forceinline__ void outside_A(const Lse32& sr, const SmemTabs<float>
 //     b+2+(30-l1), highest bit first.  Source (a-1, b+1) first contributes
 //     through FM1o (block 2, cpu.py:708-714), then through block 3.
 // `lanes`: the lanes evaluating cells together, walked together as in
-// inside_B (rows from the largest l1max among them, per row as many slots as
-// the lane with the most candidates).
+// inside_B, four rows at a time from the largest l1max among them.
 __device__ __forceinline__ void outside_B(const Lse32& sr, const SmemTabs<float>* __restrict__ tb,
                                           const SeqV& Q, const OutTabs& T, int a, int b, unsigned lanes) {
     const ParamView<float> P{tb->blob};
