@@ -465,12 +465,16 @@ int make_fold_plan(cf_engine* eng, Job job, const int64_t* offsets, std::vector<
     // Few enough for the latency kernels: a sequence on a cluster or, one after another on an SM, on CTAs of their own.
     // They win until the grouped kernels' CTAs fill the device (GB300, ms, latency / grouped, MEA and 1 sample: 200 nt n =
     // 304 19 / 24 and 10 / 13, 456 29 / 26 and 15 / 13; 100 nt n = 456 8.8 / 9.3 and 5.9 / 5.4; 320 nt n = 304 46 / 53, 456
-    // 70 / 59; 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA).  Not on a shared device: a
+    // 70 / 59; 40-400 nt n = 700 59 / 73 and 29 / 31, 911 76 / 78 and 36 / 32; posteriors as MEA), which short sequences'
+    // do earlier: half of 512 threads have nothing to do (20 nt n = 152 0.28 / 0.40 and 0.36 / 0.43, 304 0.50 / 0.43 and 0.62
+    // / 0.58; 40 nt n = 304 1.5 / 1.9 and 1.5 / 1.6, 456 2.1 / 1.9 and 2.1 / 1.8; 15-25 nt n = 304 0.51 / 0.64 and 0.61 / 0.71,
+    // 608 0.96 / 0.74 and 1.10 / 1.02; 20-40 nt n = 608 1.7 / 1.9, 760 2.1 / 1.9 and 2.07 / 1.97).  Not on a shared device: a
     // 512-thread CTA waits for an SM with room for all of it, which other engines' smaller CTAs kept taking first.
     int sms = 0, smem_optin = 0;
     CF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, eng->device));
     CF_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, eng->device));
-    const int cut = uniform ? (P.Lmax <= 128 ? 3 : 2) : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
+    const int most = P.Lmax, cut = uniform ? (most <= 20 ? 1 : most <= 48 ? 2 : most <= 128 ? 3 : 2)
+                                           : most <= 25 ? 2 : most <= 32 ? 3 : most <= 64 ? 4 : job == JOB_MEA || job == JOB_BPP ? 6 : 5;
     const bool few = batched && !eng->shared && n <= cut * sms &&
                      (job == JOB_LOGZ || job == JOB_BPP || job == JOB_MEA || job == JOB_SAMPLE);
     if (batched) {

@@ -161,6 +161,6 @@ assert plan(2046, 15, 25) == ("group", 3)        # 608 CTAs
 assert plan(10000, 20, 40) == ("group", 8)
 assert plan(3000, 100, 256) == ("group", 2)
 assert plan(2046, 40, 400) == ("group", 1)
-assert plan(700, 15, 25) == ("group", 1)         # the latency kernels
+assert plan(300, 15, 25) == ("group", 1)         # the latency kernels
 assert plan(2046, 60, 70) == ("group", 4)        # lengths alike: one wave
 """)
