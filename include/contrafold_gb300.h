@@ -98,8 +98,9 @@ int cf_engine_set_mode(cf_engine* eng, int mode);
  * folded by the 8 CTAs of a thread-block cluster -- the latency of long
  * sequences, for logZ, BPP, MEA and sampling (kind 0 follows the schedule
  * table, cf_engine_load_tuning).  logZ of up to 512 nt, FP64 logZ of up to 416
- * and Viterbi have kernels of their own on every kind; ctas_per_sm caps the residency of the persistent
- * CTA kernels (0 = automatic).  Results are identical for every choice.
+ * and Viterbi have kernels of their own on every kind; ctas_per_sm caps the
+ * residency of the persistent CTA kernels (0 = automatic).  Results are
+ * identical for every choice.
  * Kind 5 (the queue schedule, cf_queue.cu) is disabled and returns
  * CF_EINVAL: its kernel did not finish in two GPU test runs. */
 int cf_engine_set_schedule(cf_engine* eng, int kind, int ctas_per_sm);
@@ -148,8 +149,11 @@ const char* cf_last_error(void);
 const char* cf_version(void);
 
 /* log partition function in FP32 (the recurrence of gpu.py:55-184) with an
- * accurate float32 log-sum-exp (log1pf/expf), within 5e-4 of the FP64 engine.
- * The reference's Fast_LogPlusEquals value (bitwise that of cpu.py:595-678)
+ * accurate float32 log-sum-exp (log1pf/expf) beyond 512 nt and for sequences
+ * whose weights leave a float's range, sums of products up to there: within
+ * 5e-4 of the FP64 engine up to 512 nt, but for stable helices of hundreds of
+ * nucleotides and GC-rich sequences of some 300 nt and more (4e-3 at log Z
+ * 600), and within 5e-5 of its size beyond.  The reference's Fast_LogPlusEquals value (bitwise that of cpu.py:595-678)
  * is what cf_bpp returns in logz_out.  logz_out[n]. */
 int cf_logz(cf_engine* eng, const uint8_t* seqs, const int64_t* offsets,
             const uint8_t* mask, int32_t n, float* logz_out);
@@ -209,7 +213,7 @@ int cf_sample_tasks(cf_engine* eng, const uint8_t* seqs, const int64_t* offsets,
  * unpaired position, returns per sequence b:
  *   logz_out[b]                          logZ (accurate float32 log-sum-exp)
  *   counts_out[b*CF_BLOB_LEN + e]        d logZ / d(parameter-blob entry e) =
- *                                        expected uses of entry e (exact sums)
+ *                                        expected uses of entry e
  *   unpaired_out[offsets[b] + t]         d logZ / d bonus_t = P(t unpaired)
  * The raw-feature gradient is counts_out times the tying Jacobian of the
  * loader (linear, gpu_contrafold/cpu.py:40-135). */
@@ -221,8 +225,12 @@ int cf_grad(cf_engine* eng, const uint8_t* seqs, const int64_t* offsets,
  * a few diagonals (the expected counts are taken one diagonal behind the
  * outside pass); the inside FM2 is kept on every `every`-th diagonal and
  * recomputed on the others (every = 1: all kept; 0: automatic -- 1 below
- * 512 nt, else 8).  The counts are summed in exact 128-bit fixed point, so
- * the results are bitwise the same for every spacing and every run. */
+ * 512 nt, else 8).  The counts of these kernels are summed in exact 128-bit
+ * fixed point, so the results are bitwise the same for every spacing and every
+ * run.  Sequences of up to 400 nt take kernels without that choice, unless
+ * their weights leave a float's range: sums of products, whose counts are
+ * float32 sums in a fixed order (bitwise the same for every run too, and nearer
+ * to 64 bits than the exact sums of float32 log-domain terms). */
 int cf_engine_set_grad_checkpoint(cf_engine* eng, int32_t every);
 /* Device bytes cf_grad uses per sequence of L nt at checkpoint spacing
  * `every` (0: automatic); 0 for a bad length. */
@@ -258,7 +266,9 @@ int cf_plan_status(cf_plan* plan);
  * 3 decode); cf_plan_phase_ms waits for the last run and returns milliseconds. */
 int cf_plan_set_timing(cf_plan* plan, int on);
 int cf_plan_phase_ms(cf_plan* plan, float* ms, int32_t nphases);
-/* Kernels launched by the last cf_plan_run; sequences per CTA of the plan. */
+/* Kernels launched by the last cf_plan_run; sequences per CTA of the plan (for
+ * plans whose sequences all take the sums of products, as for cf_plan_schedule:
+ * what the batch would otherwise take, 1 where that had no room). */
 int cf_plan_launches(const cf_plan* plan);
 /* CUDA graph replay (no reference counterpart): with on != 0, cf_plan_run
  * records the plan's launches into a CUDA graph by stream capture the first
